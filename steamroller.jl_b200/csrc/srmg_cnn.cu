@@ -9,14 +9,14 @@
 // Parameters (FP32 master vector, layer by layer): W_l [9 taps][co][ci], then b_l [co].
 // Every convolution is an implicit GEMM on the tensor cores (mma.sync m16n8k16, BF16
 // operands, FP32 accumulation): M = 16 output pixels, N = 8 output channels, K = 16
-// input channels of one tap.  Tiles live in shared memory with an 80-byte pixel pitch
-// (conflict-free ldmatrix), weights with a 64-byte row pitch and an XOR swizzle of the
-// 16-byte chunks.
+// input channels of one tap.  Tiles and weights live in shared memory with 64-byte rows
+// (a pixel's or an output channel's 32 channels) and an XOR swizzle of the 16-byte chunks.
 //
-// Training kernels: forward (storing every layer's activations), loss and output
-// gradient, input gradient (the same convolution with the transposed, flipped
-// weights, times the ReLU mask), weight gradient (per-CTA partial sums over pixels on
-// the tensor cores, then a fixed-order reduction), and Adam.
+// Training kernels: forward (storing every layer's activations and ReLU signs), loss and
+// output gradient, the chain of input gradients of all layers (the same convolution with
+// the transposed, flipped weights, times the ReLU mask), the weight gradients of all layers
+// (per-CTA partial sums over pixels on the tensor cores, then a fixed-order reduction), and
+// Adam.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -44,14 +44,16 @@ namespace cnn {
 constexpr int kL = 6;          // layers
 constexpr int kC = 32;         // hidden channels
 constexpr int kT = 20;         // tile side (16 cells + 2 ghosts each side)
-constexpr int kTP = 22;        // padded tile side (1 zero pixel each side)
 constexpr int kNP = kT * kT;   // pixels per tile
-constexpr int kPP = 40;        // shared-memory pixel pitch (bf16): 80 bytes
-constexpr int kTileElems = kTP * kTP * kPP;
+// A tile in shared memory: rows of 21 pixels, pixel (y, x) at (y + 1) * 21 + x + 1, so that
+// one zero pixel serves as the right ring of its row and the left ring of the next; 64
+// bytes (32 channels) a pixel, the four 16-byte chunks XOR-swizzled by (pixel / 2) % 4.
+constexpr int kRP = kT + 1;
+constexpr int kTilePix = (kT + 2) * kRP + 1;  // the last tap of the last pixel included
+constexpr int kTileBytes = kTilePix * kC * 2;
+constexpr int kTiles = kNP / 16;         // M tiles of 16 pixels
 constexpr int kWMat = kC * kC;           // one tap's 32 x 32 weight matrix (bf16)
 constexpr int kWElems = kL * 9 * kWMat;  // packed weights of all layers
-constexpr int kThreads = 512;            // 16 warps
-
 __host__ __device__ constexpr int cin(int l) { return l == 0 ? 2 : kC; }
 __host__ __device__ constexpr int cout(int l) { return l == kL - 1 ? 1 : kC; }
 
@@ -84,6 +86,9 @@ __device__ __forceinline__ void ldsm4t(uint32_t a, uint32_t &r0, uint32_t &r1, u
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(a));
 }
+__device__ __forceinline__ void ldsm2t(uint32_t a, uint32_t &r0, uint32_t &r1) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(a));
+}
 __device__ __forceinline__ void ldsm2(uint32_t a, uint32_t &r0, uint32_t &r1) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(a));
 }
@@ -100,162 +105,192 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t *>(&v);
 }
 
-// Padded-tile offset (elements) of tile pixel p shifted by tap (dy, dx) = (tap/3-1, tap%3-1).
-__device__ __forceinline__ int tap_pix(int p, int tap) {
-  const int y = p / kT, x = p - kT * (p / kT);
-  return (y + tap / 3) * kTP + (x + tap % 3);
+// First tap's tile pixel of output pixel p; tap (dy, dx) reads dy * kRP + dx further on.
+__device__ __forceinline__ int tap0(int p) { return (p / kT) * kRP + p % kT; }
+// Byte offset of 16-byte chunk c (8 channels) of tile pixel q.
+__device__ __forceinline__ uint32_t tile_off(int q, int c) {
+  return (uint32_t)(q * 64 + (((c ^ (q >> 1)) & 3) << 4));
 }
 
-// One 3x3 convolution over a tile held in `in` (padded, pitch kPP): for every output
-// pixel p of the 20 x 20 tile and output channel co < 8 * ntiles,
-//   acc[p][co] = sum_{tap, ci < 16 * khalves} in[p + off(tap)][ci] * W[tap][co][ci],
-// W one 32 x 32 swizzled matrix per tap at `w` (flip: the tap order reversed).  The
-// epilogue gets (pixel, co, value) pairs for the two channels a thread holds.
-template <typename Epi>
-__device__ __forceinline__ void conv_tile(const __nv_bfloat16 *in, const __nv_bfloat16 *w, int khalves, int ntiles,
-                                          bool flip, const float *bias, Epi &&epi) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nw = blockDim.x >> 5;
-  const int g = lane >> 2, t4 = lane & 3;
-  const uint32_t in_s = smem_addr(in), w_s = smem_addr(w);
-  for (int mt = warp; mt < kNP / 16; mt += nw) {
-    const int p0 = mt * 16;
-    float acc[4][4];
-    for (int nt = 0; nt < 4; ++nt) {
-      const float b0 = (bias && nt < ntiles) ? bias[nt * 8 + 2 * t4] : 0.f;
-      const float b1 = (bias && nt < ntiles) ? bias[nt * 8 + 2 * t4 + 1] : 0.f;
-      acc[nt][0] = b0;
-      acc[nt][1] = b1;
-      acc[nt][2] = b0;
-      acc[nt][3] = b1;
+__device__ __forceinline__ void group_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// A tile is convolved by a group of WPG warps, M tile mt by warp mt % WPG.  The group keeps
+// the whole layer's output in registers (5 M tiles x 32 channels a warp with WPG = 5) and
+// writes it over the input between two barriers, so a sample holds one 29 KB tile and
+// three groups run in one CTA beside the packed weights of every layer.  A warp loads a
+// tap's weights once for its 5 M tiles (0.35 ldmatrix per mma; one M tile at a time needs
+// 0.75), and while one group waits at its barriers the others keep the tensor pipe
+// busy.  WPG = 13 spreads one sample over the CTA where there is at most one per SM: 2 M tiles a
+// warp, the shorter chain.
+//
+// mma.sync bounds it (m16n8k16 issues every ~8.7 cycles per SM sub-partition: 8550 of them per
+// sample are 272 us for 4096 samples on 148 SMs).  Measured with 16 warps on one sample,
+// one M tile at a time and two tiles in shared memory: 687 us.
+constexpr int max_tiles(int wpg) { return (kTiles + wpg - 1) / wpg; }
+constexpr int groups(int wpg) { return wpg == 5 ? 3 : 1; }
+template <int WPG>
+__device__ __forceinline__ bool has_tile(int wg, int i) { return kTiles % WPG == 0 || wg + i * WPG < kTiles; }
+
+// acc[i] = bias + the convolution of M tile wg + i * WPG: for every output pixel and output
+// channel co < 8 * NT the sum over taps and ci < 16 * KH in that order, W one 32 x 32
+// swizzled matrix per tap at `w` (FLIP: the tap order reversed).
+template <int WPG, int KH, int NT, bool FLIP>
+__device__ __forceinline__ void conv_group(uint32_t tile, uint32_t w, int wg, const float *bias,
+                                           float (&acc)[max_tiles(WPG)][4][4]) {
+  constexpr int MT = max_tiles(WPG);
+  const int lane = threadIdx.x & 31, t4 = lane & 3;
+  int q0[MT];
+#pragma unroll
+  for (int i = 0; i < MT; ++i) {
+    // this lane's ldmatrix row: pixel (lane % 16) of the M tile, chunk lane / 16
+    q0[i] = tap0((has_tile<WPG>(wg, i) ? wg + i * WPG : 0) * 16 + (lane & 15));
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const float b0 = bias ? bias[nt * 8 + 2 * t4] : 0.f, b1 = bias ? bias[nt * 8 + 2 * t4 + 1] : 0.f;
+      acc[i][nt][0] = acc[i][nt][2] = b0;
+      acc[i][nt][1] = acc[i][nt][3] = b1;
     }
-    // this lane's ldmatrix row: pixel p0 + (lane % 8) + 8 * ((lane / 8) % 2), chunk lane / 16
-    const int arow = p0 + (lane & 7) + ((lane >> 3) & 1) * 8;
-    const int achunk = lane >> 4;
-    for (int tap = 0; tap < 9; ++tap) {
-      const int wt = flip ? 8 - tap : tap;
-      const uint32_t a_base = in_s + (uint32_t)(tap_pix(arow, tap) * kPP + achunk * 8) * 2;
-      const uint32_t w_base = w_s + (uint32_t)(wt * kWMat) * 2;
-      for (int kh = 0; kh < khalves; ++kh) {
+  }
+  // weight rows of this lane: NT = 4: (co lane/16 * 8 + lane%8, ci chunk (lane/8)%2), the
+  // next two 8-row groups 1024 bytes on; NT = 1: co lane % 8
+  const int br = (NT == 4 ? (lane >> 4) * 8 : 0) + (lane & 7);
+  const uint32_t wl = w + swz(br, ((lane >> 3) & 1) * 8);
+#pragma unroll 1
+  for (int tap = 0; tap < 9; ++tap) {
+    const uint32_t wb = wl + (uint32_t)((FLIP ? 8 - tap : tap) * kWMat * 2);
+    const int qt = (tap / 3) * kRP + tap % 3;
+#pragma unroll
+    for (int kh = 0; kh < KH; ++kh) {
+      uint32_t b[NT == 4 ? 8 : 2];
+      if (NT == 4) {
+        ldsm4(wb ^ (kh * 32), b[0], b[1], b[2], b[3]);
+        ldsm4((wb + 1024) ^ (kh * 32), b[4], b[5], b[6], b[7]);
+      } else {
+        ldsm2(wb ^ (kh * 32), b[0], b[1]);
+      }
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        if (!has_tile<WPG>(wg, i)) break;  // uniform per warp
         uint32_t a0, a1, a2, a3;
-        ldsm4(a_base + kh * 32, a0, a1, a2, a3);
-        if (ntiles == 1) {
-          uint32_t b0, b1;
-          // matrices: (co 0-7, ci kh*16 + 0-7), (co 0-7, ci kh*16 + 8-15)
-          const int r = lane & 7, c = kh * 16 + ((lane >> 3) & 1) * 8;
-          ldsm2(w_base + swz(r, c), b0, b1);
-          mma16816(acc[0], a0, a1, a2, a3, b0, b1);
-        } else {
-          for (int np = 0; np < 4; np += 2) {
-            uint32_t b0, b1, b2, b3;
-            // matrices: (co np*8.., ci lo), (co np*8.., ci hi), (co (np+1)*8.., lo), (.., hi)
-            const int r = (np + (lane >> 4)) * 8 + (lane & 7), c = kh * 16 + ((lane >> 3) & 1) * 8;
-            ldsm4(w_base + swz(r, c), b0, b1, b2, b3);
-            mma16816(acc[np], a0, a1, a2, a3, b0, b1);
-            mma16816(acc[np + 1], a0, a1, a2, a3, b2, b3);
-          }
-        }
+        ldsm4((tile + tile_off(q0[i] + qt, lane >> 4)) ^ (kh * 32), a0, a1, a2, a3);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) mma16816(acc[i][nt], a0, a1, a2, a3, b[2 * nt], b[2 * nt + 1]);
       }
     }
-    for (int nt = 0; nt < ntiles; ++nt) {
-      const int co = nt * 8 + 2 * t4;
-      epi(p0 + g, co, acc[nt][0], acc[nt][1]);
-      epi(p0 + g + 8, co, acc[nt][2], acc[nt][3]);
-    }
   }
 }
 
-// Shared-memory layout of the forward / input-gradient kernels.
-struct FwdSmem {
-  __nv_bfloat16 w[kWElems];          // packed weights, all layers
-  __nv_bfloat16 tile[2][kTileElems];  // ping-pong activation tiles
-  float bias[kL][kC];
-};
+// Shared memory of the forward and the input-gradient chain: packed weights, then (forward)
+// the biases, then one tile per group.
+constexpr int kFwdW = kWElems * 2, kBwdW = (kL - 1) * 9 * kWMat * 2;
+constexpr int kBiasBytes = kL * kC * 4;
+constexpr int fwd_smem(int wpg) { return kFwdW + kBiasBytes + groups(wpg) * kTileBytes; }
+constexpr int bwd_smem(int wpg) { return kBwdW + groups(wpg) * kTileBytes; }
+constexpr int cnn_threads(int wpg) { return groups(wpg) * wpg * 32; }
 
-__device__ void zero_tile(__nv_bfloat16 *t) {
-  uint4 *p = reinterpret_cast<uint4 *>(t);
-  for (int i = threadIdx.x; i < kTileElems * 2 / 16; i += blockDim.x) p[i] = make_uint4(0, 0, 0, 0);
-}
-
-// Copy the 400 interior pixels (channels 0..31) of a padded tile to global [400][32].
-__device__ void store_tile(const __nv_bfloat16 *t, __nv_bfloat16 *g) {
-  for (int i = threadIdx.x; i < kNP * 4; i += blockDim.x) {
-    const int p = i >> 2, c = (i & 3) * 8;
-    const int y = p / kT, x = p % kT;
-    const uint4 v = *reinterpret_cast<const uint4 *>(t + ((y + 1) * kTP + x + 1) * kPP + c);
-    *reinterpret_cast<uint4 *>(g + p * kC + c) = v;
-  }
-}
-
-// Load global [400][32] into the interior of a padded tile (the ring stays as it is).
-__device__ void load_tile(__nv_bfloat16 *t, const __nv_bfloat16 *g) {
-  for (int i = threadIdx.x; i < kNP * 4; i += blockDim.x) {
-    const int p = i >> 2, c = (i & 3) * 8;
-    const int y = p / kT, x = p % kT;
-    *reinterpret_cast<uint4 *>(t + ((y + 1) * kTP + x + 1) * kPP + c) =
-        *reinterpret_cast<const uint4 *>(g + p * kC + c);
+// Copies the 400 pixels (32 channels) of a tile to global [400][32], by `nthr` threads.
+__device__ __forceinline__ void store_tile(const unsigned char *tile, __nv_bfloat16 *g, int t, int nthr) {
+  for (int i = t; i < kNP * 4; i += nthr) {
+    const int q = tap0(i >> 2) + kRP + 1;
+    reinterpret_cast<uint4 *>(g)[i] = *reinterpret_cast<const uint4 *>(tile + tile_off(q, i & 3));
   }
 }
 
 // Forward pass over n samples.  x: [n][400][2] bf16 (tile pixel order y * 20 + x).
-// y: [n][16][16] FP32 output (the tile's centre).  acts (training): [n][6][400][32]
-// bf16, the input of every layer.
-__global__ void __launch_bounds__(kThreads, 1)
+// y: [n][16][16] FP32 output (the tile's centre).  TRAIN keeps what the backward pass
+// reads: xc [n][400][2], the input; acts [n][5][400][32] bf16, the inputs of layers 1..5; signs
+// [n][5][400][4], their positive channels, byte (pixel, t4) bit 2 nt + j for channel
+// 8 nt + 2 t4 + j.
+template <int WPG, bool TRAIN>
+__global__ void __launch_bounds__(cnn_threads(WPG), 1)
 k_cnn_fwd(const __nv_bfloat16 *__restrict__ x, int n, const __nv_bfloat16 *__restrict__ wpk,
-          const float *__restrict__ bias, float *__restrict__ y, __nv_bfloat16 *__restrict__ acts,
-          const int *__restrict__ n_dev = nullptr) {
+          const float *__restrict__ bias, float *__restrict__ y, uint32_t *__restrict__ xc,
+          __nv_bfloat16 *__restrict__ acts, unsigned char *__restrict__ signs, const int *__restrict__ n_dev) {
+  constexpr int MT = max_tiles(WPG), NTHR = WPG * 32, NX = (kNP + NTHR - 1) / NTHR;
   extern __shared__ __align__(128) unsigned char smraw[];
-  FwdSmem &S = *reinterpret_cast<FwdSmem *>(smraw);
+  float *sbias = reinterpret_cast<float *>(smraw + kFwdW);
   if (n_dev) n = min(n, *n_dev);  // sample count decided on the device
   {
     const uint4 *src = reinterpret_cast<const uint4 *>(wpk);
-    uint4 *dst = reinterpret_cast<uint4 *>(S.w);
-    for (int i = threadIdx.x; i < kWElems * 2 / 16; i += blockDim.x) dst[i] = src[i];
-    for (int i = threadIdx.x; i < kL * kC; i += blockDim.x) S.bias[i / kC][i % kC] = bias[i];
-    zero_tile(S.tile[0]);
-    zero_tile(S.tile[1]);
+    uint4 *dst = reinterpret_cast<uint4 *>(smraw);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < kFwdW / 16; i += blockDim.x) dst[i] = src[i];
+    for (int i = threadIdx.x; i < kL * kC; i += blockDim.x) sbias[i] = bias[i];
+    uint4 *z = reinterpret_cast<uint4 *>(smraw + kFwdW + kBiasBytes);  // the zero ring (and the rest)
+    for (int i = threadIdx.x; i < groups(WPG) * kTileBytes / 16; i += blockDim.x) z[i] = make_uint4(0, 0, 0, 0);
   }
   __syncthreads();
-  for (int s = blockIdx.x; s < n; s += gridDim.x) {
-    // input: channels 0, 1 from x, 2..15 zero (layer 1 reads channels 0..15)
-    for (int p = threadIdx.x; p < kNP; p += blockDim.x) {
-      const int yy = p / kT, xx = p % kT;
-      __nv_bfloat16 *d = S.tile[0] + ((yy + 1) * kTP + xx + 1) * kPP;
-      const __nv_bfloat162 v = reinterpret_cast<const __nv_bfloat162 *>(x)[(int64_t)s * kNP + p];
-      uint4 *d4 = reinterpret_cast<uint4 *>(d);
-      d4[0] = make_uint4(*reinterpret_cast<const uint32_t *>(&v), 0, 0, 0);
-      d4[1] = make_uint4(0, 0, 0, 0);
-      if (acts) {
-        uint4 *g4 = reinterpret_cast<uint4 *>(acts + ((int64_t)s * kL) * kNP * kC + p * kC);
-        g4[0] = d4[0];
-        g4[1] = d4[1];
-        g4[2] = make_uint4(0, 0, 0, 0);
-        g4[3] = make_uint4(0, 0, 0, 0);
+  const int grp = threadIdx.x / NTHR, t = threadIdx.x % NTHR, wg = t >> 5;
+  const int lane = t & 31, g = lane >> 2, t4 = lane & 3;
+  unsigned char *tile = smraw + kFwdW + kBiasBytes + grp * kTileBytes;
+  const uint32_t tile_s = smem_addr(tile), w_s = smem_addr(smraw);
+  const uint32_t *x2 = reinterpret_cast<const uint32_t *>(x);
+  uint32_t xv[NX];
+  auto fetch = [&](int s) {
+#pragma unroll
+    for (int k = 0; k < NX; ++k)
+      if (s < n && t + k * NTHR < kNP) xv[k] = x2[(int64_t)s * kNP + t + k * NTHR];
+  };
+  const int s0 = blockIdx.x + gridDim.x * grp, ds = gridDim.x * groups(WPG);
+  fetch(s0);
+  for (int s = s0; s < n; s += ds) {
+    // input: channels 0, 1 from x, 2..15 zero (layer 0 reads channels 0..15)
+#pragma unroll
+    for (int k = 0; k < NX; ++k) {
+      const int p = t + k * NTHR;
+      if (p >= kNP) break;
+      const int q = tap0(p) + kRP + 1;
+      *reinterpret_cast<uint4 *>(tile + tile_off(q, 0)) = make_uint4(xv[k], 0, 0, 0);
+      *reinterpret_cast<uint4 *>(tile + tile_off(q, 1)) = make_uint4(0, 0, 0, 0);
+      if (TRAIN) xc[(int64_t)s * kNP + p] = xv[k];
+    }
+    group_sync(1 + grp, NTHR);
+    float acc[MT][4][4];
+#pragma unroll 1
+    for (int l = 0; l < kL - 1; ++l) {
+      const uint32_t w = w_s + (uint32_t)(l * 9 * kWMat * 2);
+      if (l == 0) conv_group<WPG, 1, 4, false>(tile_s, w, wg, sbias, acc);
+      else conv_group<WPG, 2, 4, false>(tile_s, w, wg, sbias + l * kC, acc);
+      group_sync(1 + grp, NTHR);  // every warp has read the layer's input
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        if (!has_tile<WPG>(wg, i)) break;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int p = (wg + i * WPG) * 16 + g + 8 * r, q = tap0(p) + kRP + 1;
+          uint32_t sg = 0;
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) {
+            const uint32_t v = pack_bf16(fmaxf(acc[i][nt][2 * r], 0.f), fmaxf(acc[i][nt][2 * r + 1], 0.f));
+            *reinterpret_cast<uint32_t *>(tile + tile_off(q, nt) + t4 * 4) = v;
+            if (TRAIN) {
+              // positive as stored: not zero, not NaN, no sign bit
+              const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162 *>(&v);
+              sg |= (__low2float(h) > 0.f ? 1u : 0u) << (2 * nt) | (__high2float(h) > 0.f ? 2u : 0u) << (2 * nt);
+            }
+          }
+          if (TRAIN) signs[((int64_t)s * (kL - 1) + l) * (kNP * 4) + p * 4 + t4] = (unsigned char)sg;
+        }
+      }
+      group_sync(1 + grp, NTHR);
+      if (TRAIN) store_tile(tile, acts + ((int64_t)s * (kL - 1) + l) * kNP * kC, t, NTHR);
+    }
+    fetch(s + ds);
+    conv_group<WPG, 2, 1, false>(tile_s, w_s + (uint32_t)((kL - 1) * 9 * kWMat * 2), wg, sbias + (kL - 1) * kC, acc);
+    if (t4 == 0) {
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        if (!has_tile<WPG>(wg, i)) break;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int p = (wg + i * WPG) * 16 + g + 8 * r, yy = p / kT, xx = p % kT;
+          if (yy >= 2 && yy < 18 && xx >= 2 && xx < 18) y[(int64_t)s * 256 + (yy - 2) * 16 + (xx - 2)] = acc[i][0][2 * r];
+        }
       }
     }
-    __syncthreads();
-    for (int l = 0; l < kL; ++l) {
-      const __nv_bfloat16 *in = S.tile[l & 1];
-      __nv_bfloat16 *out = S.tile[(l + 1) & 1];
-      const bool last = l == kL - 1;
-      if (!last) {
-        conv_tile(in, S.w + l * 9 * kWMat, l == 0 ? 1 : 2, 4, false, S.bias[l],
-                  [&](int p, int co, float v0, float v1) {
-                    const int yy = p / kT, xx = p % kT;
-                    *reinterpret_cast<uint32_t *>(out + ((yy + 1) * kTP + xx + 1) * kPP + co) =
-                        pack_bf16(fmaxf(v0, 0.f), fmaxf(v1, 0.f));
-                  });
-      } else {
-        conv_tile(in, S.w + l * 9 * kWMat, 2, 1, false, S.bias[l], [&](int p, int co, float v0, float) {
-          if (co != 0) return;
-          const int yy = p / kT, xx = p % kT;
-          if (yy >= 2 && yy < 18 && xx >= 2 && xx < 18 && y) y[(int64_t)s * 256 + (yy - 2) * 16 + (xx - 2)] = v0;
-        });
-      }
-      __syncthreads();
-      if (!last && acts) store_tile(out, acts + ((int64_t)s * kL + l + 1) * kNP * kC);
-    }
-    __syncthreads();
+    group_sync(1 + grp, NTHR);
   }
 }
 
@@ -272,224 +307,316 @@ __device__ __forceinline__ void rweights(int geom, int ir0, int qx, float &wm, f
   }
 }
 
-// Normalised residual of the guess at interior cell (qy, qx) (1..14) of sample s:
-// rho = L(y) + x1, the discrete operator applied to the output plus the normalised
-// right-hand-side change (both in units where the output scale is s_l |db|).
-__device__ __forceinline__ float resid(const float *ys, const __nv_bfloat16 *xs, int geom, int ir0, int qy, int qx) {
-  float wm, wp;
-  rweights(geom, ir0, qx, wm, wp);
-  const float c = ys[qy * 16 + qx];
-  const float L = wm * ys[qy * 16 + qx - 1] + wp * ys[qy * 16 + qx + 1] + ys[(qy - 1) * 16 + qx] +
-                  ys[(qy + 1) * 16 + qx] - 4.f * c;
-  return L + __bfloat162float(xs[((qy + 2) * kT + qx + 2) * 2 + 1]);
-}
-
-// Loss and output gradient.  Loss = mean_{n x 256} (y - t)^2 + lambda mean_{n x 196} rho^2
-// (rho on the 14 x 14 interior cells); loss partials per CTA (fixed order) and
-// dz[n][400][32] bf16 = dLoss/dy on the centre pixels of channel 0, else 0.
-__global__ void k_cnn_loss(const float *__restrict__ y, const float *__restrict__ t,
-                           const __nv_bfloat16 *__restrict__ x, const int *__restrict__ ir0s, float lambda, int geom,
-                           int n, __nv_bfloat16 *__restrict__ dz, double *__restrict__ loss_part) {
+// Loss and output gradient.  Loss = mean_{n x 256} (y - t)^2 + lambda mean_{n x 196} rho^2,
+// rho = L(y) + x1 on the 14 x 14 interior cells: the normalised residual of the guess, the
+// discrete operator applied to the output plus the normalised right-hand-side change (both
+// in units where the output scale is s_l |db|).  One sample per CTA pass, one thread per
+// cell; rho is formed once per cell in shared memory (0 off the interior) and its gradient
+// gathered from the neighbours whose stencil reads the cell.  Loss partials per CTA (fixed
+// order) and dy[n][256] = dLoss/dy.
+__global__ void __launch_bounds__(256)
+k_cnn_loss(const float *__restrict__ y, const float *__restrict__ t, const __nv_bfloat16 *__restrict__ x,
+           const int *__restrict__ ir0s, float lambda, int geom, int n, float *__restrict__ dy,
+           double *__restrict__ loss_part) {
+  __shared__ float sy[18][18], srho[18][18];  // a ring of zeros around the 16 x 16 cells
+  __shared__ double sh[8];
   const double inv = 1.0 / (256.0 * (double)n), invr = 1.0 / (196.0 * (double)n);
+  const int cy = threadIdx.x >> 4, cx = threadIdx.x & 15;
+  const bool inner = cy >= 1 && cy <= 14 && cx >= 1 && cx <= 14;
+  for (int i = threadIdx.x; i < 18 * 18; i += 256) srho[i / 18][i % 18] = sy[i / 18][i % 18] = 0.f;
   double acc = 0.0;
-  const int64_t total = (int64_t)n * kNP;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int s = (int)(i / kNP), p = (int)(i % kNP);
-    const int yy = p / kT, xx = p % kT;
-    float g = 0.f;
-    if (yy >= 2 && yy < 18 && xx >= 2 && xx < 18) {
-      const int cy = yy - 2, cx = xx - 2;
-      const int64_t k = (int64_t)s * 256 + cy * 16 + cx;
-      const float d = y[k] - t[k];
-      acc += (double)d * (double)d * inv;
-      g = (float)(2.0 * inv) * d;
-      if (lambda > 0.f) {
-        const float *ys = y + (int64_t)s * 256;
-        const __nv_bfloat16 *xs = x + (int64_t)s * kNP * 2;
-        const int ir0 = ir0s[s];
-        auto inner = [](int q) { return q >= 1 && q <= 14; };
-        float gr = 0.f;
-        if (inner(cy) && inner(cx)) {
-          const float r0 = resid(ys, xs, geom, ir0, cy, cx);
-          acc += (double)lambda * (double)r0 * (double)r0 * invr;
-          gr += -4.f * r0;
-        }
-        // neighbours whose stencil reads this cell
-        if (inner(cy) && inner(cx + 1)) {  // this cell is the r- neighbour of (cy, cx+1)
-          float wm, wp;
-          rweights(geom, ir0, cx + 1, wm, wp);
-          gr += wm * resid(ys, xs, geom, ir0, cy, cx + 1);
-        }
-        if (inner(cy) && inner(cx - 1)) {  // r+ neighbour of (cy, cx-1)
-          float wm, wp;
-          rweights(geom, ir0, cx - 1, wm, wp);
-          gr += wp * resid(ys, xs, geom, ir0, cy, cx - 1);
-        }
-        if (inner(cy + 1) && inner(cx)) gr += resid(ys, xs, geom, ir0, cy + 1, cx);
-        if (inner(cy - 1) && inner(cx)) gr += resid(ys, xs, geom, ir0, cy - 1, cx);
-        g += (float)(2.0 * invr) * lambda * gr;
+  for (int s = blockIdx.x; s < n; s += gridDim.x) {
+    const int64_t k = (int64_t)s * 256 + threadIdx.x;
+    const float yc = y[k], d = yc - t[k];
+    acc += (double)d * (double)d * inv;
+    float g = (float)(2.0 * inv) * d;
+    if (lambda > 0.f) {
+      const int ir0 = ir0s[s];
+      float wm, wp;
+      __syncthreads();
+      sy[cy + 1][cx + 1] = yc;
+      __syncthreads();
+      if (inner) {
+        rweights(geom, ir0, cx, wm, wp);
+        const float L = wm * sy[cy + 1][cx] + wp * sy[cy + 1][cx + 2] + sy[cy][cx + 1] + sy[cy + 2][cx + 1] - 4.f * yc;
+        const float rho = L + __bfloat162float(x[((int64_t)s * kNP + (cy + 2) * kT + cx + 2) * 2 + 1]);
+        srho[cy + 1][cx + 1] = rho;
+        acc += (double)lambda * (double)rho * (double)rho * invr;
       }
+      __syncthreads();
+      // this cell is the r- neighbour of (cy, cx + 1) and the r+ neighbour of (cy, cx - 1)
+      float gr = -4.f * srho[cy + 1][cx + 1];
+      rweights(geom, ir0, cx + 1, wm, wp);
+      gr += wm * srho[cy + 1][cx + 2];
+      rweights(geom, ir0, cx - 1, wm, wp);
+      if (cx >= 2) gr += wp * srho[cy + 1][cx];
+      gr += srho[cy + 2][cx + 1] + srho[cy][cx + 1];
+      g += (float)(2.0 * invr) * lambda * gr;
     }
-    uint4 *o = reinterpret_cast<uint4 *>(dz + i * kC);
-    __nv_bfloat16 gb = __float2bfloat16_rn(g);
-    o[0] = make_uint4((uint32_t)*reinterpret_cast<uint16_t *>(&gb), 0, 0, 0);
-    o[1] = make_uint4(0, 0, 0, 0);
-    o[2] = make_uint4(0, 0, 0, 0);
-    o[3] = make_uint4(0, 0, 0, 0);
+    dy[k] = g;
   }
-  __shared__ double sh[32];
   for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
     double c = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) c += sh[w];
+    for (int w = 0; w < 8; ++w) c += sh[w];
     loss_part[blockIdx.x] = c;
   }
 }
 
-// dz[n][400][32] bf16 from a given output gradient dy[n][256] (centre pixels, channel 0).
-__global__ void k_cnn_dz_from_dy(const float *__restrict__ dy, int n, __nv_bfloat16 *__restrict__ dz) {
-  const int64_t total = (int64_t)n * kNP;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int s = (int)(i / kNP), p = (int)(i % kNP);
-    const int yy = p / kT, xx = p % kT;
-    float g = 0.f;
-    if (yy >= 2 && yy < 18 && xx >= 2 && xx < 18) g = dy[(int64_t)s * 256 + (yy - 2) * 16 + (xx - 2)];
-    uint4 *o = reinterpret_cast<uint4 *>(dz + i * kC);
-    __nv_bfloat16 gb = __float2bfloat16_rn(g);
-    o[0] = make_uint4((uint32_t)*reinterpret_cast<uint16_t *>(&gb), 0, 0, 0);
-    o[1] = make_uint4(0, 0, 0, 0);
-    o[2] = make_uint4(0, 0, 0, 0);
-    o[3] = make_uint4(0, 0, 0, 0);
-  }
-}
-
-// Input gradient of layer l (l >= 1): dz_out = (dz_in conv W_l^T flipped) * (A_l > 0).
-// dz_in, dz_out: [n][400][32]; wt: transposed packed weights (rows = ci, columns = co);
-// acts: the forward activations (A_l = acts[s][l]).
-__global__ void __launch_bounds__(kThreads, 1)
-k_cnn_dx(int l, const __nv_bfloat16 *__restrict__ dz_in, const __nv_bfloat16 *__restrict__ wt,
-         const __nv_bfloat16 *__restrict__ acts, __nv_bfloat16 *__restrict__ dz_out, int n) {
+// The input gradients of layers 5..1, one chain per sample in its tile: dz_5 is dy (rounded
+// to bf16) on the centre pixels of channel 0, and dz_{l-1} = (dz_l conv W_l^T flipped) *
+// (A_l > 0), written to dz[n][5][400][32] for the weight gradients.  wt: transposed
+// packed weights of layers 1..5 (rows = ci, columns = co); signs: the forward's.  One launch
+// for the whole chain: a launch per layer read and wrote each dz and read each activation
+// again (5 x 42 us at 1024 samples; the chain is bound by mma.sync as the forward is).
+template <int WPG>
+__global__ void __launch_bounds__(cnn_threads(WPG), 1)
+k_cnn_dx(const float *__restrict__ dy, const __nv_bfloat16 *__restrict__ wt,
+         const unsigned char *__restrict__ signs, __nv_bfloat16 *__restrict__ dz, int n) {
+  constexpr int MT = max_tiles(WPG), NTHR = WPG * 32;
   extern __shared__ __align__(128) unsigned char smraw[];
-  FwdSmem &S = *reinterpret_cast<FwdSmem *>(smraw);
   {
-    const uint4 *src = reinterpret_cast<const uint4 *>(wt + l * 9 * kWMat);
-    uint4 *dst = reinterpret_cast<uint4 *>(S.w);
-    for (int i = threadIdx.x; i < 9 * kWMat * 2 / 16; i += blockDim.x) dst[i] = src[i];
-    zero_tile(S.tile[0]);
+    const uint4 *src = reinterpret_cast<const uint4 *>(wt + 9 * kWMat);
+    uint4 *dst = reinterpret_cast<uint4 *>(smraw);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < kBwdW / 16; i += blockDim.x) dst[i] = src[i];
+    uint4 *z = reinterpret_cast<uint4 *>(smraw + kBwdW);
+    for (int i = threadIdx.x; i < groups(WPG) * kTileBytes / 16; i += blockDim.x) z[i] = make_uint4(0, 0, 0, 0);
   }
   __syncthreads();
-  const int khalves = (l == kL - 1) ? 1 : 2;  // input channels of the transposed conv = co of layer l
-  for (int s = blockIdx.x; s < n; s += gridDim.x) {
-    load_tile(S.tile[0], dz_in + (int64_t)s * kNP * kC);
-    __syncthreads();
-    const __nv_bfloat16 *A = acts + ((int64_t)s * kL + l) * kNP * kC;
-    __nv_bfloat16 *o = dz_out + (int64_t)s * kNP * kC;
-    conv_tile(S.tile[0], S.w, khalves, 4, true, nullptr, [&](int p, int ci, float v0, float v1) {
-      const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162 *>(A + p * kC + ci);
-      const float m0 = __low2float(a) > 0.f ? v0 : 0.f, m1 = __high2float(a) > 0.f ? v1 : 0.f;
-      *reinterpret_cast<uint32_t *>(o + p * kC + ci) = pack_bf16(m0, m1);
-    });
-    __syncthreads();
+  const int grp = threadIdx.x / NTHR, t = threadIdx.x % NTHR, wg = t >> 5;
+  const int lane = t & 31, g = lane >> 2, t4 = lane & 3;
+  unsigned char *tile = smraw + kBwdW + grp * kTileBytes;
+  const uint32_t tile_s = smem_addr(tile), w_s = smem_addr(smraw);
+  for (int s = blockIdx.x + gridDim.x * grp; s < n; s += gridDim.x * groups(WPG)) {
+    for (int p = t; p < kNP; p += NTHR) {
+      const int yy = p / kT, xx = p % kT, q = tap0(p) + kRP + 1;
+      float v = 0.f;
+      if (yy >= 2 && yy < 18 && xx >= 2 && xx < 18) v = dy[(int64_t)s * 256 + (yy - 2) * 16 + (xx - 2)];
+      const __nv_bfloat16 h = __float2bfloat16_rn(v);
+      *reinterpret_cast<uint4 *>(tile + tile_off(q, 0)) =
+          make_uint4((uint32_t)*reinterpret_cast<const uint16_t *>(&h), 0, 0, 0);
+      *reinterpret_cast<uint4 *>(tile + tile_off(q, 1)) = make_uint4(0, 0, 0, 0);
+    }
+    group_sync(1 + grp, NTHR);
+    float acc[MT][4][4];
+#pragma unroll 1
+    for (int l = kL - 1; l >= 1; --l) {
+      const uint32_t w = w_s + (uint32_t)((l - 1) * 9 * kWMat * 2);
+      const unsigned char *sl = signs + ((int64_t)s * (kL - 1) + l - 1) * (kNP * 4) + t4;
+      unsigned char sg[MT][2];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          if (has_tile<WPG>(wg, i)) sg[i][r] = sl[((wg + i * WPG) * 16 + g + 8 * r) * 4];
+      if (l == kL - 1) conv_group<WPG, 1, 4, true>(tile_s, w, wg, nullptr, acc);
+      else conv_group<WPG, 2, 4, true>(tile_s, w, wg, nullptr, acc);
+      group_sync(1 + grp, NTHR);
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        if (!has_tile<WPG>(wg, i)) break;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int q = tap0((wg + i * WPG) * 16 + g + 8 * r) + kRP + 1;
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) {
+            const float m0 = (sg[i][r] >> (2 * nt)) & 1 ? acc[i][nt][2 * r] : 0.f;
+            const float m1 = (sg[i][r] >> (2 * nt)) & 2 ? acc[i][nt][2 * r + 1] : 0.f;
+            *reinterpret_cast<uint32_t *>(tile + tile_off(q, nt) + t4 * 4) = pack_bf16(m0, m1);
+          }
+        }
+      }
+      group_sync(1 + grp, NTHR);
+      store_tile(tile, dz + ((int64_t)s * (kL - 1) + l - 1) * kNP * kC, t, NTHR);
+    }
+    group_sync(1 + grp, NTHR);
   }
 }
 
-// Weight gradient of layer l: per CTA, over its samples,
-//   dW[tap][co][ci] += sum_p dz[p][co] * A_l[p + off(tap)][ci],  db[co] += sum_p dz[p][co],
-// written as partials [cta][9][32][32] and [cta][32].  18 warps: warp = (tap, co half).
-constexpr int kDwThreads = 18 * 32;
-struct DwSmem {
-  __nv_bfloat16 a[kTileElems];   // A_l, padded, zero ring
-  __nv_bfloat16 dz[kNP * kPP];   // dz_l, unpadded, pitch kPP
+// Weight gradients of all layers in one launch.  CTA b belongs to one layer l (the CTAs
+// shared out by the layers' work, DwParts) and sums over its samples
+//   dW[tap][co][ci] += sum_p dz_l[p][co] * A_l[p + off(tap)][ci],  db[co] += sum_p dz_l[p][co]
+// into partials [cta][9][32][32] and [cta][32].  15 warps: warp = (pixel fifth kg, tap row
+// dy), three taps x 32 co x 32 ci a warp, so that one dz fragment serves three taps and both
+// of a tap's ci halves (8 ldmatrix per 24 mma; one warp per (tap, co half) took 3 per
+// 4).  db is one more mma against a matrix of ones.  The next sample's tiles arrive by
+// cp.async while this one is summed.  mma.sync bounds it; a launch per layer without the
+// copies in flight, with a serial db sum, took 6 x 55 us at 1024 samples.
+constexpr int kDwThreads = 15 * 32;
+constexpr int kDwStage = kTileBytes + kNP * kC * 2;
+constexpr int kDwSmem = 2 * kDwStage;
+static_assert(9 * kWMat * 4 + kC * 4 <= kDwStage, "the partial sums reuse a stage");
+struct DwParts {
+  int first[kL + 1];  // CTAs first[l] .. first[l + 1] - 1 work on layer l
 };
 
-__global__ void __launch_bounds__(kDwThreads, 1)
-k_cnn_dw(int l, const __nv_bfloat16 *__restrict__ dz, const __nv_bfloat16 *__restrict__ acts, int n,
-         float *__restrict__ dw_part, float *__restrict__ db_part) {
-  extern __shared__ __align__(128) unsigned char smraw[];
-  DwSmem &S = *reinterpret_cast<DwSmem *>(smraw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t4 = lane & 3;
-  const int tap = warp >> 1, mh = warp & 1;  // co rows mh*16 .. mh*16+15
-  zero_tile(S.a);
-  float acc[4][4];
-  for (int i = 0; i < 4; ++i)
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-  float dbacc = 0.f;
-  const int ntiles = (l == 0) ? 1 : 4;      // ci columns: layer 1 has 2 input channels
-  const int mrows = (l == kL - 1) ? 1 : 2;  // co halves with real channels
-  __syncthreads();
-  for (int s = blockIdx.x; s < n; s += gridDim.x) {
-    load_tile(S.a, acts + ((int64_t)s * kL + l) * kNP * kC);
-    for (int i = threadIdx.x; i < kNP * 4; i += blockDim.x) {
-      const int p = i >> 2, c = (i & 3) * 8;
-      *reinterpret_cast<uint4 *>(S.dz + p * kPP + c) =
-          *reinterpret_cast<const uint4 *>(dz + ((int64_t)s * kNP + p) * kC + c);
-    }
-    __syncthreads();
-    if (mh < mrows) {
-      const uint32_t a_s = smem_addr(S.a), z_s = smem_addr(S.dz);
-      for (int k0 = 0; k0 < kNP; k0 += 16) {
-        // A operand (rows co, k = pixels) from dz [p][co] by transposed ldmatrix:
-        // matrices (co 0-7, p 0-7), (co 8-15, p 0-7), (co 0-7, p 8-15), (co 8-15, p 8-15)
-        uint32_t a0, a1, a2, a3;
-        {
-          const int m = lane >> 3, r = lane & 7;
-          const int p = k0 + r + (m >> 1) * 8, c = mh * 16 + (m & 1) * 8;
-          ldsm4t(z_s + (uint32_t)(p * kPP + c) * 2, a0, a1, a2, a3);
-        }
-        for (int np = 0; np < ntiles; np += 2) {
-          // B operand (k = pixels, n = ci) from A_l [p + off][ci] by transposed ldmatrix:
-          // matrices (p 0-7, ci np*8..), (p 8-15, ci np*8..), (p 0-7, ci (np+1)*8..), (p 8-15, ..)
-          const int m = lane >> 3, r = lane & 7;
-          const int p = k0 + r + (m & 1) * 8, c = (np + (m >> 1)) * 8;
-          uint32_t b0, b1, b2, b3;
-          ldsm4t(a_s + (uint32_t)(tap_pix(p, tap) * kPP + c) * 2, b0, b1, b2, b3);
-          mma16816(acc[np], a0, a1, a2, a3, b0, b1);
-          if (np + 1 < ntiles) mma16816(acc[np + 1], a0, a1, a2, a3, b2, b3);
-        }
-      }
-    }
-    // db: warp 0..1 (tap 0) sum dz over pixels for their 16 channels
-    if (tap == 0 && mh < mrows) {
-      for (int c = lane; c < 16; c += 32) {
-        float sacc = 0.f;
-        for (int p = 0; p < kNP; ++p) sacc += __bfloat162float(S.dz[p * kPP + mh * 16 + c]);
-        dbacc += sacc;
-      }
-    }
-    __syncthreads();
-  }
-  float *o = dw_part + (int64_t)blockIdx.x * 9 * kWMat + tap * kWMat;
-  for (int nt = 0; nt < 4; ++nt) {
-    const int ci = nt * 8 + 2 * t4;
-    const int co = mh * 16 + g;
-    o[co * kC + ci] = acc[nt][0];
-    o[co * kC + ci + 1] = acc[nt][1];
-    o[(co + 8) * kC + ci] = acc[nt][2];
-    o[(co + 8) * kC + ci + 1] = acc[nt][3];
-  }
-  if (tap == 0 && lane < 16) db_part[(int64_t)blockIdx.x * kC + mh * 16 + lane] = dbacc;
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// Fixed-order sum of the per-CTA partials into the gradient (master layout) of layer l.
-__global__ void k_cnn_reduce(int l, const float *__restrict__ dw_part, const float *__restrict__ db_part, int nparts,
-                             float *__restrict__ grad) {
-  const int co_n = cout(l), ci_n = cin(l);
-  const int nw = 9 * co_n * ci_n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nw + co_n; i += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    if (i < nw) {
-      const int tap = i / (co_n * ci_n), rem = i % (co_n * ci_n), co = rem / ci_n, ci = rem % ci_n;
-      for (int k = 0; k < nparts; ++k) s += dw_part[(int64_t)k * 9 * kWMat + tap * kWMat + co * kC + ci];
-      grad[woff(l) + i] = s;
+// MH: co halves with real channels; NT: ci columns / 8.
+template <int MH, int NT>
+__device__ __forceinline__ void dw_layer(unsigned char *sm, int l, int part, int nparts, const float *dy,
+                                         const __nv_bfloat16 *dz, const uint32_t *xc, const __nv_bfloat16 *acts, int n,
+                                         float *dw_part, float *db_part) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int kg = warp / 3, dyr = warp % 3;
+  for (int i = threadIdx.x; i < kDwSmem / 16; i += blockDim.x)
+    reinterpret_cast<uint4 *>(sm)[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  const uint32_t sm_s = smem_addr(sm);
+  auto load = [&](int s, int st) {
+    const uint32_t a_s = sm_s + st * kDwStage, z_s = a_s + kTileBytes;
+    if (NT == 1) {  // layer 0: the two input channels
+      for (int p = threadIdx.x; p < kNP; p += blockDim.x)
+        cp_async4(a_s + tile_off(tap0(p) + kRP + 1, 0), xc + (int64_t)s * kNP + p);
     } else {
-      const int co = i - nw;
-      for (int k = 0; k < nparts; ++k) s += db_part[(int64_t)k * kC + co];
-      grad[boff(l) + co] = s;
+      const __nv_bfloat16 *src = acts + ((int64_t)s * (kL - 1) + l - 1) * kNP * kC;
+      for (int i = threadIdx.x; i < kNP * 4; i += blockDim.x)
+        cp_async16(a_s + tile_off(tap0(i >> 2) + kRP + 1, i & 3), src + i * 8);
     }
+    if (MH == 1) {  // layer 5: dz is dy on channel 0 of the centre pixels
+      for (int k = threadIdx.x; k < 256; k += blockDim.x) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(dy[(int64_t)s * 256 + k]);
+        const int p = ((k >> 4) + 2) * kT + (k & 15) + 2;
+        *reinterpret_cast<__nv_bfloat16 *>(sm + st * kDwStage + kTileBytes + tile_off(p, 0)) = h;
+      }
+    } else {
+      const __nv_bfloat16 *src = dz + ((int64_t)s * (kL - 1) + l) * kNP * kC;
+      for (int i = threadIdx.x; i < kNP * 4; i += blockDim.x) cp_async16(z_s + tile_off(i >> 2, i & 3), src + i * 8);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[3][MH][NT][4], accb[MH][4];
+#pragma unroll
+  for (int m = 0; m < MH; ++m) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) accb[m][j] = 0.f;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[d][m][nt][j] = 0.f;
   }
+  const int mt = lane >> 3, r = lane & 7;
+  int st = 0;
+  if (part < n) load(part, 0);
+  for (int s = part; s < n; s += nparts, st ^= 1) {
+    if (s + nparts < n) {
+      load(s + nparts, st ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const uint32_t a_s = sm_s + st * kDwStage, z_s = a_s + kTileBytes;
+#pragma unroll 1
+    for (int k0 = kg * 80; k0 < kg * 80 + 80; k0 += 16) {
+      // A operand (rows co, k = pixels) from dz [p][co] by transposed ldmatrix: matrices (co
+      // 0-7, p 0-7), (co 8-15, p 0-7), (co 0-7, p 8-15), (co 8-15, p 8-15)
+      uint32_t a[MH][4];
+      const uint32_t ad = z_s + tile_off(k0 + r + (mt >> 1) * 8, mt & 1);
+#pragma unroll
+      for (int m = 0; m < MH; ++m) ldsm4t(ad ^ (m * 32), a[m][0], a[m][1], a[m][2], a[m][3]);
+      // B operand (k = pixels, n = ci) from A_l [p + off][ci]: matrices (p 0-7, ci 0-7),
+      // (p 8-15, ci 0-7), (p 0-7, ci 8-15), (p 8-15, ci 8-15)
+      const int q = tap0(k0 + r + (mt & 1) * 8) + dyr * kRP;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const uint32_t bd = a_s + tile_off(q + d, NT == 1 ? 0 : mt >> 1);
+        uint32_t b[NT == 1 ? 2 : 8];
+        if (NT == 1) ldsm2t(bd, b[0], b[1]);
+        else {
+          ldsm4t(bd, b[0], b[1], b[2], b[3]);
+          ldsm4t(bd ^ 32, b[4], b[5], b[6], b[7]);
+        }
+#pragma unroll
+        for (int m = 0; m < MH; ++m)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+            mma16816(acc[d][m][nt], a[m][0], a[m][1], a[m][2], a[m][3], b[2 * nt], b[2 * nt + 1]);
+      }
+      if (dyr == 1) {
+#pragma unroll
+        for (int m = 0; m < MH; ++m)
+          mma16816(accb[m], a[m][0], a[m][1], a[m][2], a[m][3], 0x3F803F80u, 0x3F803F80u);
+      }
+    }
+    __syncthreads();  // the stage is free for the load after next
+  }
+  // the five pixel fifths in order
+  float *red = reinterpret_cast<float *>(sm), *redb = red + 9 * kWMat;
+  for (int k = 0; k < 5; ++k) {
+    if (kg == k) {
+#pragma unroll
+      for (int m = 0; m < MH; ++m) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float *o = red + (dyr * 3 + d) * kWMat + (m * 16 + g + (j >> 1) * 8) * kC + nt * 8 + 2 * t4 + (j & 1);
+              *o = k ? *o + acc[d][m][nt][j] : acc[d][m][nt][j];
+            }
+        if (dyr == 1 && t4 == 0) {
+          float *o = redb + m * 16 + g;
+          o[0] = k ? o[0] + accb[m][0] : accb[m][0];
+          o[8] = k ? o[8] + accb[m][2] : accb[m][2];
+        }
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < 9 * kWMat; i += blockDim.x)
+    if ((MH == 2 || (i / kC) % kC < 16) && (NT == 4 || i % kC < 8)) dw_part[i] = red[i];
+  if (threadIdx.x < MH * 16) db_part[threadIdx.x] = redb[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(kDwThreads, 1)
+k_cnn_dw(DwParts parts, const float *__restrict__ dy, const __nv_bfloat16 *__restrict__ dz,
+         const uint32_t *__restrict__ xc, const __nv_bfloat16 *__restrict__ acts, int n, float *__restrict__ dw_part,
+         float *__restrict__ db_part) {
+  extern __shared__ __align__(128) unsigned char smraw[];
+  int l = 0;
+  while (l < kL - 1 && (int)blockIdx.x >= parts.first[l + 1]) ++l;
+  const int part = blockIdx.x - parts.first[l], np = parts.first[l + 1] - parts.first[l];
+  float *dw = dw_part + (int64_t)blockIdx.x * 9 * kWMat, *db = db_part + (int64_t)blockIdx.x * kC;
+  if (l == 0) dw_layer<2, 1>(smraw, l, part, np, dy, dz, xc, acts, n, dw, db);
+  else if (l < kL - 1) dw_layer<2, 4>(smraw, l, part, np, dy, dz, xc, acts, n, dw, db);
+  else dw_layer<1, 4>(smraw, l, part, np, dy, dz, xc, acts, n, dw, db);
+}
+
+// Fixed-order sum of the per-CTA partials into the gradient (master layout), all layers in
+// one launch, a thread per parameter (16 CTAs a layer were latency-bound: 6 x 37 us).
+__global__ void k_cnn_reduce(DwParts parts, const float *__restrict__ dw_part, const float *__restrict__ db_part,
+                             float *__restrict__ grad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nparams()) return;
+  int l = 0;
+  while (l < kL - 1 && i >= woff(l + 1)) ++l;
+  const int co_n = cout(l), ci_n = cin(l), j = i - woff(l);
+  const float *src;
+  int stride;
+  if (j < 9 * co_n * ci_n) {
+    const int tap = j / (co_n * ci_n), rem = j % (co_n * ci_n);
+    src = dw_part + tap * kWMat + (rem / ci_n) * kC + rem % ci_n;
+    stride = 9 * kWMat;
+  } else {
+    src = db_part + (j - 9 * co_n * ci_n);
+    stride = kC;
+  }
+  float s = 0.f;
+#pragma unroll 8
+  for (int k = parts.first[l]; k < parts.first[l + 1]; ++k) s += src[(int64_t)k * stride];
+  grad[i] = s;
 }
 
 #include "srmg_cnn_tc.cuh"
@@ -732,7 +859,7 @@ struct srmg_cnn {
   bool use_tc = false;           // the warm start's forward pass on tcgen05
   int adam_t = 0;
   int train_n = 0;  // samples of the last training forward
-  DevBuf acts, dz0, dz1, dwp, dbp, lossp, y;
+  DevBuf xc, acts, signs, dz, dy, dwp, dbp, lossp, y;
   int nsm = 0;
 };
 
@@ -747,47 +874,81 @@ int cnn_pack(srmg_cnn *net) {
 
 int cnn_setup_attrs(srmg_cnn *net) {
   srmg_ctx *ctx = net->err_ctx;
-  CK(cudaFuncSetAttribute(k_cnn_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem)));
-  CK(cudaFuncSetAttribute(k_cnn_dx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem)));
-  CK(cudaFuncSetAttribute(k_cnn_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DwSmem)));
-  CK(cudaFuncSetAttribute(k_cnn_fwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem)));
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  CK(cudaFuncSetAttribute(k_cnn_fwd<5, false>, attr, fwd_smem(5)));
+  CK(cudaFuncSetAttribute(k_cnn_fwd<5, true>, attr, fwd_smem(5)));
+  CK(cudaFuncSetAttribute(k_cnn_fwd<13, false>, attr, fwd_smem(13)));
+  CK(cudaFuncSetAttribute(k_cnn_fwd<13, true>, attr, fwd_smem(13)));
+  CK(cudaFuncSetAttribute(k_cnn_dx<5>, attr, bwd_smem(5)));
+  CK(cudaFuncSetAttribute(k_cnn_dx<13>, attr, bwd_smem(13)));
+  CK(cudaFuncSetAttribute(k_cnn_dw, attr, kDwSmem));
+  CK(cudaFuncSetAttribute(k_cnn_fwd_tc, attr, (int)sizeof(TcSmem)));
   return SRMG_OK;
+}
+
+// Launches the forward pass.  Up to one sample per SM the whole CTA works on one sample
+// (13 warps), above that three samples share an SM (5 warps each).
+template <bool TRAIN>
+void launch_fwd(srmg_cnn *net, cudaStream_t stream, const __nv_bfloat16 *x, int n, float *y, const int *n_dev) {
+  uint32_t *xc = (uint32_t *)net->xc.p;
+  __nv_bfloat16 *acts = (__nv_bfloat16 *)net->acts.p;
+  unsigned char *signs = (unsigned char *)net->signs.p;
+  if (n <= net->nsm)
+    k_cnn_fwd<13, TRAIN><<<n, cnn_threads(13), fwd_smem(13), stream>>>(x, n, net->wpk, net->bias, y, xc, acts, signs,
+                                                                      n_dev);
+  else
+    k_cnn_fwd<5, TRAIN><<<net->nsm, cnn_threads(5), fwd_smem(5), stream>>>(x, n, net->wpk, net->bias, y, xc, acts,
+                                                                          signs, n_dev);
 }
 
 // Forward pass keeping every layer's activations (training), outputs in net->y.
 int cnn_fwd_train(srmg_cnn *net, const __nv_bfloat16 *x, int n) {
   srmg_ctx *ctx = net->err_ctx;
-  const int grid = cnn_grid(net, n);
-  RC(ensure(ctx, net->acts, (size_t)n * kL * kNP * kC * 2));
-  RC(ensure(ctx, net->dz0, (size_t)n * kNP * kC * 2));
-  RC(ensure(ctx, net->dz1, (size_t)n * kNP * kC * 2));
+  const size_t layer = (size_t)n * kNP * kC * 2;  // one layer's activations or gradients
+  RC(ensure(ctx, net->xc, (size_t)n * kNP * 4));
+  RC(ensure(ctx, net->acts, (kL - 1) * layer));
+  RC(ensure(ctx, net->signs, (size_t)(kL - 1) * n * kNP * 4));
+  RC(ensure(ctx, net->dz, (kL - 1) * layer));
   RC(ensure(ctx, net->y, (size_t)n * 256 * 4));
-  RC(ensure(ctx, net->dwp, (size_t)grid * 9 * kWMat * 4));
-  RC(ensure(ctx, net->dbp, (size_t)grid * kC * 4));
+  RC(ensure(ctx, net->dy, (size_t)n * 256 * 4));
+  RC(ensure(ctx, net->dwp, (size_t)net->nsm * 9 * kWMat * 4));
+  RC(ensure(ctx, net->dbp, (size_t)net->nsm * kC * 4));
   RC(ensure(ctx, net->lossp, 1024 * 8));
-  k_cnn_fwd<<<grid, kThreads, sizeof(FwdSmem), net->stream>>>(x, n, net->wpk, net->bias, (float *)net->y.p,
-                                                              (__nv_bfloat16 *)net->acts.p);
+  launch_fwd<true>(net, net->stream, x, n, (float *)net->y.p, nullptr);
   CK(cudaGetLastError());
   net->train_n = n;
   return SRMG_OK;
 }
 
-// Backward from the output gradient held in net->dz0 (n samples of the last forward).
+// The layers' shares of the weight-gradient CTAs: one CTA per SM, by the layers' work per
+// sample (the first layer has 2 input channels, the last one output channel).
+DwParts dw_parts(int nsm, int n) {
+  static const double work[kL] = {0.4, 1, 1, 1, 1, 0.6};
+  DwParts p;
+  p.first[0] = 0;
+  double done = 0.0;
+  for (int l = 0; l < kL; ++l) {
+    done += work[l] / 5.0;
+    const int to = l == kL - 1 ? nsm : (int)std::lround(done * nsm);
+    p.first[l + 1] = p.first[l] + std::max(1, std::min(n, to - p.first[l]));
+  }
+  return p;
+}
+
+// Backward from the output gradient held in net->dy (n samples of the last forward).
 int cnn_bwd(srmg_cnn *net, int n) {
   srmg_ctx *ctx = net->err_ctx;
-  const int grid = cnn_grid(net, n);
-  __nv_bfloat16 *acts = (__nv_bfloat16 *)net->acts.p;
-  __nv_bfloat16 *dzc = (__nv_bfloat16 *)net->dz0.p, *dzn = (__nv_bfloat16 *)net->dz1.p;
-  for (int l = kL - 1; l >= 0; --l) {
-    k_cnn_dw<<<grid, kDwThreads, sizeof(DwSmem), net->stream>>>(l, dzc, acts, n, (float *)net->dwp.p,
-                                                                (float *)net->dbp.p);
-    k_cnn_reduce<<<16, 256, 0, net->stream>>>(l, (const float *)net->dwp.p, (const float *)net->dbp.p, grid,
-                                              net->grad);
-    if (l > 0) {
-      k_cnn_dx<<<grid, kThreads, sizeof(FwdSmem), net->stream>>>(l, dzc, net->wt, acts, dzn, n);
-      std::swap(dzc, dzn);
-    }
-  }
+  const float *dy = (const float *)net->dy.p;
+  const unsigned char *signs = (const unsigned char *)net->signs.p;
+  __nv_bfloat16 *dz = (__nv_bfloat16 *)net->dz.p;
+  if (n <= net->nsm) k_cnn_dx<13><<<n, cnn_threads(13), bwd_smem(13), net->stream>>>(dy, net->wt, signs, dz, n);
+  else k_cnn_dx<5><<<net->nsm, cnn_threads(5), bwd_smem(5), net->stream>>>(dy, net->wt, signs, dz, n);
+  const DwParts parts = dw_parts(net->nsm, n);
+  k_cnn_dw<<<parts.first[kL], kDwThreads, kDwSmem, net->stream>>>(parts, dy, dz, (const uint32_t *)net->xc.p,
+                                                                  (const __nv_bfloat16 *)net->acts.p, n,
+                                                                  (float *)net->dwp.p, (float *)net->dbp.p);
+  k_cnn_reduce<<<(nparams() + 127) / 128, 128, 0, net->stream>>>(parts, (const float *)net->dwp.p,
+                                                                (const float *)net->dbp.p, net->grad);
   CK(cudaGetLastError());
   return SRMG_OK;
 }
@@ -797,9 +958,9 @@ int cnn_grad(srmg_cnn *net, const __nv_bfloat16 *x, const float *t, const int *i
              double *loss) {
   srmg_ctx *ctx = net->err_ctx;
   RC(cnn_fwd_train(net, x, n));
-  const int lg = std::min(1024, std::max(1, (n * kNP + 255) / 256));
+  const int lg = std::min(1024, n);
   k_cnn_loss<<<lg, 256, 0, net->stream>>>((const float *)net->y.p, t, x, ir0, ir0 ? lambda : 0.f, geom, n,
-                                          (__nv_bfloat16 *)net->dz0.p, (double *)net->lossp.p);
+                                          (float *)net->dy.p, (double *)net->lossp.p);
   RC(cnn_bwd(net, n));
   if (loss) {
     std::vector<double> lp(lg);
@@ -881,7 +1042,7 @@ extern "C" void srmg_cnn_destroy(srmg_cnn *net) {
   for (void *p : {(void *)net->master, (void *)net->grad, (void *)net->adam_m, (void *)net->adam_v, (void *)net->wpk,
                   (void *)net->wt, (void *)net->bias, (void *)net->wtc, (void *)net->tc_err})
     if (p) cudaFree(p);
-  for (DevBuf *b : {&net->acts, &net->dz0, &net->dz1, &net->dwp, &net->dbp, &net->lossp, &net->y})
+  for (DevBuf *b : {&net->xc, &net->acts, &net->signs, &net->dz, &net->dy, &net->dwp, &net->dbp, &net->lossp, &net->y})
     if (b->p) cudaFree(b->p);
   if (net->err_ctx) srmg_destroy(net->err_ctx);
   delete net;
@@ -918,8 +1079,7 @@ extern "C" int srmg_cnn_forward(srmg_cnn *net, const uint16_t *x, float *y, int 
   if (n == 0) return SRMG_OK;
   cudaSetDevice(net->device);
   srmg_ctx *ctx = net->err_ctx;
-  k_cnn_fwd<<<cnn_grid(net, n), kThreads, sizeof(FwdSmem), net->stream>>>((const __nv_bfloat16 *)x, n, net->wpk,
-                                                                          net->bias, y, nullptr);
+  launch_fwd<false>(net, net->stream, (const __nv_bfloat16 *)x, n, y, nullptr);
   CK(cudaGetLastError());
   return SRMG_OK;
 }
@@ -987,8 +1147,8 @@ extern "C" int srmg_cnn_backward_step(srmg_cnn *net, const float *dy, int n, flo
   if (!net || !dy || n <= 0 || n != net->train_n || lr < 0) return SRMG_ERR_BADARG;
   cudaSetDevice(net->device);
   srmg_ctx *ctx = net->err_ctx;
-  k_cnn_dz_from_dy<<<std::min(1024, (n * kNP + 255) / 256), 256, 0, net->stream>>>(dy, n,
-                                                                                   (__nv_bfloat16 *)net->dz0.p);
+  // the caller's dy is its own to reuse: the backward kernels read a copy
+  CK(cudaMemcpyAsync(net->dy.p, dy, (size_t)n * 256 * 4, cudaMemcpyDeviceToDevice, net->stream));
   RC(cnn_bwd(net, n));
   if (grad_host) {
     CK(cudaMemcpyAsync(grad_host, net->grad, nparams() * 4, cudaMemcpyDeviceToHost, net->stream));
@@ -1125,8 +1285,7 @@ extern "C" int srmg_cnn_predict_dev(srmg_ctx *ctx, srmg_cnn *net, double *u, con
     k_cnn_fwd_tc<<<cnn_grid(net, n), kTcThreads, sizeof(TcSmem), ctx->stream>>>(x, n, net->wtc, net->bias, y,
                                                                                 net->tc_err, sel ? count : nullptr);
   else
-    k_cnn_fwd<<<cnn_grid(net, n), kThreads, sizeof(FwdSmem), ctx->stream>>>(x, n, net->wpk, net->bias, y, nullptr,
-                                                                            sel ? count : nullptr);
+    launch_fwd<false>(net, ctx->stream, x, n, y, sel ? count : nullptr);
   CK(cudaGetLastError());
   k_cnn_scatter<<<(int)std::min<int64_t>(4096, ((int64_t)n * 256 + 255) / 256), 256, 0, ctx->stream>>>(
       lrn, ext, y, scale, ctx->d_leaf, n, sel ? list : nullptr, sel ? count : nullptr);
