@@ -726,7 +726,7 @@ int srmg::L_fill_ghost(srmg_ctx *ctx, T *u, int l, const Signs &sg, int mask) {
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nblk == 0) return SRMG_OK;
   const int threads = 256;
-  const int gf = grid_for((int64_t)L.nblk * 4 * 32, threads, kGridCap);
+  const int gf = grid_for((int64_t)L.nblk * 32, threads, kGridCap);
   if (!L.cfaces) {
     // star faces only: the three passes touch disjoint cells and read none of each
     // other's results, so one launch does them all

@@ -79,6 +79,19 @@ template <typename T> __device__ __forceinline__ T dmul(T a, T b);
 template <> __device__ __forceinline__ double dmul<double>(double a, double b) { return __dmul_rn(a, b); }
 template <> __device__ __forceinline__ float dmul<float>(float a, float b) { return __fmul_rn(a, b); }
 
+// a / d for a fixed d > 0 and its correctly rounded reciprocal rd: two corrections of the
+// product a rd by the exact remainder.  The first makes q faithful (off by less than one
+// unit in the last place), so that by Markstein's theorem (IBM J. Res. Dev. 34, 1990) the
+// second gives the correctly rounded quotient, as long as nothing leaves the normal range;
+// there, and for zeros, infinities and NaN, the division itself is called.
+__device__ __forceinline__ double div_by(double a, double d, double rd) {
+  // the exponent field: 2^-700 <= |a| < 2^700 (an integer test; the fp64 pipe is the bound)
+  if ((unsigned)((__double2hiint(a) & 0x7ff00000) - (323 << 20)) >= (1400u << 20)) return __ddiv_rn(a, d);
+  double q = __dmul_rn(a, rd);
+  q = fma(fma(-q, d, a), rd, q);
+  return fma(fma(-q, d, a), rd, q);
+}
+
 // Stencil weights of cell (x, y) of a block at 1-based coords (cr, cz).
 template <typename T>
 struct W5 { T zm, rm, rp, zp; };
@@ -178,78 +191,76 @@ template <typename T>
 __device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelView &lv, const Signs &sg, int phase,
                                                  int64_t t);
 
-// One warp per (block, face): lane -> (layer g = lane/16, position k = lane%16).  On a
-// BoxStencil tree (lv.cfaces set) the launch covers one pass (mask 1, 2 or 4) or the
-// copy and boundary passes together (mask 3), and also fills the corner cells of those
-// passes (fill_corner_cell).
+// One warp per block, a lane one cell of each face: lane -> (layer g = lane/16, position
+// k = lane%16).  The fill is a chain of dependent scattered loads (record, value, store), so
+// it is bound by how many of them are in flight: the four faces' records are loaded
+// together, then the four copied or mirrored values, before any is stored; refinement
+// faces (three values each, few of them) follow on their own.  With a warp per (block, face)
+// 36276 blocks took 72 us.  On a BoxStencil tree (lv.cfaces set) the launch covers one pass
+// (mask 1, 2 or 4) or the copy and boundary passes together (mask 3), and lanes 0..15 also
+// fill the block's 16 corner cells in those passes (fill_corner_cell).
 template <typename T>
 __device__ __forceinline__ void d_fill_ghost(T *__restrict__ u, LevelView lv, Signs sg, int mask) {
   const int lane = threadIdx.x & 31;
-  const int warps_per_cta = blockDim.x >> 5;
   const int g = lane >> 4, k = lane & 15;
-  const int total = lv.nblk * 4;
-  for (int w = blockIdx.x * warps_per_cta + (threadIdx.x >> 5); w < total;
-       w += gridDim.x * warps_per_cta) {
-    const int bi = w >> 2, f = w & 3;
-    const int4 fi = lv.faces[w];
-    if (fi.x == FACE_NONE) continue;
-    const int blk = lv.blocks[bi].x;
-    T *ub = u + (int64_t)blk * kSS;
-    int x, y;
-    if (f == 0) { x = g; y = 2 + k; }
-    else if (f == 1) { x = 18 + g; y = 2 + k; }
-    else if (f == 2) { x = 2 + k; y = g; }
-    else { x = 2 + k; y = 18 + g; }
-    if (fi.x == FACE_NEIGHBOR) {
-      if (!(mask & 1)) continue;
-      // _fill_ghost_copy! (src/connectivity.jl:184-198): ghost <- neighbour's valid
-      // cell M positions away along the face normal.
-      const T *src = u + (int64_t)fi.y * kSS;
-      int sx = x, sy = y;
-      if (f == 0) sx = x + kM; else if (f == 1) sx = x - kM;
-      else if (f == 2) sy = y + kM; else sy = y - kM;
-      ub[x + kS * y] = src[sx + kS * sy];
-    } else if (fi.x == FACE_BOUNDARY) {
-      if (!(mask & 2)) continue;
-      // fill_ghost_bnd! (src/connectivity.jl:217-231), mirrorghost (src/blockfield.jl:513-521)
-      int mx = x, my = y;
-      if (f == 0) mx = 2 * kG - 1 - x; else if (f == 1) mx = 2 * (kG + kM) - 1 - x;
-      else if (f == 2) my = 2 * kG - 1 - y; else my = 2 * (kG + kM) - 1 - y;
-      const T a = T(sg.v[face_sign_index(f)]);
-      ub[x + kS * y] = dmul<T>(a, ub[mx + kS * my]);
-    } else {
-      if (!(mask & 4)) continue;
-      // fill_ghost_interp! (src/connectivity.jl:251-258) + interp! (src/interp.jl:24-63)
-      // from the coarse block's subblockbnd(subblock, -face) (src/blockfield.jl:416-434).
-      const T *cb = u + (int64_t)fi.y * kSS;
-      const int sbr = fi.z, sbz = fi.w;
-      int jr, jz, ir, iz;  // coarse source cell and the 0/1 child offsets per dim
-      if (f <= 1) {
-        jr = (f == 0) ? (1 + 8 * sbr) : (2 + 8 * (sbr - 1));
-        ir = g;
-        jz = 2 + 8 * (sbz - 1) + (k >> 1);
-        iz = k & 1;
-      } else {
-        jz = (f == 2) ? (1 + 8 * sbz) : (2 + 8 * (sbz - 1));
-        iz = g;
-        jr = 2 + 8 * (sbr - 1) + (k >> 1);
-        ir = k & 1;
-      }
-      const int o = jr + kS * jz;
-      if (mask & 8) {  // InterpCopy (src/interp.jl:66-85): the coarse cell's value itself
-        ub[x + kS * y] = cb[o];
-        continue;
-      }
-      T v = dmul<T>(T(0.5), cb[o]);
-      v = dadd<T>(v, dmul<T>(T(0.25), cb[o + (2 * ir - 1)]));
-      v = dadd<T>(v, dmul<T>(T(0.25), cb[o + kS * (2 * iz - 1)]));
-      ub[x + kS * y] = v;
+  const bool corners = lv.cfaces && (mask == 1 || mask == 2 || mask == 3 || mask == 4);
+  const int stride = gridDim.x * (blockDim.x >> 5);
+  for (int bi = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); bi < lv.nblk; bi += stride) {
+    int type[4], src[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const int2 r = *reinterpret_cast<const int2 *>(lv.faces + 4 * bi + f);
+      type[f] = r.x;
+      src[f] = r.y;
     }
-  }
-  if (lv.cfaces && (mask == 1 || mask == 2 || mask == 3 || mask == 4)) {
-    const int64_t ct = (int64_t)lv.nblk * 16;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ct; t += (int64_t)gridDim.x * blockDim.x)
-      fill_corner_cell<T>(u, lv, sg, mask, t);
+    T *ub = u + (int64_t)lv.blocks[bi].x * kSS;
+    T v[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const int x = f == 0 ? g : f == 1 ? 18 + g : 2 + k, y = f == 2 ? g : f == 3 ? 18 + g : 2 + k;  // the ghost
+      if (type[f] == FACE_NEIGHBOR) {
+        // _fill_ghost_copy! (src/connectivity.jl:184-198): ghost <- neighbour's valid
+        // cell M positions away along the face normal.
+        const int sx = f == 0 ? x + kM : f == 1 ? x - kM : x, sy = f == 2 ? y + kM : f == 3 ? y - kM : y;
+        if (mask & 1) v[f] = u[(int64_t)src[f] * kSS + sx + kS * sy];
+      } else if (type[f] == FACE_BOUNDARY) {
+        // fill_ghost_bnd! (src/connectivity.jl:217-231), mirrorghost (src/blockfield.jl:513-521)
+        const int mx = f == 0 ? 2 * kG - 1 - x : f == 1 ? 2 * (kG + kM) - 1 - x : x;
+        const int my = f == 2 ? 2 * kG - 1 - y : f == 3 ? 2 * (kG + kM) - 1 - y : y;
+        if (mask & 2) v[f] = ub[mx + kS * my];
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const int x = f == 0 ? g : f == 1 ? 18 + g : 2 + k, y = f == 2 ? g : f == 3 ? 18 + g : 2 + k;
+      if (type[f] == FACE_NEIGHBOR && (mask & 1)) ub[x + kS * y] = v[f];
+      else if (type[f] == FACE_BOUNDARY && (mask & 2)) ub[x + kS * y] = dmul<T>(T(sg.v[face_sign_index(f)]), v[f]);
+    }
+    if (mask & 4) {
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        if (type[f] != FACE_REFBND) continue;
+        // fill_ghost_interp! (src/connectivity.jl:251-258) + interp! (src/interp.jl:24-63)
+        // from the coarse block's subblockbnd(subblock, -face) (src/blockfield.jl:416-434):
+        // the coarse source cell and the 0/1 child offsets per dimension.
+        const int x = f == 0 ? g : f == 1 ? 18 + g : 2 + k, y = f == 2 ? g : f == 3 ? 18 + g : 2 + k;
+        const int4 fi = lv.faces[4 * bi + f];
+        const T *cb = u + (int64_t)fi.y * kSS;
+        const int sbr = fi.z, sbz = fi.w;
+        const int jr = f == 0 ? 1 + 8 * sbr : f == 1 ? 2 + 8 * (sbr - 1) : 2 + 8 * (sbr - 1) + (k >> 1);
+        const int jz = f == 2 ? 1 + 8 * sbz : f == 3 ? 2 + 8 * (sbz - 1) : 2 + 8 * (sbz - 1) + (k >> 1);
+        const int ir = f <= 1 ? g : k & 1, iz = f <= 1 ? k & 1 : g, o = jr + kS * jz;
+        T w = cb[o];
+        if (!(mask & 8)) {  // else InterpCopy (src/interp.jl:66-85): the coarse cell's value itself
+          const T wr = cb[o + (2 * ir - 1)], wz = cb[o + kS * (2 * iz - 1)];
+          w = dmul<T>(T(0.5), w);
+          w = dadd<T>(w, dmul<T>(T(0.25), wr));
+          w = dadd<T>(w, dmul<T>(T(0.25), wz));
+        }
+        ub[x + kS * y] = w;
+      }
+    }
+    if (corners && lane < 16) fill_corner_cell<T>(u, lv, sg, mask, (int64_t)bi * 16 + lane);
   }
 }
 
@@ -353,18 +364,30 @@ __device__ __forceinline__ void d_postrestrict(T *__restrict__ bf, const T *__re
 // ---- restriction (src/restrict.jl:5-37) --------------------------------------------
 // coarse = ((((0 + f00) + f10) + f01) + f11) / 4 for each Child edge of this level.
 template <typename T>
+struct alignas(2 * sizeof(T)) Pair { T x, y; };
+
+template <typename T>
 __device__ __forceinline__ void d_restrict(T *__restrict__ u, LevelView lv) {
   const int64_t total = (int64_t)lv.nch * 64;
+  const bool aligned = (reinterpret_cast<uintptr_t>(u) & (2 * sizeof(T) - 1)) == 0;  // uniform
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
     const int e = (int)(t >> 6), c = (int)(t & 63);
     const int4 ch = lv.child[e];
     const int kx = c & 7, ky = c >> 3;
     const T *fb = u + (int64_t)ch.x * kSS + (2 + 2 * kx) + kS * (2 + 2 * ky);
-    T f = dadd<T>(T(0), fb[0]);
-    f = dadd<T>(f, fb[1]);
-    f = dadd<T>(f, fb[kS]);
-    f = dadd<T>(f, fb[kS + 1]);
+    Pair<T> lo, hi;  // one load a row where the field allows it: half the load instructions
+    if (aligned) {
+      lo = *reinterpret_cast<const Pair<T> *>(fb);
+      hi = *reinterpret_cast<const Pair<T> *>(fb + kS);
+    } else {
+      lo = Pair<T>{fb[0], fb[1]};
+      hi = Pair<T>{fb[kS], fb[kS + 1]};
+    }
+    T f = dadd<T>(T(0), lo.x);
+    f = dadd<T>(f, lo.y);
+    f = dadd<T>(f, hi.x);
+    f = dadd<T>(f, hi.y);
     u[(int64_t)ch.y * kSS + (2 + 8 * (ch.z - 1) + kx) + kS * (2 + 8 * (ch.w - 1) + ky)] =
         dmul<T>(f, T(0.25));
   }
@@ -621,7 +644,7 @@ __device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelV
 // The kernels of the per-operation path: each a grid-stride loop over its work, so the
 // same bodies also run as the operations of one cooperative launch (srmg_seq.cu).
 template <typename T>
-__global__ void k_fill_ghost(T *__restrict__ u, LevelView lv, Signs sg, int mask) {
+__global__ void __launch_bounds__(256, 6) k_fill_ghost(T *__restrict__ u, LevelView lv, Signs sg, int mask) {
   d_fill_ghost<T>(u, lv, sg, mask);
 }
 

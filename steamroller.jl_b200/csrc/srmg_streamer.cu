@@ -45,7 +45,6 @@ namespace {
 
 constexpr int kSV = kS + 1;
 constexpr int kSSV = kSV * kSV;
-constexpr int kFacesPerDim = (kM + 1) * kM;  // 17 x 16 faces of validindices(e, d)
 
 constexpr double kElemCharge = 1.6021766208e-19;  // src/constants.jl:55
 constexpr double kEpsilon0 = 8.854187817620389e-12;  // src/constants.jl:56
@@ -54,14 +53,6 @@ __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, 
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double dvd(double a, double b) { return __ddiv_rn(a, b); }
-
-// koren_limited(a, b) = psi(a / b) b (src/fluid.jl:274-280).
-__device__ __forceinline__ double koren_limited(double a, double b) {
-  if (mul(a, b) < 0.0) return 0.0;
-  if (fabs(a) > fabs(mul(4.0, b))) return b;
-  if (fabs(mul(10.0, a)) > fabs(mul(4.0, b))) return add(dvd(b, 3.0), dvd(a, 6.0));
-  return a;
-}
 
 // Leaf blocks (no child in any subblock: isleaf, src/tree.jl:105-115) among the blocks
 // holding a leaf cell.
@@ -72,123 +63,174 @@ __device__ __forceinline__ void atomic_min_nonneg(double *addr, double v) {
   atomicMin(reinterpret_cast<unsigned long long *>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
-// flux! (Koren) on the leaf blocks: one 256-thread CTA per block pass, the 544 faces of
-// the block strided over its threads.  ne needs 2 ghost layers, eabs 1.
-__global__ void k_streamer_flux(double *__restrict__ flux, double *__restrict__ maxdt_blk,
-                                double *__restrict__ maxdt_min, const double *__restrict__ ne,
-                                const double *__restrict__ e, const double *__restrict__ eabs,
-                                const int2 *__restrict__ leaf, int nleaf, const int4 *__restrict__ info,
-                                double h1, srmg_transport tr) {
-  __shared__ double s_min[8];
+// min(md, a / b) without the division where it cannot win: md > 0 and a > md b (1 + 8 eps)
+// leave a / b above md.  (0 / 0 is NaN and ignored by fmin, as everywhere here.)
+__device__ __forceinline__ double min_quotient(double md, double a, double b) {
+  if (__double2hiint(md) > 0 && a > mul(mul(md, 1.0 + 8 * 2.220446049250313e-16), b)) return md;
+  return fmin(md, dvd(a, b));
+}
+
+// Cell sizes of a level: h = h1 / 2^(l-1), its reciprocal and (h h / D) / 4.  Scaling by powers
+// of two is exact, so the host forms the level-1 quotients once and the kernels need no
+// division for them.
+struct CellSize {
+  double h1, rh1, dt1;
+};
+__device__ __forceinline__ double pow2(int k) { return __hiloint2double((1023 + k) << 20, 0); }
+
+// The values a face of component d reads: E there, |E| on its two sides, n_e two cells either
+// way along d.
+struct FaceIn {
+  double ed, e0, e1, n[4];
+};
+__device__ __forceinline__ FaceIn load_face(const double *eb, const double *ea, const double *n, int d, int x, int y) {
+  const int st = d ? kS : 1, o = x + kS * y;
+  FaceIn f;
+  f.ed = eb[d * kSSV + x + kSV * y];
+  f.e0 = ea[o];
+  f.e1 = ea[o - st];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) f.n[k] = n[o + (k - 2) * st];
+  return f;
+}
+
+// The face's flux; md is lowered to its time-step limits h / |v| and the Maxwell time.
+__device__ __forceinline__ double face_flux(const FaceIn &f, const srmg_transport &tr, double h, double rh, double r3,
+                                            double r6, double &md) {
+  const double eabs1 = mul(add(f.e0, f.e1), 0.5);  // exact either way
+  const double v = mul(-f.ed, tr.mu);              // mobility / diffusion of the minimal model, theta = 1
+  const bool neg = signbit(v);
+  // downstream, upstream and twice-upstream cells along d
+  const double nd = neg ? f.n[1] : f.n[2], nu = neg ? f.n[2] : f.n[1], nu2 = neg ? f.n[3] : f.n[0];
+  const double a = sub(nu, nu2), b = sub(nd, nu);
+  // koren_limited(a, b) = psi(a / b) b (src/fluid.jl:274-280)
+  double lim = a;
+  if (mul(a, b) < 0.0) lim = 0.0;
+  else if (fabs(a) > fabs(mul(4.0, b))) lim = b;
+  else if (fabs(mul(10.0, a)) > fabs(mul(4.0, b))) lim = add(div_by(b, 3.0, r3), div_by(a, 6.0, r6));
+  double F = mul(v, add(nu, lim));
   const double maxwell = kEpsilon0 / kElemCharge;  // (co.epsilon_0 / co.elementary_charge)
-  for (int k = blockIdx.x; k < nleaf; k += gridDim.x) {
-    const int X = leaf[k].x;
-    if (!leaf_block(info, X)) continue;  // uniform per CTA
-    const double h = dvd(h1, (double)((int64_t)1 << (leaf[k].y - 1)));  // h /= 1 << (level - 1)
-    const double *n = ne + (int64_t)X * kSS;
-    const double *ea = eabs + (int64_t)X * kSS;
-    const double *eb = e + (int64_t)X * 2 * kSSV;
-    double *fb = flux + (int64_t)X * 2 * kSSV;
-    double md = INFINITY;
-    for (int q = threadIdx.x; q < 2 * kFacesPerDim; q += blockDim.x) {
-      const int d = q >= kFacesPerDim;
-      const int r = q - d * kFacesPerDim;
-      // face I = (x, y) of component d; I1 = I - e_d
-      const int x = d ? 2 + (r & 15) : 2 + r % 17;
-      const int y = d ? 2 + (r >> 4) : 2 + r / 17;
-      const int st = d ? kS : 1;  // e_d in tile offsets
-      const int o = x + kS * y;
-      const double ed = eb[d * kSSV + x + kSV * y];
-      const double eabs1 = dvd(add(ea[o], ea[o - st]), 2.0);
-      const double mu = tr.mu, diff = tr.D;  // mobility / diffusion of the minimal model, theta = 1
-      const double v = mul(-ed, mu);
-      const int sv = signbit(v) ? -1 : 1;
-      // downstream, upstream and twice-upstream cells along d
-      const int od = o + st * (sv == 1 ? 0 : -1);
-      const int ou = o + st * (sv == 1 ? -1 : 0);
-      const int ou2 = o + st * (sv == 1 ? -2 : 1);
-      double F = mul(v, add(n[ou], koren_limited(sub(n[ou], n[ou2]), sub(n[od], n[ou]))));
-      const double tmaxwell = dvd(mul(maxwell, eabs1), fabs(F));
-      F = add(F, dvd(mul(diff, sub(n[o - st], n[o])), h));
-      fb[d * kSSV + x + kSV * y] = F;
-      md = fmin(md, fmin(fmin(dvd(h, fabs(v)), dvd(dvd(mul(h, h), diff), 4.0)), tmaxwell));
-    }
-    for (int off = 16; off > 0; off >>= 1) md = fmin(md, __shfl_xor_sync(0xffffffffu, md, off));
-    if ((threadIdx.x & 31) == 0) s_min[threadIdx.x >> 5] = md;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double m = s_min[0];
-      for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmin(m, s_min[w]);
-      if (maxdt_blk) maxdt_blk[X] = m;
-      if (maxdt_min) atomic_min_nonneg(maxdt_min, m);
-    }
-    __syncthreads();
+  md = min_quotient(md, mul(maxwell, eabs1), fabs(F));
+  md = min_quotient(md, h, fabs(v));
+  return add(F, div_by(mul(tr.D, sub(f.n[1], f.n[2])), h, rh));
+}
+
+// flux! (Koren) on the leaf blocks, one 256-thread CTA a block: a thread takes its cell's
+// lower face along each dimension, the first warp also the 32 last faces (x = 18 or y = 18).
+// Latency and the fp64 pipe bound it (a face is ~40 fp64 operations on 7 loaded values, and
+// an fp64 instruction takes two issue slots): a thread's loads are issued together and
+// before the block's leaf flag is known, the divisions by h, 3 and 6 go through their
+// reciprocals, the time-step quotients are only formed where they can lower the minimum
+// (BLK off: seeded with the minimum so far over all blocks), and without BLK the warps
+// never meet.  544 faces strided over 256 threads with eight divisions each and two
+// barriers a block took 445 us on 51877 blocks.  ne needs 2 ghost layers, eabs 1.  BLK:
+// write each block's own minimum to maxdt_blk.
+template <bool BLK>
+__global__ void __launch_bounds__(256, 4)
+k_streamer_flux(double *__restrict__ flux, double *__restrict__ maxdt_blk, double *maxdt_min,
+                const double *__restrict__ ne, const double *__restrict__ e, const double *__restrict__ eabs,
+                const int2 *__restrict__ leaf, const int4 *__restrict__ info, CellSize cs, srmg_transport tr) {
+  const int2 lb = leaf[blockIdx.x];
+  const int X = lb.x;
+  const int x = 2 + (threadIdx.x & 15), y = 2 + (threadIdx.x >> 4);
+  const double *n = ne + (int64_t)X * kSS, *ea = eabs + (int64_t)X * kSS, *eb = e + (int64_t)X * 2 * kSSV;
+  double *fb = flux + (int64_t)X * 2 * kSSV;
+  const FaceIn f0 = load_face(eb, ea, n, 0, x, y), f1 = load_face(eb, ea, n, 1, x, y);
+  double seed = INFINITY;
+  if (!BLK && maxdt_min) seed = *reinterpret_cast<volatile double *>(maxdt_min);
+  if (!leaf_block(info, X)) return;  // uniform per CTA
+  const double h = mul(cs.h1, pow2(1 - lb.y)), rh = mul(cs.rh1, pow2(lb.y - 1));  // h /= 1 << (level - 1)
+  const double r3 = 1.0 / 3.0, r6 = 1.0 / 6.0;
+  double md = fmin(seed, mul(cs.dt1, pow2(2 - 2 * lb.y)));
+  if (threadIdx.x < 32) {
+    const int d = threadIdx.x >> 4, c = threadIdx.x & 15, fx = d ? 2 + c : 18, fy = d ? 18 : 2 + c;
+    fb[d * kSSV + fx + kSV * fy] = face_flux(load_face(eb, ea, n, d, fx, fy), tr, h, rh, r3, r6, md);
+  }
+  fb[x + kSV * y] = face_flux(f0, tr, h, rh, r3, r6, md);
+  fb[kSSV + x + kSV * y] = face_flux(f1, tr, h, rh, r3, r6, md);
+  if (!BLK && !maxdt_min) return;
+  for (int off = 16; off > 0; off >>= 1) md = fmin(md, __shfl_xor_sync(0xffffffffu, md, off));
+  if (!BLK) {
+    if ((threadIdx.x & 31) == 0 && md != seed) atomic_min_nonneg(maxdt_min, md);
+    return;
+  }
+  __shared__ double s_min[8];
+  if ((threadIdx.x & 31) == 0) s_min[threadIdx.x >> 5] = md;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double m = s_min[0];
+    for (int w = 1; w < 8; ++w) m = fmin(m, s_min[w]);
+    maxdt_blk[X] = m;
+    if (maxdt_min) atomic_min_nonneg(maxdt_min, m);
   }
 }
 
-// restrict_flux! over one level's refinement-boundary faces: thread (block, face, k)
-// sets the coarse block's face k (0..7) of the half `subblock` covers to the mean of
-// the two fine faces 2k, 2k + 1: f = ((0 + f_2k) + f_2k+1) / 2.
-__global__ void k_restrict_flux(double *__restrict__ flux, LevelView lv) {
-  const int64_t total = (int64_t)lv.nblk * 32;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int bi = (int)(t >> 5), f = (int)(t >> 3) & 3, k = (int)(t & 7);
-    const int4 fi = lv.faces[4 * bi + f];
-    if (fi.x != FACE_REFBND) continue;
-    const int d = f >> 1;  // the face's dimension: 0 for -r/+r, 1 for -z/+z
-    const int fine_n = (f & 1) ? 2 + kM : 2, coarse_n = (f & 1) ? 2 : 2 + kM;  // normal face index
-    const int sb = d == 0 ? fi.w : fi.z;  // the tangential half
-    const int ct = 2 + 8 * (sb - 1) + k, ft = 2 + 2 * k;
-    const double *src = flux + (int64_t)lv.blocks[bi].x * 2 * kSSV + d * kSSV;
-    double *dst = flux + (int64_t)fi.y * 2 * kSSV + d * kSSV;
-    auto at = [&](int nrm, int tan) { return d == 0 ? nrm + kSV * tan : tan + kSV * nrm; };
-    const double s = add(add(0.0, src[at(fine_n, ft)]), src[at(fine_n, ft + 1)]);
-    dst[at(coarse_n, ct)] = dvd(s, 2.0);
-  }
+// restrict_flux! over every refinement-boundary face of the tree in one launch (a face is
+// next to either a coarser or a finer block, so no level's result feeds another's): thread
+// (block, face, k) sets the coarse block's face k (0..7) of the half `subblock` covers to the
+// mean of the two fine faces 2k, 2k + 1: f = ((0 + f_2k) + f_2k+1) / 2.
+__global__ void k_restrict_flux(double *__restrict__ flux, const int4 *__restrict__ faceb,
+                                const int4 *__restrict__ info, int64_t nblk) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t X = t >> 5;
+  if (X >= nblk) return;
+  const int f = (int)(t >> 3) & 3, k = (int)(t & 7);
+  const int4 fi = faceb[4 * X + f];
+  if (fi.x != FACE_REFBND || info[X].w == 0) return;
+  const int d = f >> 1;  // the face's dimension: 0 for -r/+r, 1 for -z/+z
+  const int fine_n = (f & 1) ? 2 + kM : 2, coarse_n = (f & 1) ? 2 : 2 + kM;  // normal face index
+  const int sb = d == 0 ? fi.z >> 8 : fi.z & 255;  // the tangential half
+  const int ct = 2 + 8 * (sb - 1) + k, ft = 2 + 2 * k;
+  const double *src = flux + X * 2 * kSSV + d * kSSV;
+  double *dst = flux + (int64_t)fi.y * 2 * kSSV + d * kSSV;
+  auto at = [&](int nrm, int tan) { return d == 0 ? nrm + kSV * tan : tan + kSV * nrm; };
+  const double s = add(add(0.0, src[at(fine_n, ft)]), src[at(fine_n, ft + 1)]);
+  dst[at(coarse_n, ct)] = dvd(s, 2.0);
 }
 
 // chemderivs! (init, then add) and fluxderivs! on the valid cells of the leaf blocks:
 // dni = pre + post; dne = (((pre + post) + lower-r) - upper-r) + lower-z) - upper-z,
 // each face term (factor F) / h, factor = |1 + delta / (2 J - 1)| along the radial
 // dimension (1 along the others and in Cartesian geometry).
-__global__ void k_streamer_rates(double *__restrict__ dne, double *__restrict__ dni,
-                                 const double *__restrict__ ne, const double *__restrict__ eabs,
-                                 const double *__restrict__ flux, const int2 *__restrict__ leaf, int nleaf,
-                                 const int4 *__restrict__ info, double h1, int geom, srmg_transport tr) {
-  const int64_t total = (int64_t)nleaf * 256;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int k = (int)(t >> 8), c = (int)(t & 255);
-    const int X = leaf[k].x;
-    const int4 bi = info[X];
-    if ((bi.z & 15) != 0) continue;
-    const double h = dvd(h1, (double)((int64_t)1 << (leaf[k].y - 1)));
-    const int x = 2 + (c & 15), y = 2 + (c >> 4);
-    const int64_t o = (int64_t)X * kSS + x + kS * y;
-    const double n1 = ne[o], E = eabs[o];
-    // NetIonization, MinimalTransportModel: mobility mu, townsend ai exp(-Ei / E),
-    // attachment aa exp(-Ea / E)
-    const double pre = mul(mul(mul(tr.mu, E), n1), mul(tr.ai, exp(dvd(-tr.Ei, E))));
-    const double post = mul(mul(mul(-tr.mu, E), n1), mul(tr.aa, exp(dvd(-tr.Ea, E))));
-    const double chem = add(pre, post);
-    dni[o] = chem;
-    const double *fb = flux + (int64_t)X * 2 * kSSV;
-    const int64_t Jr = gidx(bi.x, x), Jz = gidx(bi.y, y);
-    auto fac = [&](int dim, int delta) -> double {  // factor(geom, J, delta e_dim)
-      const bool radial = (geom == 1 && dim == 0) || (geom == 2 && dim == 1);
-      if (geom == 0) return 1.0;
-      const int64_t J = dim == 0 ? Jr : Jz;
-      const double q = radial ? dvd((double)delta, (double)(2 * J - 1)) : 0.0;
-      return fabs(add(1.0, q));
-    };
-    double v = chem;
-    v = add(v, dvd(mul(fac(0, -1), fb[x + kSV * y]), h));
-    v = sub(v, dvd(mul(fac(0, 1), fb[(x + 1) + kSV * y]), h));
-    v = add(v, dvd(mul(fac(1, -1), fb[kSSV + x + kSV * y]), h));
-    v = sub(v, dvd(mul(fac(1, 1), fb[kSSV + x + kSV * (y + 1)]), h));
-    dne[o] = v;
+// One 256-thread CTA a block, a thread a cell, all of its values loaded before the
+// chemistry: grid-strided cells with ten divisions each took 202 us on 51877 blocks (75 us
+// of bytes); the factors' shared quotient and div_by leave three divisions and two exp.
+__global__ void __launch_bounds__(256)
+k_streamer_rates(double *__restrict__ dne, double *__restrict__ dni, const double *__restrict__ ne,
+                 const double *__restrict__ eabs, const double *__restrict__ flux, const int2 *__restrict__ leaf,
+                 const int4 *__restrict__ info, CellSize cs, int geom, srmg_transport tr) {
+  const int2 lb = leaf[blockIdx.x];
+  const int X = lb.x;
+  const int4 bi = info[X];
+  const int x = 2 + (threadIdx.x & 15), y = 2 + (threadIdx.x >> 4);
+  const int64_t o = (int64_t)X * kSS + x + kS * y;
+  const double *fb = flux + (int64_t)X * 2 * kSSV;
+  const double n1 = ne[o], E = eabs[o];
+  const double rl = fb[x + kSV * y], ru = fb[(x + 1) + kSV * y];
+  const double zl = fb[kSSV + x + kSV * y], zu = fb[kSSV + x + kSV * (y + 1)];
+  if ((bi.z & 15) != 0) return;  // not a leaf block: its values were loaded in vain
+  const double h = mul(cs.h1, pow2(1 - lb.y)), rh = mul(cs.rh1, pow2(lb.y - 1));
+  // NetIonization, MinimalTransportModel: mobility mu, townsend ai exp(-Ei / E),
+  // attachment aa exp(-Ea / E)
+  const double pre = mul(mul(mul(tr.mu, E), n1), mul(tr.ai, exp(dvd(-tr.Ei, E))));
+  const double post = mul(mul(mul(-tr.mu, E), n1), mul(tr.aa, exp(dvd(-tr.Ea, E))));
+  const double chem = add(pre, post);
+  dni[o] = chem;
+  // factor(geom, J, +-e_dim) = |1 +- 1 / (2 J - 1)| along the radial dimension, else 1
+  double lo = 1.0, up = 1.0;
+  if (geom != 0) {
+    const int64_t J = geom == 1 ? gidx(bi.x, x) : gidx(bi.y, y);
+    const double q = dvd(1.0, (double)(2 * J - 1));
+    lo = fabs(sub(1.0, q));
+    up = fabs(add(1.0, q));
   }
+  const bool r1 = geom == 1, r2 = geom == 2;
+  double v = chem;
+  v = add(v, div_by(r1 ? mul(lo, rl) : rl, h, rh));
+  v = sub(v, div_by(r1 ? mul(up, ru) : ru, h, rh));
+  v = add(v, div_by(r2 ? mul(lo, zl) : zl, h, rh));
+  v = sub(v, div_by(r2 ? mul(up, zu) : zu, h, rh));
+  dne[o] = v;
 }
 
 __global__ void k_init_min(double *m) { *m = INFINITY; }
@@ -210,6 +252,13 @@ __global__ void k_ssprk3(double *__restrict__ out, const double *__restrict__ n,
 int grid_of(int64_t work, int threads, int cap) {
   const int64_t g = (work + threads - 1) / threads;
   return (int)std::max<int64_t>(1, std::min<int64_t>(g, cap));
+}
+
+// Plain double operations, one rounding each (no contraction on the host side).
+CellSize cell_size(double h, const srmg_transport &tr) {
+  volatile double hh = h * h;
+  volatile double q = hh / tr.D;
+  return CellSize{h, 1.0 / h, q / 4.0};
 }
 
 int check_transport(srmg_ctx *ctx, const srmg_transport *tr, const char *who) {
@@ -235,14 +284,17 @@ extern "C" int srmg_streamer_flux_dev(srmg_ctx *ctx, double *flux, double *maxdt
     ctx->launches++;
   }
   if (ctx->nleaf > 0) {
-    k_streamer_flux<<<std::min(ctx->nleaf, 148 * 8), 256, 0, ctx->stream>>>(
-        flux, maxdt_blk, maxdt_min, ne, e, eabs, ctx->d_leaf, ctx->nleaf, ctx->d_info, h, *tr);
+    if (maxdt_blk)
+      k_streamer_flux<true><<<ctx->nleaf, 256, 0, ctx->stream>>>(flux, maxdt_blk, maxdt_min, ne, e, eabs, ctx->d_leaf,
+                                                                ctx->d_info, cell_size(h, *tr), *tr);
+    else
+      k_streamer_flux<false><<<ctx->nleaf, 256, 0, ctx->stream>>>(flux, nullptr, maxdt_min, ne, e, eabs, ctx->d_leaf,
+                                                                 ctx->d_info, cell_size(h, *tr), *tr);
     ctx->launches++;
   }
-  for (int l = 2; l <= ctx->nlev; l++) {
-    if (!((ctx->refbnd_levels >> l) & 1)) continue;
-    const int n = ctx->nblk_host[l - 1];
-    k_restrict_flux<<<grid_of((int64_t)n * 32, 256, 148 * 8), 256, 0, ctx->stream>>>(flux, ctx->lv[l - 1].view(l));
+  if (ctx->refbnd_levels) {
+    k_restrict_flux<<<(unsigned)((ctx->max_blk * 32 + 255) / 256), 256, 0, ctx->stream>>>(flux, ctx->d_faceb,
+                                                                                          ctx->d_info, ctx->max_blk);
     ctx->launches++;
   }
   CK(cudaGetLastError());
@@ -258,8 +310,8 @@ extern "C" int srmg_streamer_rates_dev(srmg_ctx *ctx, double *dne, double *dni, 
   if (geom < 0 || geom > 2) return fail(ctx, SRMG_ERR_BADARG, "srmg_streamer_rates_dev: geom must be 0, 1 or 2");
   RC(check_transport(ctx, tr, "srmg_streamer_rates_dev"));
   if (ctx->nleaf > 0) {
-    k_streamer_rates<<<grid_of((int64_t)ctx->nleaf * 256, 256, 148 * 16), 256, 0, ctx->stream>>>(
-        dne, dni, ne, eabs, flux, ctx->d_leaf, ctx->nleaf, ctx->d_info, h, geom, *tr);
+    k_streamer_rates<<<ctx->nleaf, 256, 0, ctx->stream>>>(dne, dni, ne, eabs, flux, ctx->d_leaf, ctx->d_info, cell_size(h, *tr), geom,
+                                                          *tr);
     ctx->launches++;
   }
   CK(cudaGetLastError());
