@@ -92,6 +92,24 @@ __device__ __forceinline__ double div_by(double a, double d, double rd) {
   return fma(fma(-q, d, a), rd, q);
 }
 
+// Whole-tile copies global -> shared by the CTA's threads (cp.async, CH = 16 or 8 bytes a
+// copy: 16 needs 16-byte aligned fields), for kernels that stream blocks through a ring of
+// tiles: a later block's tiles are in flight while one is worked on, without registers
+// to hold them.  Every thread commits one group per ring step, empty or not, and waits
+// with cp_async_wait<groups that may still be in flight>.
+template <int CH>
+__device__ __forceinline__ void cp_tile(double *dst, const double *src, int n) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  for (int i = threadIdx.x; i < n * 8 / CH; i += blockDim.x) {
+    const char *s = reinterpret_cast<const char *>(src) + i * CH;
+    if (CH == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + i * CH), "l"(s) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + i * CH), "l"(s) : "memory");
+  }
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // Stencil weights of cell (x, y) of a block at 1-based coords (cr, cz).
 template <typename T>
 struct W5 { T zm, rm, rp, zp; };

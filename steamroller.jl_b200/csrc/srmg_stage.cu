@@ -6,6 +6,7 @@
 //   * electric_field! (src/multigrid.jl:421-449) with a constant background field.
 // For order-2 discretisations rhs_level! (src/multigrid.jl:363-388) is the identity,
 // so the net charge itself is the solve's right-hand side.
+#include <algorithm>
 #include <cmath>
 
 #include "srmg_ctx.h"
@@ -64,39 +65,54 @@ __global__ void __launch_bounds__(256) k_netcharge(double *__restrict__ q, const
 // multiply-add; the quarter is exact either way), as in the reference.  One launch for
 // all levels (info: block coordinates, child mask, level, 0 for no block): a launch per
 // level was 287 us on 51877 blocks, 650 MB of traffic (99 us).
-__global__ void __launch_bounds__(256) k_efield(double *__restrict__ e, double *__restrict__ eabs,
-                                                const double *__restrict__ u, const int4 *__restrict__ info,
-                                                double h1, double rh1, double e0r, double e0z) {
-  const int64_t X = blockIdx.x;
+// CTAs stream blocks through a ring of u tiles (cp.async, three blocks ahead).
+constexpr int kEfRing = 4;
+template <int CH>
+__global__ void __launch_bounds__(256, 5) k_efield(double *__restrict__ e, double *__restrict__ eabs,
+                                                   const double *__restrict__ u, const int4 *__restrict__ info,
+                                                   int nblk, double h1, double rh1, double e0r, double e0z) {
+  __shared__ __align__(16) double tile[kEfRing][kSS];
   const int lane = threadIdx.x & 31, cx = lane & 15, p = threadIdx.x >> 5;
   const int x = 2 + cx, y0 = 2 + 2 * p, y = y0 + (lane >> 4);
-  const double *ub = u + X * kSS;
-  double *eb = e + X * (2 * kSSV);
-  const double uc = ub[x + kS * y], ul = ub[x - 1 + kS * y], ud = ub[x + kS * (y - 1)];
   const bool ez = lane < 16, er = lane == 16 || lane == 17;
-  const int eo = ez ? x + kS * (y0 + 2) : 18 + kS * (y0 + (lane & 1));
-  double xc = 0.0, xl = 0.0;
-  if (ez || er) {
-    xc = ub[eo];
-    xl = ub[eo - (ez ? kS : 1)];
+  // the lane's extra face (any face of the tile where it has none)
+  const int eo = ez ? x + kS * (y0 + 2) : 18 + kS * (y0 + (lane & 1)), el = eo - (ez ? kS : 1);
+  auto fetch = [&](int j) {
+    const int64_t X = blockIdx.x + (int64_t)j * gridDim.x;
+    if (X < nblk) cp_tile<CH>(tile[j % kEfRing], u + X * kSS, kSS);
+    cp_async_commit();
+  };
+  for (int j = 0; j < kEfRing - 1; ++j) fetch(j);
+  for (int j = 0;; ++j) {
+    const int64_t X = blockIdx.x + (int64_t)j * gridDim.x;
+    if (X >= nblk) break;
+    const int level = info[X].w;
+    cp_async_wait<kEfRing - 2>();
+    __syncthreads();  // the tile is here, and no thread reads the last one's any more
+    fetch(j + kEfRing - 1);
+    if (level == 0) continue;  // no such block
+    const double *ub = tile[j % kEfRing];
+    double *eb = e + X * (2 * kSSV);
+    const double hl = __dmul_rn(h1, __hiloint2double((1024 - level) << 20, 0));   // h / 2^(level - 1)
+    const double rh = __dmul_rn(rh1, __hiloint2double((1022 + level) << 20, 0));  // its reciprocal
+    auto face = [&](double lo, double up, double e0) { return __dadd_rn(div_by(__dsub_rn(lo, up), hl, rh), e0); };
+    const int o = x + kS * y;
+    const double uc = ub[o];
+    const double fr0 = face(ub[o - 1], uc, e0r), fz0 = face(ub[o - kS], uc, e0z);
+    const double fx = face(ub[el], ub[eo], ez ? e0z : e0r);
+    eb[x + kSV * y] = fr0;
+    eb[kSSV + x + kSV * y] = fz0;
+    if (er) eb[18 + kSV * (y0 + (lane & 1))] = fx;
+    if (ez && p == 7) eb[kSSV + x + kSV * 18] = fx;
+    const unsigned all = 0xffffffffu;
+    const double nr = __shfl_down_sync(all, fr0, 1), xr = __shfl_sync(all, fx, 16 + (lane >> 4));
+    const double nz = __shfl_down_sync(all, fz0, 16), xz = __shfl_sync(all, fx, cx);
+    const double sr = __dadd_rn(fr0, cx == 15 ? xr : nr), sz = __dadd_rn(fz0, ez ? nz : xz);
+    double f2 = __dadd_rn(0.0, __dmul_rn(__dmul_rn(sr, sr), 0.25));
+    f2 = __dadd_rn(f2, __dmul_rn(__dmul_rn(sz, sz), 0.25));
+    eabs[X * kSS + o] = __dsqrt_rn(f2);
   }
-  const int level = info[X].w;
-  if (level == 0) return;  // no such block
-  const double hl = __dmul_rn(h1, __hiloint2double((1024 - level) << 20, 0));   // h / 2^(level - 1)
-  const double rh = __dmul_rn(rh1, __hiloint2double((1022 + level) << 20, 0));  // its reciprocal
-  auto face = [&](double lo, double up, double e0) { return __dadd_rn(div_by(__dsub_rn(lo, up), hl, rh), e0); };
-  const double fr0 = face(ul, uc, e0r), fz0 = face(ud, uc, e0z), fx = face(xl, xc, ez ? e0z : e0r);
-  eb[x + kSV * y] = fr0;
-  eb[kSSV + x + kSV * y] = fz0;
-  if (er) eb[18 + kSV * (y0 + (lane & 1))] = fx;
-  if (ez && p == 7) eb[kSSV + x + kSV * 18] = fx;
-  const unsigned all = 0xffffffffu;
-  const double nr = __shfl_down_sync(all, fr0, 1), xr = __shfl_sync(all, fx, 16 + (lane >> 4));
-  const double nz = __shfl_down_sync(all, fz0, 16), xz = __shfl_sync(all, fx, cx);
-  const double sr = __dadd_rn(fr0, cx == 15 ? xr : nr), sz = __dadd_rn(fz0, ez ? nz : xz);
-  double f2 = __dadd_rn(0.0, __dmul_rn(__dmul_rn(sr, sr), 0.25));
-  f2 = __dadd_rn(f2, __dmul_rn(__dmul_rn(sz, sz), 0.25));
-  eabs[X * kSS + x + kS * y] = __dsqrt_rn(f2);
+  cp_async_wait<0>();
 }
 
 }  // namespace
@@ -130,7 +146,9 @@ extern "C" int srmg_electric_field_dev(srmg_ctx *ctx, double *e, double *eabs, c
   if (!e || !eabs || !u || !e0) return fail(ctx, SRMG_ERR_BADARG, "srmg_electric_field: null argument");
   if (!(h > 0.0) || !std::isfinite(h)) return fail(ctx, SRMG_ERR_BADARG, "srmg_electric_field: h must be > 0");
   if (ctx->max_blk > 0) {
-    k_efield<<<(unsigned)ctx->max_blk, 256, 0, ctx->stream>>>(e, eabs, u, ctx->d_info, h, 1.0 / h, e0[0], e0[1]);
+    const int grid = (int)std::min<int64_t>(ctx->max_blk, 148 * 5);
+    const auto kern = (reinterpret_cast<uintptr_t>(u) & 15) == 0 ? k_efield<16> : k_efield<8>;
+    kern<<<grid, 256, 0, ctx->stream>>>(e, eabs, u, ctx->d_info, (int)ctx->max_blk, h, 1.0 / h, e0[0], e0[1]);
     ctx->launches++;
   }
   CK(cudaGetLastError());

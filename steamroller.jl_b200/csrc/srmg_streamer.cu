@@ -23,7 +23,9 @@
 // (src/blockfield.jl:84-95): 21 x 21 values per component, component d at offset 441 d,
 // 882 values per block; face (x, y) of component d (0-based local indices) is the face
 // between cell (x, y) - e_d and cell (x, y).
+#include <algorithm>
 #include <cmath>
+#include <initializer_list>
 
 #include "srmg_ctx.h"
 #include "srmg_internal.h"
@@ -115,53 +117,83 @@ __device__ __forceinline__ double face_flux(const FaceIn &f, const srmg_transpor
   return add(F, div_by(mul(tr.D, sub(f.n[1], f.n[2])), h, rh));
 }
 
-// flux! (Koren) on the leaf blocks, one 256-thread CTA a block: a thread takes its cell's
-// lower face along each dimension, the first warp also the 32 last faces (x = 18 or y = 18).
-// Latency and the fp64 pipe bound it (a face is ~40 fp64 operations on 7 loaded values, and
-// an fp64 instruction takes two issue slots): a thread's loads are issued together and
-// before the block's leaf flag is known, the divisions by h, 3 and 6 go through their
-// reciprocals, the time-step quotients are only formed where they can lower the minimum
-// (BLK off: seeded with the minimum so far over all blocks), and without BLK the warps
-// never meet.  544 faces strided over 256 threads with eight divisions each and two
-// barriers a block took 445 us on 51877 blocks.  ne needs 2 ghost layers, eabs 1.  BLK:
-// write each block's own minimum to maxdt_blk.
-template <bool BLK>
-__global__ void __launch_bounds__(256, 4)
+// The blocks a CTA streams: list entries blockIdx.x, + gridDim.x, ...; a ring of kRing tile
+// sets in shared memory, the next kRing - 1 blocks' tiles in flight.
+constexpr int kRing = 3;
+constexpr int kTileSet = 2 * kSS + 2 * kSSV;  // n_e, |E| and a vector field, whole blocks
+constexpr int kTileSetBytes = kTileSet * (int)sizeof(double);
+constexpr int kFluxThreads = 288;             // 9 warps: 17 x 16 faces per dimension, one each a thread
+constexpr int kFluxFaces = (kM + 1) * kM;
+
+template <int CH>
+__device__ __forceinline__ void load_set(double *sm, const double *a, const double *b, const double *vec, int X) {
+  cp_tile<CH>(sm, a + (int64_t)X * kSS, kSS);
+  cp_tile<CH>(sm + kSS, b + (int64_t)X * kSS, kSS);
+  cp_tile<CH>(sm + 2 * kSS, vec + (int64_t)X * 2 * kSSV, 2 * kSSV);
+}
+
+// flux! (Koren) on the leaf blocks.  CTAs stream blocks: n_e, |E| and E tiles arrive by cp.async
+// two blocks ahead, 272 threads take one face of each dimension.  A face is ~40 fp64
+// operations (an fp64 instruction takes two issue slots) on 7 values: the divisions by h,
+// 3 and 6 go through their reciprocals, and the time-step quotients are only formed where
+// they can lower the minimum so far (over the thread's blocks; with BLK over the block, whose
+// own minimum goes to maxdt_blk).  Bound by DRAM (740 MB on 51877 blocks, 113 us) and the
+// fp64 pipe; 544 faces strided over 256 threads with eight divisions each, loads issued as
+// needed and two barriers a block took 445 us.  ne needs 2 ghost layers, eabs 1.
+template <bool BLK, int CH>
+__global__ void __launch_bounds__(kFluxThreads, 4)
 k_streamer_flux(double *__restrict__ flux, double *__restrict__ maxdt_blk, double *maxdt_min,
                 const double *__restrict__ ne, const double *__restrict__ e, const double *__restrict__ eabs,
-                const int2 *__restrict__ leaf, const int4 *__restrict__ info, CellSize cs, srmg_transport tr) {
-  const int2 lb = leaf[blockIdx.x];
-  const int X = lb.x;
-  const int x = 2 + (threadIdx.x & 15), y = 2 + (threadIdx.x >> 4);
-  const double *n = ne + (int64_t)X * kSS, *ea = eabs + (int64_t)X * kSS, *eb = e + (int64_t)X * 2 * kSSV;
-  double *fb = flux + (int64_t)X * 2 * kSSV;
-  const FaceIn f0 = load_face(eb, ea, n, 0, x, y), f1 = load_face(eb, ea, n, 1, x, y);
-  double seed = INFINITY;
-  if (!BLK && maxdt_min) seed = *reinterpret_cast<volatile double *>(maxdt_min);
-  if (!leaf_block(info, X)) return;  // uniform per CTA
-  const double h = mul(cs.h1, pow2(1 - lb.y)), rh = mul(cs.rh1, pow2(lb.y - 1));  // h /= 1 << (level - 1)
+                const int2 *__restrict__ leaf, int nleaf, const int4 *__restrict__ info, CellSize cs,
+                srmg_transport tr) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ double s_min[kFluxThreads / 32];
+  const int t = threadIdx.x, rx = 2 + t % (kM + 1), ry = 2 + t / (kM + 1), zx = 2 + (t & 15), zy = 2 + (t >> 4);
+  const bool act = t < kFluxFaces;
   const double r3 = 1.0 / 3.0, r6 = 1.0 / 6.0;
-  double md = fmin(seed, mul(cs.dt1, pow2(2 - 2 * lb.y)));
-  if (threadIdx.x < 32) {
-    const int d = threadIdx.x >> 4, c = threadIdx.x & 15, fx = d ? 2 + c : 18, fy = d ? 18 : 2 + c;
-    fb[d * kSSV + fx + kSV * fy] = face_flux(load_face(eb, ea, n, d, fx, fy), tr, h, rh, r3, r6, md);
+  double md = INFINITY;
+  auto fetch = [&](int j) {
+    const int k = blockIdx.x + j * gridDim.x;
+    if (k < nleaf) load_set<CH>(sm + (j % kRing) * kTileSet, ne, eabs, e, leaf[k].x);
+    cp_async_commit();
+  };
+  for (int j = 0; j < kRing - 1; ++j) fetch(j);
+  for (int j = 0;; ++j) {
+    const int k = blockIdx.x + j * gridDim.x;
+    if (k >= nleaf) break;
+    const int2 lb = leaf[k];
+    const int X = lb.x;
+    const bool is_leaf = leaf_block(info, X);  // uniform per CTA
+    cp_async_wait<kRing - 2>();
+    __syncthreads();  // the block's tiles are here, and no thread reads the tiles of the last one any more
+    fetch(j + kRing - 1);
+    if (!is_leaf) continue;
+    const double *n = sm + (j % kRing) * kTileSet, *ea = n + kSS, *eb = n + 2 * kSS;
+    double *fb = flux + (int64_t)X * 2 * kSSV;
+    const double h = mul(cs.h1, pow2(1 - lb.y)), rh = mul(cs.rh1, pow2(lb.y - 1));  // h /= 1 << (level - 1)
+    const double dt = mul(cs.dt1, pow2(2 - 2 * lb.y));
+    md = BLK ? fmin(INFINITY, dt) : fmin(md, dt);
+    if (act) {
+      fb[rx + kSV * ry] = face_flux(load_face(eb, ea, n, 0, rx, ry), tr, h, rh, r3, r6, md);
+      fb[kSSV + zx + kSV * zy] = face_flux(load_face(eb, ea, n, 1, zx, zy), tr, h, rh, r3, r6, md);
+    }
+    if (BLK) {
+      double m = md;
+      for (int off = 16; off > 0; off >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, off));
+      if ((t & 31) == 0) s_min[t >> 5] = m;
+      __syncthreads();
+      if (t == 0) {
+        for (int w = 1; w < kFluxThreads / 32; ++w) m = fmin(m, s_min[w]);
+        maxdt_blk[X] = m;
+        if (maxdt_min) atomic_min_nonneg(maxdt_min, m);
+      }
+    }
   }
-  fb[x + kSV * y] = face_flux(f0, tr, h, rh, r3, r6, md);
-  fb[kSSV + x + kSV * y] = face_flux(f1, tr, h, rh, r3, r6, md);
-  if (!BLK && !maxdt_min) return;
-  for (int off = 16; off > 0; off >>= 1) md = fmin(md, __shfl_xor_sync(0xffffffffu, md, off));
-  if (!BLK) {
-    if ((threadIdx.x & 31) == 0 && md != seed) atomic_min_nonneg(maxdt_min, md);
-    return;
-  }
-  __shared__ double s_min[8];
-  if ((threadIdx.x & 31) == 0) s_min[threadIdx.x >> 5] = md;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m = s_min[0];
-    for (int w = 1; w < 8; ++w) m = fmin(m, s_min[w]);
-    maxdt_blk[X] = m;
-    if (maxdt_min) atomic_min_nonneg(maxdt_min, m);
+  cp_async_wait<0>();
+  if constexpr (!BLK) {
+    if (!maxdt_min) return;
+    for (int off = 16; off > 0; off >>= 1) md = fmin(md, __shfl_xor_sync(0xffffffffu, md, off));
+    if ((t & 31) == 0 && md < INFINITY) atomic_min_nonneg(maxdt_min, md);
   }
 }
 
@@ -192,45 +224,61 @@ __global__ void k_restrict_flux(double *__restrict__ flux, const int4 *__restric
 // dni = pre + post; dne = (((pre + post) + lower-r) - upper-r) + lower-z) - upper-z,
 // each face term (factor F) / h, factor = |1 + delta / (2 J - 1)| along the radial
 // dimension (1 along the others and in Cartesian geometry).
-// One 256-thread CTA a block, a thread a cell, all of its values loaded before the
-// chemistry: grid-strided cells with ten divisions each took 202 us on 51877 blocks (75 us
-// of bytes); the factors' shared quotient and div_by leave three divisions and two exp.
-__global__ void __launch_bounds__(256)
+// CTAs stream blocks as in k_streamer_flux, a thread a cell: grid-strided cells with ten
+// divisions each, loads issued as needed, took 202 us on 51877 blocks (676 MB, 103 us); the
+// factors' shared quotient and div_by leave three divisions and two exp, which the fp64
+// pipe now shares the bound with.
+template <int CH>
+__global__ void __launch_bounds__(256, 4)
 k_streamer_rates(double *__restrict__ dne, double *__restrict__ dni, const double *__restrict__ ne,
                  const double *__restrict__ eabs, const double *__restrict__ flux, const int2 *__restrict__ leaf,
-                 const int4 *__restrict__ info, CellSize cs, int geom, srmg_transport tr) {
-  const int2 lb = leaf[blockIdx.x];
-  const int X = lb.x;
-  const int4 bi = info[X];
-  const int x = 2 + (threadIdx.x & 15), y = 2 + (threadIdx.x >> 4);
-  const int64_t o = (int64_t)X * kSS + x + kS * y;
-  const double *fb = flux + (int64_t)X * 2 * kSSV;
-  const double n1 = ne[o], E = eabs[o];
-  const double rl = fb[x + kSV * y], ru = fb[(x + 1) + kSV * y];
-  const double zl = fb[kSSV + x + kSV * y], zu = fb[kSSV + x + kSV * (y + 1)];
-  if ((bi.z & 15) != 0) return;  // not a leaf block: its values were loaded in vain
-  const double h = mul(cs.h1, pow2(1 - lb.y)), rh = mul(cs.rh1, pow2(lb.y - 1));
-  // NetIonization, MinimalTransportModel: mobility mu, townsend ai exp(-Ei / E),
-  // attachment aa exp(-Ea / E)
-  const double pre = mul(mul(mul(tr.mu, E), n1), mul(tr.ai, exp(dvd(-tr.Ei, E))));
-  const double post = mul(mul(mul(-tr.mu, E), n1), mul(tr.aa, exp(dvd(-tr.Ea, E))));
-  const double chem = add(pre, post);
-  dni[o] = chem;
-  // factor(geom, J, +-e_dim) = |1 +- 1 / (2 J - 1)| along the radial dimension, else 1
-  double lo = 1.0, up = 1.0;
-  if (geom != 0) {
-    const int64_t J = geom == 1 ? gidx(bi.x, x) : gidx(bi.y, y);
-    const double q = dvd(1.0, (double)(2 * J - 1));
-    lo = fabs(sub(1.0, q));
-    up = fabs(add(1.0, q));
+                 int nleaf, const int4 *__restrict__ info, CellSize cs, int geom, srmg_transport tr) {
+  extern __shared__ __align__(16) double sm[];
+  const int x = 2 + (threadIdx.x & 15), y = 2 + (threadIdx.x >> 4), o = x + kS * y;
+  auto fetch = [&](int j) {
+    const int k = blockIdx.x + j * gridDim.x;
+    if (k < nleaf) load_set<CH>(sm + (j % kRing) * kTileSet, ne, eabs, flux, leaf[k].x);
+    cp_async_commit();
+  };
+  for (int j = 0; j < kRing - 1; ++j) fetch(j);
+  for (int j = 0;; ++j) {
+    const int k = blockIdx.x + j * gridDim.x;
+    if (k >= nleaf) break;
+    const int2 lb = leaf[k];
+    const int64_t X = lb.x;
+    const int4 bi = info[X];
+    cp_async_wait<kRing - 2>();
+    __syncthreads();  // as in k_streamer_flux
+    fetch(j + kRing - 1);
+    if ((bi.z & 15) != 0) continue;  // not a leaf block
+    const double *s = sm + (j % kRing) * kTileSet, *fb = s + 2 * kSS;
+    const double n1 = s[o], E = s[kSS + o];
+    const double rl = fb[x + kSV * y], ru = fb[(x + 1) + kSV * y];
+    const double zl = fb[kSSV + x + kSV * y], zu = fb[kSSV + x + kSV * (y + 1)];
+    const double h = mul(cs.h1, pow2(1 - lb.y)), rh = mul(cs.rh1, pow2(lb.y - 1));
+    // NetIonization, MinimalTransportModel: mobility mu, townsend ai exp(-Ei / E),
+    // attachment aa exp(-Ea / E)
+    const double pre = mul(mul(mul(tr.mu, E), n1), mul(tr.ai, exp(dvd(-tr.Ei, E))));
+    const double post = mul(mul(mul(-tr.mu, E), n1), mul(tr.aa, exp(dvd(-tr.Ea, E))));
+    const double chem = add(pre, post);
+    dni[X * kSS + o] = chem;
+    // factor(geom, J, +-e_dim) = |1 +- 1 / (2 J - 1)| along the radial dimension, else 1
+    double lo = 1.0, up = 1.0;
+    if (geom != 0) {
+      const int64_t J = geom == 1 ? gidx(bi.x, x) : gidx(bi.y, y);
+      const double q = dvd(1.0, (double)(2 * J - 1));
+      lo = fabs(sub(1.0, q));
+      up = fabs(add(1.0, q));
+    }
+    const bool r1 = geom == 1, r2 = geom == 2;
+    double v = chem;
+    v = add(v, div_by(r1 ? mul(lo, rl) : rl, h, rh));
+    v = sub(v, div_by(r1 ? mul(up, ru) : ru, h, rh));
+    v = add(v, div_by(r2 ? mul(lo, zl) : zl, h, rh));
+    v = sub(v, div_by(r2 ? mul(up, zu) : zu, h, rh));
+    dne[X * kSS + o] = v;
   }
-  const bool r1 = geom == 1, r2 = geom == 2;
-  double v = chem;
-  v = add(v, div_by(r1 ? mul(lo, rl) : rl, h, rh));
-  v = sub(v, div_by(r1 ? mul(up, ru) : ru, h, rh));
-  v = add(v, div_by(r2 ? mul(lo, zl) : zl, h, rh));
-  v = sub(v, div_by(r2 ? mul(up, zu) : zu, h, rh));
-  dne[o] = v;
+  cp_async_wait<0>();
 }
 
 __global__ void k_init_min(double *m) { *m = INFINITY; }
@@ -252,6 +300,12 @@ __global__ void k_ssprk3(double *__restrict__ out, const double *__restrict__ n,
 int grid_of(int64_t work, int threads, int cap) {
   const int64_t g = (work + threads - 1) / threads;
   return (int)std::max<int64_t>(1, std::min<int64_t>(g, cap));
+}
+
+bool aligned16(std::initializer_list<const void *> ps) {
+  uintptr_t v = 0;
+  for (const void *p : ps) v |= reinterpret_cast<uintptr_t>(p);
+  return (v & 15) == 0;
 }
 
 // Plain double operations, one rounding each (no contraction on the host side).
@@ -284,12 +338,12 @@ extern "C" int srmg_streamer_flux_dev(srmg_ctx *ctx, double *flux, double *maxdt
     ctx->launches++;
   }
   if (ctx->nleaf > 0) {
-    if (maxdt_blk)
-      k_streamer_flux<true><<<ctx->nleaf, 256, 0, ctx->stream>>>(flux, maxdt_blk, maxdt_min, ne, e, eabs, ctx->d_leaf,
-                                                                ctx->d_info, cell_size(h, *tr), *tr);
-    else
-      k_streamer_flux<false><<<ctx->nleaf, 256, 0, ctx->stream>>>(flux, nullptr, maxdt_min, ne, e, eabs, ctx->d_leaf,
-                                                                 ctx->d_info, cell_size(h, *tr), *tr);
+    const bool al = aligned16({flux, ne, e, eabs});
+    const auto kern = maxdt_blk ? (al ? k_streamer_flux<true, 16> : k_streamer_flux<true, 8>)
+                                : (al ? k_streamer_flux<false, 16> : k_streamer_flux<false, 8>);
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing * kTileSetBytes));
+    kern<<<std::min(ctx->nleaf, 148 * 4), kFluxThreads, kRing * kTileSetBytes, ctx->stream>>>(
+        flux, maxdt_blk, maxdt_min, ne, e, eabs, ctx->d_leaf, ctx->nleaf, ctx->d_info, cell_size(h, *tr), *tr);
     ctx->launches++;
   }
   if (ctx->refbnd_levels) {
@@ -310,8 +364,10 @@ extern "C" int srmg_streamer_rates_dev(srmg_ctx *ctx, double *dne, double *dni, 
   if (geom < 0 || geom > 2) return fail(ctx, SRMG_ERR_BADARG, "srmg_streamer_rates_dev: geom must be 0, 1 or 2");
   RC(check_transport(ctx, tr, "srmg_streamer_rates_dev"));
   if (ctx->nleaf > 0) {
-    k_streamer_rates<<<ctx->nleaf, 256, 0, ctx->stream>>>(dne, dni, ne, eabs, flux, ctx->d_leaf, ctx->d_info, cell_size(h, *tr), geom,
-                                                          *tr);
+    const auto kern = aligned16({ne, eabs, flux}) ? k_streamer_rates<16> : k_streamer_rates<8>;
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing * kTileSetBytes));
+    kern<<<std::min(ctx->nleaf, 148 * 4), 256, kRing * kTileSetBytes, ctx->stream>>>(
+        dne, dni, ne, eabs, flux, ctx->d_leaf, ctx->nleaf, ctx->d_info, cell_size(h, *tr), geom, *tr);
     ctx->launches++;
   }
   CK(cudaGetLastError());
