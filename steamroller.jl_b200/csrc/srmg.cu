@@ -731,7 +731,7 @@ int srmg::L_fill_ghost(srmg_ctx *ctx, T *u, int l, const Signs &sg, int mask) {
     // star faces only: the three passes touch disjoint cells and read none of each
     // other's results, so one launch does them all
     if (seq_push<T>(ctx, SEQ_FILL, mask, 0, u, nullptr, nullptr, L.view(l), nullptr, &sg)) return SRMG_OK;
-    k_fill_ghost<T><<<gf, threads, 0, ctx->stream>>>(u, L.view(l), sg, mask);
+    launch_pdl(k_fill_ghost<T>, gf, threads, 0, ctx->stream, u, L.view(l), sg, mask);
     ctx->launches++;
     return SRMG_OK;
   }
@@ -741,7 +741,7 @@ int srmg::L_fill_ghost(srmg_ctx *ctx, T *u, int l, const Signs &sg, int mask) {
   // ghost it mirrors itself, fill_corner_cell); interpolation follows on its own.
   if ((mask & 3) == 3) {
     if (!seq_push<T>(ctx, SEQ_FILL, 3, 0, u, nullptr, nullptr, L.view(l), nullptr, &sg)) {
-      k_fill_ghost<T><<<gf, threads, 0, ctx->stream>>>(u, L.view(l), sg, 3);
+      launch_pdl(k_fill_ghost<T>, gf, threads, 0, ctx->stream, u, L.view(l), sg, 3);
       ctx->launches++;
     }
     mask &= ~3;
@@ -749,7 +749,7 @@ int srmg::L_fill_ghost(srmg_ctx *ctx, T *u, int l, const Signs &sg, int mask) {
   for (int phase = 1; phase <= 4; phase <<= 1) {
     if (!(mask & phase)) continue;
     if (seq_push<T>(ctx, SEQ_FILL, phase, 0, u, nullptr, nullptr, L.view(l), nullptr, &sg)) continue;
-    k_fill_ghost<T><<<gf, threads, 0, ctx->stream>>>(u, L.view(l), sg, phase);
+    launch_pdl(k_fill_ghost<T>, gf, threads, 0, ctx->stream, u, L.view(l), sg, phase);
     ctx->launches++;
   }
   return SRMG_OK;
@@ -923,14 +923,12 @@ int srmg::L_gs_colour(srmg_ctx *ctx, T *u, const T *b, int l, const OpParams<T> 
   if (p.op == SRMG_OP_LAPLACIAN4) {
     // FourColors{parity >> 1, parity & 1}
     if (seq_push<T>(ctx, SEQ_GS4, parity >> 1, parity & 1, u, b, nullptr, L.view(l), &p, nullptr)) return SRMG_OK;
-    k_gs4<T><<<grid_for((int64_t)L.nblk * 64, threads, kGridCap), threads, 0, ctx->stream>>>(
-        u, b, L.view(l), p, parity >> 1, parity & 1);
+    launch_pdl(k_gs4<T>, grid_for((int64_t)L.nblk * 64, threads, kGridCap), threads, 0, ctx->stream, u, b, L.view(l), p, parity >> 1, parity & 1);
     ctx->launches++;
     return SRMG_OK;
   }
   if (seq_push<T>(ctx, SEQ_GS_COLOUR, parity, 0, u, b, nullptr, L.view(l), &p, nullptr)) return SRMG_OK;
-  k_gs_colour<T><<<grid_for((int64_t)L.nblk * 128, threads, kGridCap), threads, 0, ctx->stream>>>(
-      u, b, L.view(l), p, wtab<T>(ctx), parity);
+  launch_pdl(k_gs_colour<T>, grid_for((int64_t)L.nblk * 128, threads, kGridCap), threads, 0, ctx->stream, u, b, L.view(l), p, wtab<T>(ctx), parity);
   ctx->launches++;
   return SRMG_OK;
 }
@@ -944,11 +942,9 @@ static int L_gs_colour_push(srmg_ctx *ctx, T *u, const T *b, int l, const OpPara
   unsigned sw = 0;  // entry + 1, two bits an entry (every entry is -1, 0 or 1 here)
   for (int i = 0; i < 9; i++) sw |= (unsigned)((int)sg.v[i] + 1) << (2 * i);
   if (p.op == SRMG_OP_LAPLACIAN4)
-    k_gs4_push<T><<<grid_for((int64_t)L.nblk * 64, threads, kGridCap), threads, 0, ctx->stream>>>(
-        u, b, L.view(l), p, parity >> 1, parity & 1, ctx->push_lv[l - 1], sw);
+    launch_pdl(k_gs4_push<T>, grid_for((int64_t)L.nblk * 64, threads, kGridCap), threads, 0, ctx->stream, u, b, L.view(l), p, parity >> 1, parity & 1, ctx->push_lv[l - 1], sw);
   else
-    k_gs_colour_push<T><<<grid_for((int64_t)L.nblk * 128, threads, kGridCap), threads, 0, ctx->stream>>>(
-        u, b, L.view(l), p, wtab<T>(ctx), parity, ctx->push_lv[l - 1], sw);
+    launch_pdl(k_gs_colour_push<T>, grid_for((int64_t)L.nblk * 128, threads, kGridCap), threads, 0, ctx->stream, u, b, L.view(l), p, wtab<T>(ctx), parity, ctx->push_lv[l - 1], sw);
   ctx->launches++;
   return SRMG_OK;
 }
@@ -987,8 +983,7 @@ int srmg::L_residual(srmg_ctx *ctx, T *r, const T *u, const T *b, int l, const O
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nblk == 0) return SRMG_OK;
   if (seq_push<T>(ctx, SEQ_RESIDUAL, 0, 0, r, u, b, L.view(l), &p, nullptr)) return SRMG_OK;
-  k_residual<T><<<grid_for((int64_t)L.nblk * 256, 256, kGridCap), 256, 0, ctx->stream>>>(
-      r, u, b, L.view(l), p, wtab<T>(ctx));
+  launch_pdl(k_residual<T>, grid_for((int64_t)L.nblk * 256, 256, kGridCap), 256, 0, ctx->stream, r, u, b, L.view(l), p, wtab<T>(ctx));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -998,8 +993,7 @@ int srmg::L_postrestrict(srmg_ctx *ctx, T *bf, const T *u, const T *r, int l, co
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nch == 0) return SRMG_OK;
   if (seq_push<T>(ctx, SEQ_POSTRESTRICT, 0, 0, bf, u, r, L.view(l), &pc, nullptr)) return SRMG_OK;
-  k_postrestrict<T><<<grid_for((int64_t)L.nch * 64, 256, kGridCap), 256, 0, ctx->stream>>>(
-      bf, u, r, L.view(l), ctx->d_coord_of, pc, wtab<T>(ctx));
+  launch_pdl(k_postrestrict<T>, grid_for((int64_t)L.nch * 64, 256, kGridCap), 256, 0, ctx->stream, bf, u, r, L.view(l), ctx->d_coord_of, pc, wtab<T>(ctx));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -1009,7 +1003,7 @@ int srmg::L_restrict(srmg_ctx *ctx, T *u, int l) {
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nch == 0) return SRMG_OK;
   if (seq_push<T>(ctx, SEQ_RESTRICT, 0, 0, u, nullptr, nullptr, L.view(l), nullptr, nullptr)) return SRMG_OK;
-  k_restrict<T><<<grid_for((int64_t)L.nch * 64, 256, kGridCap), 256, 0, ctx->stream>>>(u, L.view(l));
+  launch_pdl(k_restrict<T>, grid_for((int64_t)L.nch * 64, 256, kGridCap), 256, 0, ctx->stream, u, L.view(l));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -1019,8 +1013,7 @@ int srmg::L_interp_add(srmg_ctx *ctx, T *u, const T *u1, int l) {
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nch == 0) return SRMG_OK;
   if (seq_push<T>(ctx, SEQ_INTERP_ADD, 0, 0, u, u1, nullptr, L.view(l), nullptr, nullptr)) return SRMG_OK;
-  k_interp_add<T><<<grid_for((int64_t)L.nch * 256, 256, kGridCap), 256, 0, ctx->stream>>>(
-      u, u1, L.view(l));
+  launch_pdl(k_interp_add<T>, grid_for((int64_t)L.nch * 256, 256, kGridCap), 256, 0, ctx->stream, u, u1, L.view(l));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -1030,8 +1023,7 @@ int srmg::L_copy(srmg_ctx *ctx, T *dst, const T *src, int l) {
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nblk == 0) return SRMG_OK;
   if (seq_push<T>(ctx, SEQ_COPY, 0, 0, dst, src, nullptr, L.view(l), nullptr, nullptr)) return SRMG_OK;
-  k_copy_level<T><<<grid_for((int64_t)L.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream>>>(
-      dst, src, L.view(l));
+  launch_pdl(k_copy_level<T>, grid_for((int64_t)L.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, dst, src, L.view(l));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -1041,8 +1033,7 @@ int srmg::L_diff(srmg_ctx *ctx, T *dst, const T *a1, const T *a2, int l) {
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nblk == 0) return SRMG_OK;
   if (seq_push<T>(ctx, SEQ_DIFF, 0, 0, dst, a1, a2, L.view(l), nullptr, nullptr)) return SRMG_OK;
-  k_diff_level<T><<<grid_for((int64_t)L.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream>>>(
-      dst, a1, a2, L.view(l));
+  launch_pdl(k_diff_level<T>, grid_for((int64_t)L.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, dst, a1, a2, L.view(l));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -1161,7 +1152,7 @@ int srmg::leafnorm_dev(srmg_ctx *ctx, const T *u, const T *b, double s, int op, 
     const double sl = level_scale(s, l);
     const OpParams<T> p = op_params<T>(op, geom, k2, sl, 1.0);
     const double wl = 1.0 / (double)((int64_t)1 << (2 * (l - 1)));
-    k_leafsq<T, NT><<<grids[l - 1], NT, 0, ctx->stream>>>(part + off, u, b, ctx->lv[l - 1].view(l), p,
+    launch_pdl(k_leafsq<T, NT>, grids[l - 1], NT, 0, ctx->stream, part + off, u, b, ctx->lv[l - 1].view(l), p,
                                                         wtab<T>(ctx), wl, mode);
     ctx->launches++;
     off += grids[l - 1];
@@ -1171,7 +1162,7 @@ int srmg::leafnorm_dev(srmg_ctx *ctx, const T *u, const T *b, double s, int op, 
     CK(cudaMemsetAsync(out, 0, sizeof(double), ctx->stream));
     return SRMG_OK;
   }
-  k_reduce_sqrt<1024><<<1, 1024, 0, ctx->stream>>>(out, part, total_parts);
+  launch_pdl(k_reduce_sqrt<1024>, 1, 1024, 0, ctx->stream, out, part, total_parts);
   ctx->launches++;
   return SRMG_OK;
 }
@@ -1482,7 +1473,7 @@ extern "C" int srmg_rhs_level_dev(srmg_ctx *ctx, double *q1, const double *q, in
   }
   const DevLevel &L = ctx->lv[level - 1];
   if (L.nblk > 0) {
-    k_rhs<double><<<grid_for((int64_t)L.nblk * 256, 256, kGridCap), 256, 0, ctx->stream>>>(q1, q, L.view(level),
+    launch_pdl(k_rhs<double>, grid_for((int64_t)L.nblk * 256, 256, kGridCap), 256, 0, ctx->stream, q1, q, L.view(level),
                                                                                          op, geom);
     ctx->launches++;
   }

@@ -342,21 +342,46 @@ __device__ __forceinline__ void d3_copy(double *__restrict__ dst, const double *
 }
 
 // The per-operation kernels: each one body, launched alone or run by the sequencer.
-__global__ void k3_fill(double *__restrict__ u, Level3View L, Signs27 sg, int phase) { d3_fill(u, L, sg, phase); }
-__global__ void k3_gs_rb(double *__restrict__ u, const double *__restrict__ b, Level3View L, Op3 p, int parity) { d3_gs_rb(u, b, L, p, parity); }
+__global__ void k3_fill(double *__restrict__ u, Level3View L, Signs27 sg, int phase) {
+  pdl_enter();
+  d3_fill(u, L, sg, phase);
+}
+__global__ void k3_gs_rb(double *__restrict__ u, const double *__restrict__ b, Level3View L, Op3 p, int parity) {
+  pdl_enter();
+  d3_gs_rb(u, b, L, p, parity);
+}
 __global__ void k3_gs_rb_push(double *__restrict__ u, const double *__restrict__ b, Level3View L, Op3 p, int parity,
                               Signs27 sg) {
+  pdl_enter();
   d3_gs_rb_push(u, b, L, p, parity, sg);
 }
-__global__ void k3_gs4(double *__restrict__ u, const double *__restrict__ b, Level3View L, Op3 p, int P1, int P2) { d3_gs4(u, b, L, p, P1, P2); }
+__global__ void k3_gs4(double *__restrict__ u, const double *__restrict__ b, Level3View L, Op3 p, int P1, int P2) {
+  pdl_enter();
+  d3_gs4(u, b, L, p, P1, P2);
+}
 __global__ void k3_residual(double *__restrict__ r, const double *__restrict__ u, const double *__restrict__ b,
-                            Level3View L, Op3 p) { d3_residual(r, u, b, L, p); }
+                            Level3View L, Op3 p) {
+  pdl_enter();
+  d3_residual(r, u, b, L, p);
+}
 __global__ void k3_postrestrict(double *__restrict__ bf, const double *__restrict__ u, const double *__restrict__ r,
-                                Level3View L, Op3 pc) { d3_postrestrict(bf, u, r, L, pc); }
-__global__ void k3_restrict(double *__restrict__ u, Level3View L) { d3_restrict(u, L); }
-__global__ void k3_interp_add(double *__restrict__ u, const double *__restrict__ u1, Level3View L) { d3_interp_add(u, u1, L); }
+                                Level3View L, Op3 pc) {
+  pdl_enter();
+  d3_postrestrict(bf, u, r, L, pc);
+}
+__global__ void k3_restrict(double *__restrict__ u, Level3View L) {
+  pdl_enter();
+  d3_restrict(u, L);
+}
+__global__ void k3_interp_add(double *__restrict__ u, const double *__restrict__ u1, Level3View L) {
+  pdl_enter();
+  d3_interp_add(u, u1, L);
+}
 __global__ void k3_copy(double *__restrict__ dst, const double *__restrict__ a1, const double *__restrict__ a2,
-                        Level3View L) { d3_copy(dst, a1, a2, L); }
+                        Level3View L) {
+  pdl_enter();
+  d3_copy(dst, a1, a2, L);
+}
 
 // Table-driven ghost pushes of a colour sweep (octrees other than StarStencil{3} at
 // order 2): off[bi*4096 + cell] .. off[bi*4096 + cell + 1] index ent = {the ghost's
@@ -383,6 +408,7 @@ __device__ __forceinline__ void push3(double *__restrict__ u, const PushView &pv
 // d3_gs_rb / d3_gs4 with the table pushes after each update.
 __global__ void k3_gs_rb_tpush(double *__restrict__ u, const double *__restrict__ b, Level3View L, Op3 p, int parity,
                                PushView pv, unsigned long long sg) {
+  pdl_enter();
   const int64_t total = (int64_t)L.nblk * (kM * kM * kM / 2);
   const double nwc = -(p.omega / p.diag);
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -402,6 +428,7 @@ __global__ void k3_gs_rb_tpush(double *__restrict__ u, const double *__restrict_
 
 __global__ void k3_gs4_push(double *__restrict__ u, const double *__restrict__ b, Level3View L, Op3 p, int P1, int P2,
                             PushView pv, unsigned long long sg) {
+  pdl_enter();
   const int64_t total = (int64_t)L.nblk * 1024;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int bi = (int)(t / 1024), c = (int)(t % 1024);
@@ -495,6 +522,7 @@ bool seq3_push(srmg_ctx *ctx, int kind, int i0, int i1, double *a, const double 
 // rhs! (src/multigrid.jl:363-388): identity at order 2, the 7-point right-hand side
 // (centre 6) / 12 at order 4 (src/laplacian.jl:322-337)
 __global__ void k3_rhs(double *__restrict__ q1, const double *__restrict__ q, Level3View L, int op) {
+  pdl_enter();
   const int64_t total = (int64_t)L.nblk * 4096;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int bi = (int)(t / 4096), c = (int)(t % 4096);
@@ -524,6 +552,7 @@ template <int NT>
 __global__ void __launch_bounds__(NT) k3_leafsq(double *__restrict__ part, const double *__restrict__ u,
                                                 const double *__restrict__ b, Level3View L, Op3 p, double wl,
                                                 int mode) {
+  pdl_enter();
   double acc = 0.0;
   const int64_t total = (int64_t)L.nblk * 4096;
   for (int64_t t = blockIdx.x * (int64_t)NT + threadIdx.x; t < total; t += (int64_t)gridDim.x * NT) {
@@ -575,13 +604,13 @@ int fill(srmg_ctx *ctx, double *u, int l, const Signs27 &sg, int mask) {
   if (!n) return SRMG_OK;
   if (!ctx->has_corners) {
     if (seq3_push(ctx, S3_FILL, mask, 0, u, nullptr, nullptr, view(ctx, l), nullptr, &sg)) return SRMG_OK;
-    k3_fill<<<grid3((int64_t)n * kGhost3, 256), 256, 0, ctx->stream>>>(u, view(ctx, l), sg, mask);
+    launch_pdl(k3_fill, grid3((int64_t)n * kGhost3, 256), 256, 0, ctx->stream, u, view(ctx, l), sg, mask);
     ctx->launches++;
     return SRMG_OK;
   }
   if ((mask & 3) == 3 && ctx->merge_fill) {
     if (!seq3_push(ctx, S3_FILL, 3, 0, u, nullptr, nullptr, view(ctx, l), nullptr, &sg)) {
-      k3_fill<<<grid3((int64_t)n * kGhost3, 256), 256, 0, ctx->stream>>>(u, view(ctx, l), sg, 3);
+      launch_pdl(k3_fill, grid3((int64_t)n * kGhost3, 256), 256, 0, ctx->stream, u, view(ctx, l), sg, 3);
       ctx->launches++;
     }
     mask &= ~3;
@@ -589,7 +618,7 @@ int fill(srmg_ctx *ctx, double *u, int l, const Signs27 &sg, int mask) {
   for (int phase = 1; phase <= 4; phase <<= 1) {
     if (!(mask & phase)) continue;
     if (seq3_push(ctx, S3_FILL, phase, 0, u, nullptr, nullptr, view(ctx, l), nullptr, &sg)) continue;
-    k3_fill<<<grid3((int64_t)n * kGhost3, 256), 256, 0, ctx->stream>>>(u, view(ctx, l), sg, phase);
+    launch_pdl(k3_fill, grid3((int64_t)n * kGhost3, 256), 256, 0, ctx->stream, u, view(ctx, l), sg, phase);
     ctx->launches++;
   }
   return SRMG_OK;
@@ -748,9 +777,9 @@ int gs_colour(srmg_ctx *ctx, double *u, const double *b, int l, const Op3 &p, in
   if (p.op != SRMG_OP_LAPLACIAN4 && seq3_push(ctx, S3_GS_RB, colour, 0, u, b, nullptr, view(ctx, l), &p, nullptr))
     return SRMG_OK;
   if (p.op == SRMG_OP_LAPLACIAN4)
-    k3_gs4<<<grid3((int64_t)n * 1024, 256), 256, 0, ctx->stream>>>(u, b, view(ctx, l), p, colour >> 1, colour & 1);
+    launch_pdl(k3_gs4, grid3((int64_t)n * 1024, 256), 256, 0, ctx->stream, u, b, view(ctx, l), p, colour >> 1, colour & 1);
   else
-    k3_gs_rb<<<grid3((int64_t)n * 2048, 256), 256, 0, ctx->stream>>>(u, b, view(ctx, l), p, colour);
+    launch_pdl(k3_gs_rb, grid3((int64_t)n * 2048, 256), 256, 0, ctx->stream, u, b, view(ctx, l), p, colour);
   ctx->launches++;
   return SRMG_OK;
 }
@@ -782,16 +811,16 @@ int gs_iter(srmg_ctx *ctx, double *u, const double *b, int l, const Op3 &p, int 
     for (int c = 0; c < ncol; ++c) {
       if (push) {
         if (!nb || seq3_push(ctx, S3_GS_RB_PUSH, c, 0, u, b, nullptr, view(ctx, l), &p, &sg)) continue;
-        k3_gs_rb_push<<<grid3((int64_t)nb * 2048, 256), 256, 0, ctx->stream>>>(u, b, view(ctx, l), p, c, sg);
+        launch_pdl(k3_gs_rb_push, grid3((int64_t)nb * 2048, 256), 256, 0, ctx->stream, u, b, view(ctx, l), p, c, sg);
         ctx->launches++;
         continue;
       }
       if (tpush && (i > 0 || c > 0)) {
         if (p.op == SRMG_OP_LAPLACIAN4)
-          k3_gs4_push<<<grid3((int64_t)nb * 1024, 256), 256, 0, ctx->stream>>>(u, b, view(ctx, l), p, c >> 1, c & 1,
+          launch_pdl(k3_gs4_push, grid3((int64_t)nb * 1024, 256), 256, 0, ctx->stream, u, b, view(ctx, l), p, c >> 1, c & 1,
                                                                                ctx->push_lv[l - 1], sw);
         else
-          k3_gs_rb_tpush<<<grid3((int64_t)nb * 2048, 256), 256, 0, ctx->stream>>>(u, b, view(ctx, l), p, c,
+          launch_pdl(k3_gs_rb_tpush, grid3((int64_t)nb * 2048, 256), 256, 0, ctx->stream, u, b, view(ctx, l), p, c,
                                                                                   ctx->push_lv[l - 1], sw);
         ctx->launches++;
         continue;
@@ -806,7 +835,7 @@ int residual(srmg_ctx *ctx, double *r, const double *u, const double *b, int l, 
   const int n = ctx->nblk_host[l - 1];
   if (!n) return SRMG_OK;
   if (seq3_push(ctx, S3_RESIDUAL, 0, 0, r, u, b, view(ctx, l), &p, nullptr)) return SRMG_OK;
-  k3_residual<<<grid3((int64_t)n * 4096, 256), 256, 0, ctx->stream>>>(r, u, b, view(ctx, l), p);
+  launch_pdl(k3_residual, grid3((int64_t)n * 4096, 256), 256, 0, ctx->stream, r, u, b, view(ctx, l), p);
   ctx->launches++;
   return SRMG_OK;
 }
@@ -815,7 +844,7 @@ int postrestrict(srmg_ctx *ctx, double *bf, const double *u, const double *r, in
   const int n = ctx->nch_host[l - 1];
   if (!n) return SRMG_OK;
   if (seq3_push(ctx, S3_POSTRESTRICT, 0, 0, bf, u, r, view(ctx, l), &pc, nullptr)) return SRMG_OK;
-  k3_postrestrict<<<grid3((int64_t)n * 512, 256), 256, 0, ctx->stream>>>(bf, u, r, view(ctx, l), pc);
+  launch_pdl(k3_postrestrict, grid3((int64_t)n * 512, 256), 256, 0, ctx->stream, bf, u, r, view(ctx, l), pc);
   ctx->launches++;
   return SRMG_OK;
 }
@@ -824,7 +853,7 @@ int restrict_l(srmg_ctx *ctx, double *u, int l) {
   const int n = ctx->nch_host[l - 1];
   if (!n) return SRMG_OK;
   if (seq3_push(ctx, S3_RESTRICT, 0, 0, u, nullptr, nullptr, view(ctx, l), nullptr, nullptr)) return SRMG_OK;
-  k3_restrict<<<grid3((int64_t)n * 512, 256), 256, 0, ctx->stream>>>(u, view(ctx, l));
+  launch_pdl(k3_restrict, grid3((int64_t)n * 512, 256), 256, 0, ctx->stream, u, view(ctx, l));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -833,7 +862,7 @@ int interp_add(srmg_ctx *ctx, double *u, const double *u1, int l) {
   const int n = ctx->nch_host[l - 1];
   if (!n) return SRMG_OK;
   if (seq3_push(ctx, S3_INTERP_ADD, 0, 0, u, u1, nullptr, view(ctx, l), nullptr, nullptr)) return SRMG_OK;
-  k3_interp_add<<<grid3((int64_t)n * 4096, 256), 256, 0, ctx->stream>>>(u, u1, view(ctx, l));
+  launch_pdl(k3_interp_add, grid3((int64_t)n * 4096, 256), 256, 0, ctx->stream, u, u1, view(ctx, l));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -842,7 +871,7 @@ int copy_l(srmg_ctx *ctx, double *dst, const double *a1, const double *a2, int l
   const int n = ctx->nblk_host[l - 1];
   if (!n) return SRMG_OK;
   if (seq3_push(ctx, S3_COPY, 0, 0, dst, a1, a2, view(ctx, l), nullptr, nullptr)) return SRMG_OK;
-  k3_copy<<<grid3((int64_t)n * S3, 256), 256, 0, ctx->stream>>>(dst, a1, a2, view(ctx, l));
+  launch_pdl(k3_copy, grid3((int64_t)n * S3, 256), 256, 0, ctx->stream, dst, a1, a2, view(ctx, l));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -894,7 +923,7 @@ int leafnorm(srmg_ctx *ctx, const double *u, const double *b, double s, int op, 
   for (int l = 1; l <= ctx->nlev; ++l) {
     if (!grids[l - 1]) continue;
     const double wl = 1.0 / (double)((int64_t)1 << (3 * (l - 1)));
-    k3_leafsq<NT><<<grids[l - 1], NT, 0, ctx->stream>>>(part + off, u, b, view(ctx, l),
+    launch_pdl(k3_leafsq<NT>, grids[l - 1], NT, 0, ctx->stream, part + off, u, b, view(ctx, l),
                                                        op3(op, k2, level_scale(s, l), 1.0), wl, mode);
     ctx->launches++;
     off += grids[l - 1];
@@ -904,7 +933,7 @@ int leafnorm(srmg_ctx *ctx, const double *u, const double *b, double s, int op, 
     CK(cudaMemsetAsync(out, 0, sizeof(double), ctx->stream));
     return SRMG_OK;
   }
-  k_reduce_sqrt<1024><<<1, 1024, 0, ctx->stream>>>(out, part, total);
+  launch_pdl(k_reduce_sqrt<1024>, 1, 1024, 0, ctx->stream, out, part, total);
   ctx->launches++;
   return SRMG_OK;
 }
@@ -1138,7 +1167,7 @@ int srmg::d3_rhs_level(srmg_ctx *ctx, double *q1, const double *q, int level, in
   if (level < 1 || level > ctx->nlev) return fail(ctx, SRMG_ERR_BADARG, "rhs_level: bad level");
   const int n = ctx->nblk_host[level - 1];
   if (n) {
-    k3_rhs<<<grid3((int64_t)n * 4096, 256), 256, 0, ctx->stream>>>(q1, q, view(ctx, level), op);
+    launch_pdl(k3_rhs, grid3((int64_t)n * 4096, 256), 256, 0, ctx->stream, q1, q, view(ctx, level), op);
     ctx->launches++;
   }
   return SRMG_OK;

@@ -8,6 +8,29 @@
 namespace srmg {
 
 int fail(srmg_ctx *c, int code, const char *fmt, ...);
+
+// Launches a kernel that may begin while its predecessor on the stream still runs
+// (programmatic dependent launch): its blocks are scheduled as the predecessor's last ones
+// have started, and pdl_enter() at its top waits until the predecessor has completed and
+// its writes are visible.  The sequences of short per-operation kernels -- 2 to 5 us each --
+// spend most of a launch's cost that way before the wait instead of between the kernels
+// (order-4 V-cycle on 2725 blocks: see k_gs4_push).  Every kernel launched with it must call
+// pdl_enter() in every thread before it touches memory that other kernels write.
+template <typename... KArgs, typename... Args>
+void launch_pdl(void (*kernel)(KArgs...), int64_t grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  // errors surface in the callers' cudaGetLastError, as a plain launch's do
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
 int cuda_check(srmg_ctx *c, cudaError_t e, const char *what);
 int ensure(srmg_ctx *ctx, DevBuf &b, size_t bytes);
 int check_call(srmg_ctx *ctx, int64_t nblk_alloc, int op, int geom, const int8_t *bc);

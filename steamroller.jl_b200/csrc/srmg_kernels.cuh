@@ -31,6 +31,15 @@ constexpr int kNormChunk = 4;
 // defect-correction steps run (mixed mode; 0 in FP64 mode)}.
 constexpr int kItemRec = 5;
 
+// Top of a kernel launched by launch_pdl: lets the next kernel's blocks be scheduled, then
+// waits for the previous kernel on the stream to complete.  (A load through a const
+// __restrict__ pointer may be moved above the wait unless its address comes from a load that
+// cannot; in these kernels it comes from the tree's tables.)
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Face numbering (the four StarStencil directions): 0 = -r, 1 = +r, 2 = -z, 3 = +z.
 enum FaceType : int { FACE_NONE = 0, FACE_NEIGHBOR = 1, FACE_BOUNDARY = 2, FACE_REFBND = 3 };
 
@@ -467,6 +476,7 @@ template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_leafsq(double *__restrict__ part, const T *__restrict__ u,
                                                const T *__restrict__ b, LevelView lv,
                                                OpParams<T> p, WTab<T> wt, double wl, int mode) {
+  pdl_enter();
   double acc = 0.0;
   const int64_t total = (int64_t)lv.nblk * 256;
   for (int64_t t = blockIdx.x * (int64_t)NT + threadIdx.x; t < total; t += (int64_t)gridDim.x * NT) {
@@ -497,10 +507,12 @@ __global__ void __launch_bounds__(NT) k_leafsq(double *__restrict__ part, const 
   }
 }
 
-// Final fixed-order reduction of n partials into out[0] (sqrt applied).
+// Final fixed-order reduction of n partials into out[0] (sqrt applied).  part is not
+// __restrict__: its loads must stay below pdl_enter().
 template <int NT>
-__global__ void __launch_bounds__(NT) k_reduce_sqrt(double *__restrict__ out,
-                                                    const double *__restrict__ part, int n) {
+__global__ void __launch_bounds__(NT) k_reduce_sqrt(double *out,
+                                                    const double *part, int n) {
+  pdl_enter();
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += NT) acc += part[i];
   __shared__ double sh[NT / 32];
@@ -548,6 +560,7 @@ __device__ __forceinline__ void d_gs4(T *__restrict__ u, const T *__restrict__ b
 // (0,-1), (-1,0), (0,0), (1,0), (0,1), then divided by 12.
 template <typename T>
 __global__ void k_rhs(T *__restrict__ q1, const T *__restrict__ q, LevelView lv, int op, int geom) {
+  pdl_enter();
   const int64_t total = (int64_t)lv.nblk * 256;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -663,18 +676,21 @@ __device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelV
 // same bodies also run as the operations of one cooperative launch (srmg_seq.cu).
 template <typename T>
 __global__ void __launch_bounds__(256, 6) k_fill_ghost(T *__restrict__ u, LevelView lv, Signs sg, int mask) {
+  pdl_enter();
   d_fill_ghost<T>(u, lv, sg, mask);
 }
 
 template <typename T>
 __global__ void k_gs_colour(T *__restrict__ u, const T *__restrict__ b, LevelView lv,
                             OpParams<T> p, WTab<T> wt, int parity) {
+  pdl_enter();
   d_gs_colour<T>(u, b, lv, p, wt, parity);
 }
 
 template <typename T>
 __global__ void k_residual(T *__restrict__ r, const T *__restrict__ u, const T *__restrict__ b,
                            LevelView lv, OpParams<T> p, WTab<T> wt) {
+  pdl_enter();
   d_residual<T>(r, u, b, lv, p, wt);
 }
 
@@ -682,32 +698,38 @@ template <typename T>
 __global__ void k_postrestrict(T *__restrict__ bf, const T *__restrict__ u, const T *__restrict__ r,
                                LevelView lv, const int2 *__restrict__ coord_of, OpParams<T> p,
                                WTab<T> wt) {
+  pdl_enter();
   d_postrestrict<T>(bf, u, r, lv, coord_of, p, wt);
 }
 
 template <typename T>
 __global__ void k_restrict(T *__restrict__ u, LevelView lv) {
+  pdl_enter();
   d_restrict<T>(u, lv);
 }
 
 template <typename T>
 __global__ void k_interp_add(T *__restrict__ u, const T *__restrict__ u1, LevelView lv) {
+  pdl_enter();
   d_interp_add<T>(u, u1, lv);
 }
 
 template <typename T>
 __global__ void k_copy_level(T *__restrict__ dst, const T *__restrict__ src, LevelView lv) {
+  pdl_enter();
   d_copy_level<T>(dst, src, lv);
 }
 
 template <typename T>
 __global__ void k_diff_level(T *__restrict__ dst, const T *__restrict__ a1, const T *a2,
                              LevelView lv) {
+  pdl_enter();
   d_diff_level<T>(dst, a1, a2, lv);
 }
 
 template <typename T>
 __global__ void k_gs4(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p, int p1, int p2) {
+  pdl_enter();
   d_gs4<T>(u, b, lv, p, p1, p2);
 }
 
@@ -715,12 +737,14 @@ __global__ void k_gs4(T *__restrict__ u, const T *__restrict__ b, LevelView lv, 
 template <typename T>
 __global__ void k_gs_colour_push(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p,
                                  WTab<T> wt, int parity, PushView pv, unsigned sg) {
+  pdl_enter();
   d_gs_colour_impl<T, true>(u, b, lv, p, wt, parity, pv, sg);
 }
 
 template <typename T>
 __global__ void k_gs4_push(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p, int p1, int p2,
                            PushView pv, unsigned sg) {
+  pdl_enter();
   d_gs4_impl<T, true>(u, b, lv, p, p1, p2, pv, sg);
 }
 
