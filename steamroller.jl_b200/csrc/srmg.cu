@@ -105,6 +105,8 @@ void srmg::free_tree(srmg_ctx *ctx) {
   ctx->fbc_built = false;
   if (ctx->push_tab.p) cudaFree(ctx->push_tab.p);
   ctx->push_tab = DevBuf{};
+  if (ctx->coef4.p) cudaFree(ctx->coef4.p);
+  ctx->coef4 = DevBuf{};
   ctx->push_lv.clear();
   ctx->push_state = 0;
 }
@@ -687,6 +689,8 @@ OpParams<T> srmg::op_params(int op, int geom, double k2, double sl, double omega
   const double c = (op == SRMG_OP_HELMHOLTZ) ? (-4 - sl * k2) : -4.0;  // diagelm (order 2)
   p.nwc = (T)(-(omega / c));
   p.omega = (T)omega;
+  p.rs = (T)recip_of(sl);
+  p.c4 = nullptr;
   return p;
 }
 template OpParams<double> srmg::op_params<double>(int, int, double, double, double);
@@ -725,33 +729,15 @@ template <typename T>
 int srmg::L_fill_ghost(srmg_ctx *ctx, T *u, int l, const Signs &sg, int mask) {
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nblk == 0) return SRMG_OK;
-  const int threads = 256;
-  const int gf = grid_for((int64_t)L.nblk * 32, threads, kGridCap);
-  if (!L.cfaces) {
-    // star faces only: the three passes touch disjoint cells and read none of each
-    // other's results, so one launch does them all
-    if (seq_push<T>(ctx, SEQ_FILL, mask, 0, u, nullptr, nullptr, L.view(l), nullptr, &sg)) return SRMG_OK;
-    launch_pdl(k_fill_ghost<T>, gf, threads, 0, ctx->stream, u, L.view(l), sg, mask);
-    ctx->launches++;
-    return SRMG_OK;
-  }
-  // BoxStencil tree: copy, boundary and interpolation are ordered passes (fill_ghost!,
-  // src/connectivity.jl:155-159), each launch filling the faces and corners of its
-  // passes.  Copy and boundary share one launch (a boundary corner evaluates the face
-  // ghost it mirrors itself, fill_corner_cell); interpolation follows on its own.
-  if ((mask & 3) == 3) {
-    if (!seq_push<T>(ctx, SEQ_FILL, 3, 0, u, nullptr, nullptr, L.view(l), nullptr, &sg)) {
-      launch_pdl(k_fill_ghost<T>, gf, threads, 0, ctx->stream, u, L.view(l), sg, 3);
-      ctx->launches++;
-    }
-    mask &= ~3;
-  }
-  for (int phase = 1; phase <= 4; phase <<= 1) {
-    if (!(mask & phase)) continue;
-    if (seq_push<T>(ctx, SEQ_FILL, phase, 0, u, nullptr, nullptr, L.view(l), nullptr, &sg)) continue;
-    launch_pdl(k_fill_ghost<T>, gf, threads, 0, ctx->stream, u, L.view(l), sg, phase);
-    ctx->launches++;
-  }
+  // every pass in one launch: on StarStencil trees the passes touch disjoint cells and read
+  // none of each other's results, on BoxStencil trees a block's warp runs them in order
+  // (d_fill_ghost).  A level without refinement faces has nothing to interpolate.
+  if (!((ctx->refbnd_levels >> l) & 1)) mask &= ~12;
+  if (!(mask & 7)) return SRMG_OK;
+  if (seq_push<T>(ctx, SEQ_FILL, mask, 0, u, nullptr, nullptr, L.view(l), nullptr, &sg)) return SRMG_OK;
+  launch_pdl(k_fill_ghost<T>, grid_for((int64_t)L.nblk * 32, 256, kGridCap), 256, 0, ctx->stream, u, L.view(l), sg,
+             mask);
+  ctx->launches++;
   return SRMG_OK;
 }
 
@@ -786,6 +772,11 @@ int srmg::ensure_gs_push(srmg_ctx *ctx, int op) {
   CK(cudaStreamIsCapturing(ctx->stream, &cap));
   if (cap != cudaStreamCaptureStatusNone) return SRMG_OK;
   ctx->push_state = -1;
+  if (ctx->has_corners && ctx->coef4.bytes == 0) {
+    RC(ensure(ctx, ctx->coef4, (size_t)ctx->wtab_n * kCoef4 * sizeof(double)));
+    k_coef4<<<(ctx->wtab_n + 127) / 128, 128, 0, ctx->stream>>>((double *)ctx->coef4.p, ctx->wtab_n);
+    CK(cudaGetLastError());
+  }
   const int64_t nf = ctx->max_blk * kSS;
   if (nf <= 0 || nf >= ((int64_t)1 << 31)) return SRMG_OK;
   static const int kPrime[9] = {2, 3, 5, 7, 11, 13, 17, 19, 23};
@@ -873,14 +864,34 @@ int srmg::ensure_gs_push(srmg_ctx *ctx, int op) {
       }
     }
   if (!ok2 && !ok4) return SRMG_OK;
-  // per level: offsets (nblk * 256 + 1 ints), then the entries sorted by source cell
+  // per level: the index of each child edge's fine block, and whether a boundary corner
+  // mirrors a refinement ghost (a ghost no cell's push refreshes)
+  std::vector<std::vector<int>> cbi(ctx->nlev);
+  ctx->mref_levels = 0;
+  for (int l = 1; l <= ctx->nlev; l++) {
+    const DevLevel &L = ctx->lv[l - 1];
+    std::vector<int4> ch(L.nch), fc(4 * (size_t)L.nblk), cf(L.cfaces ? 4 * (size_t)L.nblk : 0);
+    if (L.nch) CK(cudaMemcpy(ch.data(), L.child, ch.size() * sizeof(int4), cudaMemcpyDeviceToHost));
+    for (const int4 &e : ch) cbi[l - 1].push_back(bi_of[e.x]);
+    if (cf.empty()) continue;
+    CK(cudaMemcpy(fc.data(), L.faces, fc.size() * sizeof(int4), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(cf.data(), L.cfaces, cf.size() * sizeof(int4), cudaMemcpyDeviceToHost));
+    for (size_t k = 0; k < cf.size(); k++) {
+      if (cf[k].x != FACE_BOUNDARY || (cf[k].z == 0) == (cf[k].w == 0)) continue;
+      const size_t f = cf[k].z == 0 ? (k & 1) : 2 + ((k >> 1) & 1);
+      const int t = fc[(k & ~(size_t)3) + f].x;
+      if (t != FACE_NEIGHBOR && t != FACE_BOUNDARY) ctx->mref_levels |= 1u << l;
+    }
+  }
+  // per level: offsets (nblk * 256 + 1 ints), the child indices, then the entries sorted by
+  // source cell
   std::vector<size_t> at(ctx->nlev);
   size_t bytes = 0;
   for (int l = 1; l <= ctx->nlev; l++) {
     at[l - 1] = bytes;
     const int nb = ctx->lv[l - 1].nblk;
     if (!nb) continue;
-    bytes += ((size_t)nb * 256 + 1) * sizeof(int);
+    bytes += ((size_t)nb * 256 + 1 + cbi[l - 1].size()) * sizeof(int);
     bytes = (bytes + 15) & ~(size_t)15;
     bytes += ents[l - 1].size() * sizeof(int2);
     bytes = (bytes + 15) & ~(size_t)15;
@@ -890,8 +901,9 @@ int srmg::ensure_gs_push(srmg_ctx *ctx, int op) {
     const int nb = ctx->lv[l - 1].nblk;
     if (!nb) continue;
     int *off = reinterpret_cast<int *>(stage.data() + at[l - 1]);
-    const size_t ent_at = (at[l - 1] + ((size_t)nb * 256 + 1) * sizeof(int) + 15) & ~(size_t)15;
+    const size_t ent_at = (at[l - 1] + ((size_t)nb * 256 + 1 + cbi[l - 1].size()) * sizeof(int) + 15) & ~(size_t)15;
     int2 *ent = reinterpret_cast<int2 *>(stage.data() + ent_at);
+    std::copy(cbi[l - 1].begin(), cbi[l - 1].end(), off + nb * 256 + 1);
     std::fill(off, off + nb * 256 + 1, 0);
     for (const Ent &e : ents[l - 1]) off[e.key + 1]++;
     for (int k = 0; k < nb * 256; k++) off[k + 1] += off[k];
@@ -900,14 +912,14 @@ int srmg::ensure_gs_push(srmg_ctx *ctx, int op) {
   }
   RC(ensure(ctx, ctx->push_tab, bytes));
   CK(cudaMemcpy(ctx->push_tab.p, stage.data(), bytes, cudaMemcpyHostToDevice));
-  ctx->push_lv.assign(ctx->nlev, PushView{nullptr, nullptr});
+  ctx->push_lv.assign(ctx->nlev, PushView{nullptr, nullptr, nullptr});
   for (int l = 1; l <= ctx->nlev; l++) {
     const int nb = ctx->lv[l - 1].nblk;
     if (!nb) continue;
     char *base = static_cast<char *>(ctx->push_tab.p);
-    const size_t ent_at = (at[l - 1] + ((size_t)nb * 256 + 1) * sizeof(int) + 15) & ~(size_t)15;
-    ctx->push_lv[l - 1] = PushView{reinterpret_cast<const int *>(base + at[l - 1]),
-                                   reinterpret_cast<const int2 *>(base + ent_at)};
+    const size_t ent_at = (at[l - 1] + ((size_t)nb * 256 + 1 + cbi[l - 1].size()) * sizeof(int) + 15) & ~(size_t)15;
+    const int *off = reinterpret_cast<const int *>(base + at[l - 1]);
+    ctx->push_lv[l - 1] = PushView{off, reinterpret_cast<const int2 *>(base + ent_at), off + nb * 256 + 1};
   }
   ctx->push_ok2 = ok2;
   ctx->push_ok4 = ok4;
@@ -915,11 +927,19 @@ int srmg::ensure_gs_push(srmg_ctx *ctx, int op) {
   return SRMG_OK;
 }
 
+// The operator with the tree's order-4 coefficient table, where it has been built.
 template <typename T>
-int srmg::L_gs_colour(srmg_ctx *ctx, T *u, const T *b, int l, const OpParams<T> &p, int parity) {
+static OpParams<T> tabled(const srmg_ctx *ctx, OpParams<T> p) {
+  if (p.op == SRMG_OP_LAPLACIAN4) p.c4 = (const double *)ctx->coef4.p;
+  return p;
+}
+
+template <typename T>
+int srmg::L_gs_colour(srmg_ctx *ctx, T *u, const T *b, int l, const OpParams<T> &p0, int parity) {
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nblk == 0) return SRMG_OK;
   const int threads = 128;
+  const OpParams<T> p = tabled(ctx, p0);
   if (p.op == SRMG_OP_LAPLACIAN4) {
     // FourColors{parity >> 1, parity & 1}
     if (seq_push<T>(ctx, SEQ_GS4, parity >> 1, parity & 1, u, b, nullptr, L.view(l), &p, nullptr)) return SRMG_OK;
@@ -933,14 +953,26 @@ int srmg::L_gs_colour(srmg_ctx *ctx, T *u, const T *b, int l, const OpParams<T> 
   return SRMG_OK;
 }
 
+// A boundary table of -1, 0 and 1 as bits: entry + 1, two bits an entry.
+static unsigned sign_bits(const Signs &sg) {
+  unsigned sw = 0;
+  for (int i = 0; i < 9; i++) sw |= (unsigned)((int)sg.v[i] + 1) << (2 * i);
+  return sw;
+}
+static bool unit_signs(const Signs &sg) {
+  for (int i = 0; i < 9; i++)
+    if (sg.v[i] != 1.0 && sg.v[i] != -1.0 && sg.v[i] != 0.0) return false;
+  return true;
+}
+
 // One colour sweep that writes the copy and boundary ghosts of the cells it updates.
 template <typename T>
-static int L_gs_colour_push(srmg_ctx *ctx, T *u, const T *b, int l, const OpParams<T> &p, int parity,
+static int L_gs_colour_push(srmg_ctx *ctx, T *u, const T *b, int l, const OpParams<T> &p0, int parity,
                             const Signs &sg) {
   const DevLevel &L = ctx->lv[l - 1];
   const int threads = 128;
-  unsigned sw = 0;  // entry + 1, two bits an entry (every entry is -1, 0 or 1 here)
-  for (int i = 0; i < 9; i++) sw |= (unsigned)((int)sg.v[i] + 1) << (2 * i);
+  const OpParams<T> p = tabled(ctx, p0);
+  const unsigned sw = sign_bits(sg);
   if (p.op == SRMG_OP_LAPLACIAN4)
     launch_pdl(k_gs4_push<T>, grid_for((int64_t)L.nblk * 64, threads, kGridCap), threads, 0, ctx->stream, u, b, L.view(l), p, parity >> 1, parity & 1, ctx->push_lv[l - 1], sw);
   else
@@ -961,9 +993,7 @@ int srmg::L_gs_iter(srmg_ctx *ctx, T *u, const T *b, int l, const OpParams<T> &p
                     const Signs &sg) {
   const bool four = p.op == SRMG_OP_LAPLACIAN4;
   if (ctx->push_state == 0) RC(ensure_gs_push(ctx, p.op));
-  bool unit = true;
-  for (int i = 0; i < 9; i++) unit = unit && (sg.v[i] == 1.0 || sg.v[i] == -1.0 || sg.v[i] == 0.0);
-  const bool push = ctx->use_gs_push && ctx->push_state == 1 && !ctx->seq_rec && unit &&
+  const bool push = ctx->use_gs_push && ctx->push_state == 1 && !ctx->seq_rec && unit_signs(sg) &&
                     (four ? ctx->push_ok4 : ctx->push_ok2) && ctx->lv[l - 1].nblk > 0;
   const int ncol = four ? 4 : 2;
   for (int i = 0; i < n; i++)
@@ -983,7 +1013,8 @@ int srmg::L_residual(srmg_ctx *ctx, T *r, const T *u, const T *b, int l, const O
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nblk == 0) return SRMG_OK;
   if (seq_push<T>(ctx, SEQ_RESIDUAL, 0, 0, r, u, b, L.view(l), &p, nullptr)) return SRMG_OK;
-  launch_pdl(k_residual<T>, grid_for((int64_t)L.nblk * 256, 256, kGridCap), 256, 0, ctx->stream, r, u, b, L.view(l), p, wtab<T>(ctx));
+  launch_pdl(k_residual<T>, grid_for((int64_t)L.nblk * 256, 256, kGridCap), 256, 0, ctx->stream, r, u, b, L.view(l),
+             tabled(ctx, p), wtab<T>(ctx));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -993,7 +1024,8 @@ int srmg::L_postrestrict(srmg_ctx *ctx, T *bf, const T *u, const T *r, int l, co
   const DevLevel &L = ctx->lv[l - 1];
   if (L.nch == 0) return SRMG_OK;
   if (seq_push<T>(ctx, SEQ_POSTRESTRICT, 0, 0, bf, u, r, L.view(l), &pc, nullptr)) return SRMG_OK;
-  launch_pdl(k_postrestrict<T>, grid_for((int64_t)L.nch * 64, 256, kGridCap), 256, 0, ctx->stream, bf, u, r, L.view(l), ctx->d_coord_of, pc, wtab<T>(ctx));
+  launch_pdl(k_postrestrict<T>, grid_for((int64_t)L.nch * 64, 256, kGridCap), 256, 0, ctx->stream, bf, u, r, L.view(l), ctx->d_coord_of,
+             tabled(ctx, pc), wtab<T>(ctx));
   ctx->launches++;
   return SRMG_OK;
 }
@@ -1040,6 +1072,96 @@ int srmg::L_diff(srmg_ctx *ctx, T *dst, const T *a1, const T *a2, int l) {
 
 // ------------------------------------------------------------------ V-cycle / FMG
 
+// The V-cycle on trees whose sweeps push their ghosts, with its steps fused (the same values
+// in u and in b; r and u1, scratch, end with other contents).  A level's ghosts stay what
+// a fill would make of them -- the sweeps and the prolongation push their cells' copies and
+// mirrors, refinement ghosts are interpolated once the parent level is final -- so of the
+// reference's fills only the one after the restriction remains, besides the one after the
+// first colour on the finest level (the caller's ghosts are not known) and on levels whose
+// boundary corners mirror refinement ghosts.  Levels 1..top, at most kLocalBlocks blocks
+// each, run in one CTA.  On the 2725-block order-4 tree a cycle is 131 kernels instead of
+// 281 and 1.98 -> see DESIGN ms for two cycles.
+template <typename T>
+static int vcycle_fused(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, double k2, int geom, const Signs &sg,
+                        int lmax, int ndown, int ntop, int nup, double omega) {
+  const unsigned sw = sign_bits(sg);
+  const bool four = op == SRMG_OP_LAPLACIAN4;
+  auto par = [&](int l) { return tabled(ctx, op_params<T>(op, geom, k2, level_scale(s, l), omega)); };
+  auto refined = [&](int l) { return ((ctx->refbnd_levels >> l) & 1) != 0; };
+  // the reference's cycle starts on the finest level with blocks; above it only that
+  // level's ghost fill has an effect
+  const int lend = lmax;
+  while (lmax > 1 && ctx->lv[lmax - 1].nblk == 0) --lmax;
+  const bool filled = lmax < lend;
+  if (filled) RC(L_fill_ghost<T>(ctx, u, lmax, sg, 7));
+  auto gs = [&](int l, int n, bool known) -> int {
+    const OpParams<T> p = par(l);
+    for (int i = 0; i < n; i++)
+      for (int c = 0; c < (four ? 4 : 2); c++) {
+        RC(L_gs_colour_push<T>(ctx, u, b, l, p, c, sg));
+        if (i == 0 && c == 0 && (!known || ((ctx->mref_levels >> l) & 1))) RC(L_fill_ghost<T>(ctx, u, l, sg, 3));
+      }
+    return SRMG_OK;
+  };
+  int top = 0;
+  while (top < lmax && top < kLocalLevels && ctx->lv[top].nblk > 0 && ctx->lv[top].nblk <= kLocalBlocks) ++top;
+  const int lo = std::max(top, 1);
+  for (int l = lmax; l > lo; l--) {
+    const DevLevel &L = ctx->lv[l - 1], &C = ctx->lv[l - 2];
+    RC(gs(l, ndown, filled || l < lmax));
+    launch_pdl(k_down<T>, grid_for((int64_t)L.nch * 64, 128, kGridCap), 128, 0, ctx->stream, u, r, b, L.view(l),
+               ctx->d_coord_of, par(l), wtab<T>(ctx));
+    ctx->launches++;
+    if (l - 1 == top) break;  // k_vcycle_local takes it from here
+    RC(L_fill_ghost<T>(ctx, u, l - 1, sg, 7));
+    launch_pdl(k_save_rhs<T>, grid_for((int64_t)C.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, u1, b, u, r,
+               C.view(l - 1), L.view(l), ctx->d_coord_of, par(l - 1), wtab<T>(ctx));
+    ctx->launches++;
+  }
+  if (top >= 1) {
+    LocalCycle<T> A;
+    memset(&A, 0, sizeof A);
+    for (int l = 1; l <= std::min(top + 1, lmax); l++) {
+      A.lv[l] = ctx->lv[l - 1].view(l);
+      A.p[l] = par(l);
+      if (l <= top) A.pv[l] = ctx->push_lv[l - 1];
+    }
+    A.u = u;
+    A.b = b;
+    A.r = r;
+    A.u1 = u1;
+    A.sg = sg;
+    A.sw = sw;
+    A.refined = ctx->refbnd_levels;
+    A.mref = ctx->mref_levels;
+    A.wt = wtab<T>(ctx);
+    A.coord_of = ctx->d_coord_of;
+    A.top = top;
+    A.inner = lmax > top;
+    A.known = filled;
+    A.ndown = ndown;
+    A.ntop = ntop;
+    A.nup = nup;
+    launch_pdl(k_vcycle_local<T>, 1, 1024, 0, ctx->stream, A);
+    ctx->launches++;
+  } else {
+    RC(gs(1, ntop, filled || lmax > 1));
+  }
+  for (int l = lo + 1; l <= lmax; l++) {
+    const DevLevel &L = ctx->lv[l - 1], &C = ctx->lv[l - 2];
+    if (l - 1 != top) {
+      launch_pdl(k_correction<T>, grid_for((int64_t)C.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, r, u, u1,
+                 C.view(l - 1), sg);
+      ctx->launches++;
+    }
+    launch_pdl(k_interp_push<T>, grid_for((int64_t)L.nch * 256, 256, kGridCap), 256, 0, ctx->stream, u, r, L.view(l),
+               ctx->push_lv[l - 1], sw, sg, refined(l));
+    ctx->launches++;
+    RC(gs(l, nup, true));
+  }
+  return SRMG_OK;
+}
+
 template <typename T>
 int srmg::vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, double k2, int geom,
                      const Signs &sg, int lmax, int ndown, int ntop, int nup, double omega) {
@@ -1060,6 +1182,14 @@ int srmg::vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, d
     RC(prepare_items(ctx, specs.data(), geom, omega, false, 0, 0.0, &tabs));
     return engine_vcycle<T>(ctx, u, b, u1, r, tabs, geom, lmax, ndown, ntop, nup);
   }
+  RC(ensure_gs_push(ctx, op));
+  // every level down to 1 has blocks, and each block of levels 2.. is some child edge's fine block
+  bool whole = ctx->nlev <= 30 && ndown >= 1 && ntop >= 1 && nup >= 1 && ctx->lv[0].nblk > 0;
+  for (int l = 2; l <= lmax; l++)
+    whole = whole && ctx->lv[l - 1].nch == ctx->lv[l - 1].nblk && (ctx->lv[l - 1].nblk == 0 || ctx->lv[l - 2].nblk > 0);
+  if (whole && ctx->use_gs_push && ctx->push_state == 1 && !ctx->seq_rec && unit_signs(sg) &&
+      (op == SRMG_OP_LAPLACIAN4 ? ctx->push_ok4 : ctx->push_ok2))
+    return vcycle_fused<T>(ctx, u, b, r, u1, s, op, k2, geom, sg, lmax, ndown, ntop, nup, omega);
   for (int l = lmax; l >= 2; l--) {
     const double sl = level_scale(s, l);
     const OpParams<T> p = op_params<T>(op, geom, k2, sl, omega);
@@ -1107,21 +1237,28 @@ static int fmg_dev_t(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, d
                      const Signs &sg, int ndown, int ntop, int nup, double omega) {
   const int lmax = finest_level(ctx);
   for (int l = lmax; l >= 2; l--) {
-    const double sl = level_scale(s, l);
-    const OpParams<T> p = op_params<T>(op, geom, k2, sl, omega);
-    const OpParams<T> pc = op_params<T>(op, geom, k2, 4 * sl, omega);
-    RC(L_restrict<T>(ctx, u, l));
+    const DevLevel &L = ctx->lv[l - 1];
+    const OpParams<T> p = tabled(ctx, op_params<T>(op, geom, k2, level_scale(s, l), omega));
+    if (L.nch > 0) {
+      launch_pdl(k_down<T>, grid_for((int64_t)L.nch * 64, 128, kGridCap), 128, 0, ctx->stream, u, r, b, L.view(l),
+                 ctx->d_coord_of, p, wtab<T>(ctx));
+      ctx->launches++;
+    }
     RC(L_fill_ghost<T>(ctx, u, l - 1, sg, 7));
-    RC(L_residual<T>(ctx, r, u, b, l, p));
-    RC(L_restrict<T>(ctx, r, l));
-    RC(L_postrestrict<T>(ctx, b, u, r, l, pc));
+    RC(L_postrestrict<T>(ctx, b, u, r, l, op_params<T>(op, geom, k2, 4 * level_scale(s, l), omega)));
   }
   for (int l = 1; l <= lmax; l++) {
-    RC(L_copy<T>(ctx, u1, u, l));
-    if (l > 1) {
-      RC(L_diff<T>(ctx, u1, u, u1, l - 1));
-      RC(L_fill_ghost<T>(ctx, u1, l - 1, sg, 7));
-      RC(L_interp_add<T>(ctx, u, u1, l));
+    const DevLevel &L = ctx->lv[l - 1];
+    if (l == 1) {
+      RC(L_copy<T>(ctx, u1, u, l));
+    } else {
+      const DevLevel &C = ctx->lv[l - 2];
+      if (L.nblk + C.nblk > 0) {
+        launch_pdl(k_fmg_step<T>, grid_for((int64_t)std::max(L.nblk, C.nblk) * kSS, 256, kGridCap), 256, 0, ctx->stream,
+                   r, u1, u, L.view(l), C.view(l - 1), sg);
+        ctx->launches++;
+      }
+      RC(L_interp_add<T>(ctx, u, r, l));
     }
     RC(L_fill_ghost<T>(ctx, u, l, sg, 7));
     RC(vcycle_dev<T>(ctx, u, b, r, u1, s, op, k2, geom, sg, l, ndown, ntop, nup, omega));

@@ -121,6 +121,8 @@ struct srmg_ctx {
   bool push_ok2 = false, push_ok4 = false;  // race-free for red-black / four-colour sweeps
   srmg::DevBuf push_tab;
   std::vector<srmg::PushView> push_lv;      // per level, index l-1
+  unsigned mref_levels = 0;                 // bit l: boundary corners of level l mirror refinement ghosts
+  srmg::DevBuf coef4;                       // order-4 coefficients per radial index (BoxStencil trees)
   bool trace_on = false;
   srmg::DevBuf trace;        // %globaltimer stamps after every engine phase (CTA 0)
 

@@ -58,6 +58,28 @@ struct LevelView {
   const int4 *cfaces;
 };
 
+// The reciprocal div_by takes for a divisor: 1 / d, or 0 (plain divisions) where d is so small
+// or large that an intermediate result could leave the normal range.
+inline double recip_of(double d) {
+  const double m = d < 0 ? -d : d;
+  return m > 1e-90 && m < 1e90 ? 1.0 / d : 0.0;
+}
+
+// a / d for a fixed d and its correctly rounded reciprocal rd: two corrections of the
+// product a rd by the exact remainder.  The first makes q faithful (off by less than one
+// unit in the last place), so that by Markstein's theorem (IBM J. Res. Dev. 34, 1990) the
+// second gives the correctly rounded quotient, as long as nothing leaves the normal range;
+// there, and for zeros, infinities and NaN, the division itself is called.
+__device__ __forceinline__ double div_by(double a, double d, double rd) {
+  // the exponent field: 2^-700 <= |a| < 2^700 (an integer test; the fp64 pipe is the bound),
+  // and a reciprocal from recip_of
+  if ((unsigned)((__double2hiint(a) & 0x7ff00000) - (323 << 20)) >= (1400u << 20) || __double2hiint(rd) == 0)
+    return __ddiv_rn(a, d);
+  double q = __dmul_rn(a, rd);
+  q = fma(fma(-q, d, a), rd, q);
+  return fma(fma(-q, d, a), rd, q);
+}
+
 // Operator parameters for one level.
 template <typename T>
 struct OpParams {
@@ -67,7 +89,15 @@ struct OpParams {
   T centre;      // -4 or -4 - s_l*k2 (stencil centre, src/helmholtz.jl:43-45)
   T nwc;         // -(omega / diagelm)  (src/multigrid.jl:177)
   T omega;       // the relaxation factor itself (order 4 divides by a per-cell diagonal)
+  T rs;          // 1 / s, correctly rounded
+  const double *c4;  // order 4, cylindrical: kCoef4 coefficients per radial index, or null (formed per cell)
 };
+// Order-4 coefficients of one radial index: am, ap, em, cc, ep (coeffs9) and the diagonal.
+constexpr int kCoef4 = 6;
+
+// a / d with rd = 1 / d correctly rounded: div_by in double, the plain quotient in float.
+__device__ __forceinline__ double quot(double a, double d, double rd) { return div_by(a, d, rd); }
+__device__ __forceinline__ float quot(float a, float d, float) { return a / d; }
 
 struct Signs { double v[9]; };  // boundary-condition table as doubles, column-major
 
@@ -87,19 +117,6 @@ template <> __device__ __forceinline__ float dadd<float>(float a, float b) { ret
 template <typename T> __device__ __forceinline__ T dmul(T a, T b);
 template <> __device__ __forceinline__ double dmul<double>(double a, double b) { return __dmul_rn(a, b); }
 template <> __device__ __forceinline__ float dmul<float>(float a, float b) { return __fmul_rn(a, b); }
-
-// a / d for a fixed d > 0 and its correctly rounded reciprocal rd: two corrections of the
-// product a rd by the exact remainder.  The first makes q faithful (off by less than one
-// unit in the last place), so that by Markstein's theorem (IBM J. Res. Dev. 34, 1990) the
-// second gives the correctly rounded quotient, as long as nothing leaves the normal range;
-// there, and for zeros, infinities and NaN, the division itself is called.
-__device__ __forceinline__ double div_by(double a, double d, double rd) {
-  // the exponent field: 2^-700 <= |a| < 2^700 (an integer test; the fp64 pipe is the bound)
-  if ((unsigned)((__double2hiint(a) & 0x7ff00000) - (323 << 20)) >= (1400u << 20)) return __ddiv_rn(a, d);
-  double q = __dmul_rn(a, rd);
-  q = fma(fma(-q, d, a), rd, q);
-  return fma(fma(-q, d, a), rd, q);
-}
 
 // Whole-tile copies global -> shared by the CTA's threads (cp.async, CH = 16 or 8 bytes a
 // copy: 16 needs 16-byte aligned fields), for kernels that stream blocks through a ring of
@@ -180,17 +197,33 @@ __device__ __forceinline__ void coeffs9(int geom, int64_t ir, int64_t iz, double
   }
 }
 
+// The same from the table of this radial index (k_coef4, the same operations): forming the
+// coefficients takes five divisions, more than the rest of a cell's update.
+__device__ __forceinline__ void coeffs9(const double *c4, int geom, int64_t ir, int64_t iz, double c[9]) {
+  if (!c4 || geom == 0) {
+    coeffs9(geom, ir, iz, c);
+    return;
+  }
+  const double *t = c4 + kCoef4 * (geom == 1 ? ir : iz);
+  const double am = t[0], ap = t[1], em = t[2], cc = t[3], ep = t[4];
+  if (geom == 1) {
+    c[0] = am; c[1] = 4; c[2] = ap; c[3] = em; c[4] = cc; c[5] = ep; c[6] = am; c[7] = 4; c[8] = ap;
+  } else {
+    c[0] = am; c[1] = em; c[2] = am; c[3] = 4; c[4] = cc; c[5] = 4; c[6] = ap; c[7] = ep; c[8] = ap;
+  }
+}
+
 template <typename T>
-__device__ __forceinline__ T apply9(const T *ub, int x, int y, int geom, int64_t ir, int64_t iz) {
+__device__ __forceinline__ T apply9(const T *ub, int x, int y, int geom, int64_t ir, int64_t iz, const double *c4) {
   double c[9];
-  coeffs9(geom, ir, iz, c);
+  coeffs9(c4, geom, ir, iz, c);
   T v = T(0);
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     const int d1 = k % 3 - 1, d2 = k / 3 - 1;
     v = dadd<T>(v, dmul<T>(T(c[k]), ub[(x + d1) + kS * (y + d2)]));
   }
-  return v / T(6);
+  return quot(v, T(6), T(1) / T(6));  // exact: a sixth of a double is never halfway between two
 }
 
 // diagelm, order 4 (src/laplacian.jl:150-151, 205-209).
@@ -198,6 +231,21 @@ __device__ __forceinline__ double diagelm4(int geom, int64_t ir, int64_t iz) {
   if (geom == 0) return -20.0 / 6.0;
   const int64_t i = geom == 1 ? ir : iz;
   return __ddiv_rn(__ddiv_rn((double)(-16 * (1 - 5 * i + 5 * i * i)), (double)((1 - 2 * i) * (1 - 2 * i))), 6.0);
+}
+
+// The table of a tree: entry i for every radial 1-based global index i < n.
+static __global__ void k_coef4(double *__restrict__ tab, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 1 || i >= n) return;
+  double c[9];
+  coeffs9(1, i, 0, c);
+  double *t = tab + kCoef4 * i;
+  t[0] = c[0];
+  t[1] = c[2];
+  t[2] = c[3];
+  t[3] = c[4];
+  t[4] = c[5];
+  t[5] = diagelm4(1, i, 0);
 }
 
 // 1-based global indices of local cell (x, y) of a block at 1-based coords (cr, cz)
@@ -208,7 +256,7 @@ __device__ __forceinline__ int64_t gidx(int c, int x) { return (int64_t)kM * (c 
 template <typename T>
 __device__ __forceinline__ T lhs_apply(const T *ub, int x, int y, const OpParams<T> &p, const WTab<T> &wt,
                                        int cr, int cz) {
-  if (p.op == 2) return apply9<T>(ub, x, y, p.geom, gidx(cr, x), gidx(cz, y));
+  if (p.op == 2) return apply9<T>(ub, x, y, p.geom, gidx(cr, x), gidx(cz, y), p.c4);
   const W5<T> w = weights<T>(wt, p.geom, cr, cz, x, y);
   return apply5<T>(ub, x, y, w, p.centre);
 }
@@ -223,14 +271,15 @@ __device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelV
 // it is bound by how many of them are in flight: the four faces' records are loaded
 // together, then the four copied or mirrored values, before any is stored; refinement
 // faces (three values each, few of them) follow on their own.  With a warp per (block, face)
-// 36276 blocks took 72 us.  On a BoxStencil tree (lv.cfaces set) the launch covers one pass
-// (mask 1, 2 or 4) or the copy and boundary passes together (mask 3), and lanes 0..15 also
-// fill the block's 16 corner cells in those passes (fill_corner_cell).
+// 36276 blocks took 72 us.  On a BoxStencil tree (lv.cfaces set) lanes 0..15 also fill the
+// block's 16 corner cells (fill_corner_cell), in the order of fill_ghost!'s passes: the
+// copy and boundary passes, a warp barrier, then interpolation -- a boundary corner mirrors
+// its own block's refinement ghosts as they were before the fill, and no pass reads
+// another block's ghosts of this level, so one launch does all three.
 template <typename T>
 __device__ __forceinline__ void d_fill_ghost(T *__restrict__ u, LevelView lv, Signs sg, int mask) {
   const int lane = threadIdx.x & 31;
   const int g = lane >> 4, k = lane & 15;
-  const bool corners = lv.cfaces && (mask == 1 || mask == 2 || mask == 3 || mask == 4);
   const int stride = gridDim.x * (blockDim.x >> 5);
   for (int bi = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); bi < lv.nblk; bi += stride) {
     int type[4], src[4];
@@ -263,6 +312,10 @@ __device__ __forceinline__ void d_fill_ghost(T *__restrict__ u, LevelView lv, Si
       if (type[f] == FACE_NEIGHBOR && (mask & 1)) ub[x + kS * y] = v[f];
       else if (type[f] == FACE_BOUNDARY && (mask & 2)) ub[x + kS * y] = dmul<T>(T(sg.v[face_sign_index(f)]), v[f]);
     }
+    if (lv.cfaces) {
+      if ((mask & 3) && lane < 16) fill_corner_cell<T>(u, lv, sg, mask & 3, (int64_t)bi * 16 + lane);
+      __syncwarp();
+    }
     if (mask & 4) {
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
@@ -287,7 +340,7 @@ __device__ __forceinline__ void d_fill_ghost(T *__restrict__ u, LevelView lv, Si
         ub[x + kS * y] = w;
       }
     }
-    if (corners && lane < 16) fill_corner_cell<T>(u, lv, sg, mask, (int64_t)bi * 16 + lane);
+    if (lv.cfaces && (mask & 4) && lane < 16) fill_corner_cell<T>(u, lv, sg, 4, (int64_t)bi * 16 + lane);
   }
 }
 
@@ -304,6 +357,7 @@ __device__ __forceinline__ void d_fill_ghost(T *__restrict__ u, LevelView lv, Si
 struct PushView {
   const int *off;
   const int2 *ent;
+  const int *cbi;  // [child edge] index of its fine block in the level's block list (2D trees)
 };
 
 template <typename T>
@@ -347,7 +401,7 @@ __device__ __forceinline__ void d_gs_colour_impl(T *__restrict__ u, const T *__r
 template <typename T>
 __device__ __forceinline__ void d_gs_colour(T *__restrict__ u, const T *__restrict__ b, LevelView lv,
                                             OpParams<T> p, WTab<T> wt, int parity) {
-  d_gs_colour_impl<T, false>(u, b, lv, p, wt, parity, PushView{nullptr, nullptr}, 0u);
+  d_gs_colour_impl<T, false>(u, b, lv, p, wt, parity, PushView{nullptr, nullptr, nullptr}, 0u);
 }
 
 // ---- residual (src/multigrid.jl:309-323, 349-354): r = -(b + Lu/s) ---------------
@@ -363,7 +417,7 @@ __device__ __forceinline__ void d_residual(T *__restrict__ r, const T *__restric
     const int64_t base = (int64_t)bk.x * kSS;
     const T Lu = lhs_apply<T>(u + base, x, y, p, wt, bk.y, bk.z);
     const int64_t o = base + x + kS * y;
-    r[o] = -(b[o] + Lu / p.s);
+    r[o] = -(b[o] + quot(Lu, p.s, p.rs));
   }
 }
 
@@ -384,7 +438,7 @@ __device__ __forceinline__ void d_postrestrict(T *__restrict__ bf, const T *__re
     const int64_t base = (int64_t)cblk * kSS;
     const T Lu = lhs_apply<T>(u + base, x, y, p, wt, cc.x, cc.y);
     const int64_t o = base + x + kS * y;
-    bf[o] = -(r[o] + Lu / p.s);
+    bf[o] = -(r[o] + quot(Lu, p.s, p.rs));
   }
 }
 
@@ -539,9 +593,10 @@ __device__ __forceinline__ void d_gs4_impl(T *__restrict__ u, const T *__restric
     const int4 bk = lv.blocks[bi];
     T *ub = u + (int64_t)bk.x * kSS;
     const int64_t ir = gidx(bk.y, x), iz = gidx(bk.z, y);
-    const T Lu = apply9<T>(ub, x, y, p.geom, ir, iz);
+    const T Lu = apply9<T>(ub, x, y, p.geom, ir, iz, p.c4);
     const int o = x + kS * y;
-    const T cdiag = T(diagelm4(p.geom, ir, iz));
+    const T cdiag =
+        T(p.c4 && p.geom ? p.c4[kCoef4 * (p.geom == 1 ? ir : iz) + 5] : diagelm4(p.geom, ir, iz));
     const T upd = dmul<T>(p.omega, dadd<T>(Lu, dmul<T>(p.s, b[(int64_t)bk.x * kSS + o]))) / cdiag;
     const T nv = ub[o] - upd;
     ub[o] = nv;
@@ -551,7 +606,7 @@ __device__ __forceinline__ void d_gs4_impl(T *__restrict__ u, const T *__restric
 
 template <typename T>
 __device__ __forceinline__ void d_gs4(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p, int p1, int p2) {
-  d_gs4_impl<T, false>(u, b, lv, p, p1, p2, PushView{nullptr, nullptr}, 0u);
+  d_gs4_impl<T, false>(u, b, lv, p, p1, p2, PushView{nullptr, nullptr, nullptr}, 0u);
 }
 
 // rhs! over rhs_level! (src/multigrid.jl:363-388): q1 = R q on the valid cells.  Order
@@ -596,12 +651,11 @@ __global__ void k_rhs(T *__restrict__ q1, const T *__restrict__ q, LevelView lv,
 // from the parent's subblockbnd cell (src/blockfield.jl:416-434, src/interp.jl:24-63).
 // A boundary corner whose bnd is zero along one dimension mirrors the adjacent face's
 // ghost cells, which fill_ghost! writes in an earlier pass.  fill_ghost! runs copy,
-// boundary and interpolation in that order; here copy and boundary may share one launch
-// (mask 3): such a corner then evaluates the face ghost it mirrors from that face's own
+// boundary and interpolation in that order; here copy and boundary share one pass
+// (mask 3): such a corner evaluates the face ghost it mirrors from that face's own
 // source -- the neighbour's valid cell, or the mirrored valid cell -- with the same
-// operations as the face pass, instead of reading it.  Interpolation (mask 4) stays a
-// launch of its own after them: the boundary pass reads a refinement face's ghosts as
-// they were before this fill.
+// operations as the face pass, instead of reading it.  Interpolation (mask 4) follows: the
+// boundary pass reads a refinement face's ghosts as they were before this fill.
 template <typename T>
 __device__ __forceinline__ T face_ghost_value(const T *__restrict__ u, const T *ub, const LevelView &lv,
                                               const Signs &sg, int bi, int f, int x, int y) {
@@ -672,6 +726,139 @@ __device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelV
 }
 
 
+// ---- fused steps of the per-operation V-cycle (vcycle_fused) -------------------------
+// The restriction half of a level's descent in one pass over its child edges: the fine
+// block's residual is formed where it is restricted (residual_level! writes it and
+// restrict_level! reads it back, two more launches), u and r restricted in the
+// reference's order.  r's fine cells are not written.
+template <typename T>
+__device__ __forceinline__ void d_down(T *__restrict__ u, T *__restrict__ r, const T *__restrict__ b, const LevelView &lv,
+                                       const int2 *__restrict__ coord_of, const OpParams<T> &p, const WTab<T> &wt) {
+  const int64_t total = (int64_t)lv.nch * 64;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int e = (int)(t >> 6), c = (int)(t & 63);
+    const int4 ch = lv.child[e];
+    const int kx = c & 7, ky = c >> 3;
+    const int2 fc = coord_of[ch.x];
+    const T *ub = u + (int64_t)ch.x * kSS, *bb = b + (int64_t)ch.x * kSS;
+    T f = T(0), g = T(0);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int x = 2 + 2 * kx + i, y = 2 + 2 * ky + j, o = x + kS * y;
+        f = dadd<T>(f, ub[o]);
+        const T Lu = lhs_apply<T>(ub, x, y, p, wt, fc.x, fc.y);
+        g = dadd<T>(g, -(bb[o] + quot(Lu, p.s, p.rs)));
+      }
+    const int64_t co = (int64_t)ch.y * kSS + (2 + 8 * (ch.z - 1) + kx) + kS * (2 + 8 * (ch.w - 1) + ky);
+    u[co] = dmul<T>(f, T(0.25));
+    r[co] = dmul<T>(g, T(0.25));
+  }
+}
+
+// Value of the field a - a1 that a ghost or valid cell (x, y) of block index bi holds after a
+// fill_ghost! of it, refinement ghosts interpolated from the parent level of e (already
+// filled): what copying or subtracting the whole blocks and filling them would leave, cell
+// by cell.
+template <typename T>
+__device__ __forceinline__ T filled_diff(const T *__restrict__ a, const T *__restrict__ a1, const T *e,
+                                         const LevelView &lv, const Signs &sg, int bi, int64_t blk, int x, int y) {
+  auto diff = [&](int64_t X, int o) { return dadd<T>(a[X * kSS + o], -a1[X * kSS + o]); };
+  const int fr = x < kG ? -1 : x >= kG + kM ? 1 : 0, fz = y < kG ? -1 : y >= kG + kM ? 1 : 0;
+  const int o = x + kS * y;
+  if (!fr && !fz) return diff(blk, o);
+  const bool corner = fr && fz;
+  if (corner && !lv.cfaces) return diff(blk, o);
+  const int f = fr ? (fr < 0 ? 0 : 1) : (fz < 0 ? 2 : 3);
+  const int4 fi = corner ? lv.cfaces[4 * bi + (fr + 1) / 2 + (fz + 1)] : lv.faces[4 * bi + f];
+  if (fi.x == FACE_NEIGHBOR) return diff(fi.y, (x - kM * fr) + kS * (y - kM * fz));
+  if (fi.x == FACE_BOUNDARY) {
+    const int b0 = corner ? fi.z : fr, b1 = corner ? fi.w : fz;
+    const int mx = b0 < 0 ? 2 * kG - 1 - x : b0 > 0 ? 2 * (kG + kM) - 1 - x : x;
+    const int my = b1 < 0 ? 2 * kG - 1 - y : b1 > 0 ? 2 * (kG + kM) - 1 - y : y;
+    T v;
+    if (corner && (b0 == 0) != (b1 == 0)) {
+      // the mirror lands in the ghosts of the face along the zero component, filled by the
+      // copy and boundary passes (fill_corner_cell)
+      const int g = b0 == 0 ? (fr < 0 ? 0 : 1) : (fz < 0 ? 2 : 3);
+      const int4 ff = lv.faces[4 * bi + g];
+      const int gr = g < 2 ? 2 * g - 1 : 0, gz = g < 2 ? 0 : 2 * g - 5;
+      if (ff.x == FACE_NEIGHBOR) {
+        v = diff(ff.y, (mx - kM * gr) + kS * (my - kM * gz));
+      } else if (ff.x == FACE_BOUNDARY) {
+        const int nx = gr < 0 ? 2 * kG - 1 - mx : gr > 0 ? 2 * (kG + kM) - 1 - mx : mx;
+        const int ny = gz < 0 ? 2 * kG - 1 - my : gz > 0 ? 2 * (kG + kM) - 1 - my : my;
+        v = dmul<T>(T(sg.v[face_sign_index(g)]), diff(blk, nx + kS * ny));
+      } else {
+        v = diff(blk, mx + kS * my);
+      }
+    } else {
+      v = diff(blk, mx + kS * my);
+    }
+    return dmul<T>(T(sg.v[(1 + b0) + 3 * (1 + b1)]), v);
+  }
+  if (fi.x == FACE_REFBND) {
+    const T *cb = e + (int64_t)fi.y * kSS;
+    const int jr = fr < 0 ? 1 + 8 * fi.z : fr > 0 ? 2 + 8 * (fi.z - 1) : 2 + 8 * (fi.z - 1) + ((x - kG) >> 1);
+    const int jz = fz < 0 ? 1 + 8 * fi.w : fz > 0 ? 2 + 8 * (fi.w - 1) : 2 + 8 * (fi.w - 1) + ((y - kG) >> 1);
+    const int ir = x & 1, iz = y & 1, q = jr + kS * jz;  // both ghost pairs start at an even index
+    T v = dmul<T>(T(0.5), cb[q]);
+    v = dadd<T>(v, dmul<T>(T(0.25), cb[q + (2 * ir - 1)]));
+    return dadd<T>(v, dmul<T>(T(0.25), cb[q + kS * (2 * iz - 1)]));
+  }
+  return diff(blk, o);
+}
+
+// The coarse correction e = u - u1 of a level with its ghosts filled (e's parent level filled
+// already), one launch instead of a difference and the fill passes.  e must be neither u nor u1.
+template <typename T>
+__device__ __forceinline__ void d_correction(T *__restrict__ e, const T *__restrict__ u, const T *__restrict__ u1,
+                                             const LevelView &lv, const Signs &sg) {
+  const int64_t total = (int64_t)lv.nblk * kSS;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int bi = (int)(t / kSS), c = (int)(t % kSS);
+    const int64_t blk = lv.blocks[bi].x;
+    e[blk * kSS + c] = filled_diff<T>(u, u1, e, lv, sg, bi, blk, c % kS, c / kS);
+  }
+}
+
+// interp_add_level! that also leaves u's ghosts filled: each updated cell is written to the
+// copy and mirror ghosts of it (PushView; nothing here reads a ghost of this level), and
+// the level's refinement ghosts are interpolated from its parent level.  pv.cbi gives the
+// index of a child edge's fine block in the level's block list.
+template <typename T>
+__device__ __forceinline__ void d_interp_push(T *__restrict__ u, const T *__restrict__ e, const LevelView &lv,
+                                              const PushView &pv, unsigned sw, const Signs &sg, bool refined) {
+  const int64_t total = (int64_t)lv.nch * 256;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int k = (int)(t >> 8), c = (int)(t & 255);
+    const int4 ch = lv.child[k];
+    const int dx = c & 15, dy = c >> 4;
+    const int ir = dx & 1, iz = dy & 1;
+    const int o = 2 + 8 * (ch.z - 1) + (dx >> 1) + kS * (2 + 8 * (ch.w - 1) + (dy >> 1));
+    const T *cb = e + (int64_t)ch.y * kSS;
+    T v = dmul<T>(T(0.5), cb[o]);
+    v = dadd<T>(v, dmul<T>(T(0.25), cb[o + (2 * ir - 1)]));
+    v = dadd<T>(v, dmul<T>(T(0.25), cb[o + kS * (2 * iz - 1)]));
+    T *d = u + (int64_t)ch.x * kSS + (2 + dx) + kS * (2 + dy);
+    v = dadd<T>(v, *d);
+    *d = v;
+    push_ghosts<T>(u, pv, sw, pv.cbi[k], 2 + dx, 2 + dy, v);
+  }
+  if (refined) d_fill_ghost<T>(u, lv, sg, 4);
+}
+
+// The saved copy of the coarse level (for the correction) and its FAS right-hand side under
+// the children of lf: both read the coarse u after its ghost fill.
+template <typename T>
+__device__ __forceinline__ void d_save_rhs(T *__restrict__ u1, T *__restrict__ b, const T *__restrict__ u,
+                                           const T *__restrict__ r, const LevelView &lc, const LevelView &lf,
+                                           const int2 *__restrict__ coord_of, const OpParams<T> &pc, const WTab<T> &wt) {
+  d_postrestrict<T>(b, u, r, lf, coord_of, pc, wt);
+  d_copy_level<T>(u1, u, lc);
+}
+
 // The kernels of the per-operation path: each a grid-stride loop over its work, so the
 // same bodies also run as the operations of one cooperative launch (srmg_seq.cu).
 template <typename T>
@@ -731,6 +918,109 @@ template <typename T>
 __global__ void k_gs4(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p, int p1, int p2) {
   pdl_enter();
   d_gs4<T>(u, b, lv, p, p1, p2);
+}
+
+template <typename T>
+__global__ void k_down(T *__restrict__ u, T *__restrict__ r, const T *__restrict__ b, LevelView lv,
+                       const int2 *__restrict__ coord_of, OpParams<T> p, WTab<T> wt) {
+  pdl_enter();
+  d_down<T>(u, r, b, lv, coord_of, p, wt);
+}
+
+template <typename T>
+__global__ void k_save_rhs(T *__restrict__ u1, T *__restrict__ b, const T *__restrict__ u, const T *__restrict__ r,
+                           LevelView lc, LevelView lf, const int2 *__restrict__ coord_of, OpParams<T> pc, WTab<T> wt) {
+  pdl_enter();
+  d_save_rhs<T>(u1, b, u, r, lc, lf, coord_of, pc, wt);
+}
+
+template <typename T>
+__global__ void k_correction(T *__restrict__ e, const T *__restrict__ u, const T *__restrict__ u1, LevelView lv,
+                             Signs sg) {
+  pdl_enter();
+  d_correction<T>(e, u, u1, lv, sg);
+}
+
+template <typename T>
+__global__ void k_interp_push(T *__restrict__ u, const T *__restrict__ e, LevelView lv, PushView pv, unsigned sw,
+                              Signs sg, bool refined) {
+  pdl_enter();
+  d_interp_push<T>(u, e, lv, pv, sw, sg, refined);
+}
+
+// The coarse end of a fused V-cycle in one CTA: levels 1..top (each of at most
+// kLocalBlocks blocks), every step a body above over the CTA's threads with a CTA barrier
+// after it.  A step costs a barrier and L1 latencies (~0.6 us) where a launch costs ~3 us, and
+// levels of 1, 4 and 16 blocks have ~75 of them a cycle; above 16 blocks one SM's fp64 rate
+// is the longer of the two (a colour of 64 blocks is 2 us of it).
+constexpr int kLocalBlocks = 16, kLocalLevels = 12;
+template <typename T>
+struct LocalCycle {
+  LevelView lv[kLocalLevels + 2];  // levels 1..top + 1
+  PushView pv[kLocalLevels + 1];
+  OpParams<T> p[kLocalLevels + 2];
+  T *u, *b, *r, *u1;
+  Signs sg;
+  unsigned sw, refined, mref;      // boundary table as bits; per-level bits
+  WTab<T> wt;
+  const int2 *coord_of;
+  int top, inner, known, ndown, ntop, nup;  // inner: level top + 1 exists and has been restricted;
+                                            // known: else, whether level top's ghosts are filled
+};
+
+// gauss_seidel_iter! with ghost pushes, n sweeps.  known: the ghosts are what a fill would
+// make of the cells now (else, and where boundary corners mirror refinement ghosts, the
+// first colour is followed by a fill).
+template <typename T>
+__device__ __forceinline__ void local_gs(const LocalCycle<T> &L, int l, int n, bool known) {
+  const bool four = L.p[l].op == 2;
+  for (int i = 0; i < n; ++i)
+    for (int c = 0; c < (four ? 4 : 2); ++c) {
+      const bool plain = i == 0 && c == 0 && (!known || ((L.mref >> l) & 1));
+      if (four) d_gs4_impl<T, true>(L.u, L.b, L.lv[l], L.p[l], c >> 1, c & 1, L.pv[l], L.sw);
+      else d_gs_colour_impl<T, true>(L.u, L.b, L.lv[l], L.p[l], L.wt, c, L.pv[l], L.sw);
+      __syncthreads();
+      if (plain) {
+        d_fill_ghost<T>(L.u, L.lv[l], L.sg, 3);
+        __syncthreads();
+      }
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(1024, 1) k_vcycle_local(const __grid_constant__ LocalCycle<T> L) {
+  pdl_enter();
+  auto down = [&](int l) {  // after level l's restriction
+    d_fill_ghost<T>(L.u, L.lv[l - 1], L.sg, (L.refined >> (l - 1)) & 1 ? 7 : 3);
+    __syncthreads();
+    d_save_rhs<T>(L.u1, L.b, L.u, L.r, L.lv[l - 1], L.lv[l], L.coord_of, L.p[l - 1], L.wt);
+    __syncthreads();
+  };
+  if (L.inner) down(L.top + 1);
+  for (int l = L.top; l >= 2; --l) {
+    local_gs<T>(L, l, L.ndown, L.known || L.inner || l < L.top);
+    d_down<T>(L.u, L.r, L.b, L.lv[l], L.coord_of, L.p[l], L.wt);
+    __syncthreads();
+    down(l);
+  }
+  local_gs<T>(L, 1, L.ntop, L.known || L.inner || L.top > 1);
+  for (int l = 2; l <= L.top; ++l) {
+    d_correction<T>(L.r, L.u, L.u1, L.lv[l - 1], L.sg);
+    __syncthreads();
+    d_interp_push<T>(L.u, L.r, L.lv[l], L.pv[l], L.sw, L.sg, (L.refined >> l) & 1);
+    __syncthreads();
+    local_gs<T>(L, l, L.nup, true);
+  }
+  if (L.inner) d_correction<T>(L.r, L.u, L.u1, L.lv[L.top], L.sg);
+}
+
+// FMG's step up to level lf: level lf saved, and the correction of the level below it.
+template <typename T>
+__global__ void k_fmg_step(T *__restrict__ e, T *__restrict__ u1, const T *__restrict__ u, LevelView lf, LevelView lc,
+                           Signs sg) {
+  pdl_enter();
+  d_correction<T>(e, u, u1, lc, sg);
+  d_copy_level<T>(u1, u, lf);
 }
 
 // The colour sweeps with their ghost pushes (PushView).

@@ -148,7 +148,7 @@ extern "C" int srmg_electric_field_dev(srmg_ctx *ctx, double *e, double *eabs, c
   if (ctx->max_blk > 0) {
     const int grid = (int)std::min<int64_t>(ctx->max_blk, 148 * 5);
     const auto kern = (reinterpret_cast<uintptr_t>(u) & 15) == 0 ? k_efield<16> : k_efield<8>;
-    kern<<<grid, 256, 0, ctx->stream>>>(e, eabs, u, ctx->d_info, (int)ctx->max_blk, h, 1.0 / h, e0[0], e0[1]);
+    kern<<<grid, 256, 0, ctx->stream>>>(e, eabs, u, ctx->d_info, (int)ctx->max_blk, h, recip_of(h), e0[0], e0[1]);
     ctx->launches++;
   }
   CK(cudaGetLastError());

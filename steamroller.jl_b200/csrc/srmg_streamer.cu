@@ -312,7 +312,7 @@ bool aligned16(std::initializer_list<const void *> ps) {
 CellSize cell_size(double h, const srmg_transport &tr) {
   volatile double hh = h * h;
   volatile double q = hh / tr.D;
-  return CellSize{h, 1.0 / h, q / 4.0};
+  return CellSize{h, recip_of(h), q / 4.0};
 }
 
 int check_transport(srmg_ctx *ctx, const srmg_transport *tr, const char *who) {
