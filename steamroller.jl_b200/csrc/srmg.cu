@@ -973,10 +973,15 @@ static int L_gs_colour_push(srmg_ctx *ctx, T *u, const T *b, int l, const OpPara
   const int threads = 128;
   const OpParams<T> p = tabled(ctx, p0);
   const unsigned sw = sign_bits(sg);
-  if (p.op == SRMG_OP_LAPLACIAN4)
-    launch_pdl(k_gs4_push<T>, grid_for((int64_t)L.nblk * 64, threads, kGridCap), threads, 0, ctx->stream, u, b, L.view(l), p, parity >> 1, parity & 1, ctx->push_lv[l - 1], sw);
-  else
-    launch_pdl(k_gs_colour_push<T>, grid_for((int64_t)L.nblk * 128, threads, kGridCap), threads, 0, ctx->stream, u, b, L.view(l), p, wtab<T>(ctx), parity, ctx->push_lv[l - 1], sw);
+  const bool four = p.op == SRMG_OP_LAPLACIAN4;
+  const auto kern = four ? (p.geom == 0   ? k_gs_push<T, true, 0>
+                            : p.geom == 1 ? k_gs_push<T, true, 1>
+                                          : k_gs_push<T, true, 2>)
+                         : (p.geom == 0   ? k_gs_push<T, false, 0>
+                            : p.geom == 1 ? k_gs_push<T, false, 1>
+                                          : k_gs_push<T, false, 2>);
+  launch_pdl(kern, grid_for((int64_t)L.nblk * (four ? 64 : 128), threads, kGridCap), threads, 0, ctx->stream, u, b,
+             L.view(l), p, wtab<T>(ctx), four ? parity >> 1 : parity, four ? parity & 1 : 0, ctx->push_lv[l - 1], sw);
   ctx->launches++;
   return SRMG_OK;
 }
@@ -1078,9 +1083,10 @@ int srmg::L_diff(srmg_ctx *ctx, T *dst, const T *a1, const T *a2, int l) {
 // mirrors, refinement ghosts are interpolated once the parent level is final -- so of the
 // reference's fills only the one after the restriction remains, besides the one after the
 // first colour on the finest level (the caller's ghosts are not known) and on levels whose
-// boundary corners mirror refinement ghosts.  Levels 1..top, at most kLocalBlocks blocks
-// each, run in one CTA.  On the 2725-block order-4 tree a cycle is 131 kernels instead of
-// 281 and 1.98 -> see DESIGN ms for two cycles.
+// boundary corners mirror refinement ghosts.  On the 2725-block order-4 tree a cycle is 190
+// kernels instead of 281 and 501 us instead of 990.  (Its coarse levels in one CTA, fields in shared memory, or in one
+// cluster, fields in global memory, were no faster than launches: a colour of 16 blocks is
+// bound by one SM's shared memory, 3.4 us, and one of a cluster by two trips to L2, 2.0 us.)
 template <typename T>
 static int vcycle_fused(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, double k2, int geom, const Signs &sg,
                         int lmax, int ndown, int ntop, int nup, double omega) {
@@ -1103,57 +1109,23 @@ static int vcycle_fused(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op
       }
     return SRMG_OK;
   };
-  int top = 0;
-  while (top < lmax && top < kLocalLevels && ctx->lv[top].nblk > 0 && ctx->lv[top].nblk <= kLocalBlocks) ++top;
-  const int lo = std::max(top, 1);
-  for (int l = lmax; l > lo; l--) {
+  for (int l = lmax; l > 1; l--) {
     const DevLevel &L = ctx->lv[l - 1], &C = ctx->lv[l - 2];
     RC(gs(l, ndown, filled || l < lmax));
     launch_pdl(k_down<T>, grid_for((int64_t)L.nch * 64, 128, kGridCap), 128, 0, ctx->stream, u, r, b, L.view(l),
                ctx->d_coord_of, par(l), wtab<T>(ctx));
     ctx->launches++;
-    if (l - 1 == top) break;  // k_vcycle_local takes it from here
     RC(L_fill_ghost<T>(ctx, u, l - 1, sg, 7));
     launch_pdl(k_save_rhs<T>, grid_for((int64_t)C.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, u1, b, u, r,
                C.view(l - 1), L.view(l), ctx->d_coord_of, par(l - 1), wtab<T>(ctx));
     ctx->launches++;
   }
-  if (top >= 1) {
-    LocalCycle<T> A;
-    memset(&A, 0, sizeof A);
-    for (int l = 1; l <= std::min(top + 1, lmax); l++) {
-      A.lv[l] = ctx->lv[l - 1].view(l);
-      A.p[l] = par(l);
-      if (l <= top) A.pv[l] = ctx->push_lv[l - 1];
-    }
-    A.u = u;
-    A.b = b;
-    A.r = r;
-    A.u1 = u1;
-    A.sg = sg;
-    A.sw = sw;
-    A.refined = ctx->refbnd_levels;
-    A.mref = ctx->mref_levels;
-    A.wt = wtab<T>(ctx);
-    A.coord_of = ctx->d_coord_of;
-    A.top = top;
-    A.inner = lmax > top;
-    A.known = filled;
-    A.ndown = ndown;
-    A.ntop = ntop;
-    A.nup = nup;
-    launch_pdl(k_vcycle_local<T>, 1, 1024, 0, ctx->stream, A);
-    ctx->launches++;
-  } else {
-    RC(gs(1, ntop, filled || lmax > 1));
-  }
-  for (int l = lo + 1; l <= lmax; l++) {
+  RC(gs(1, ntop, filled || lmax > 1));
+  for (int l = 2; l <= lmax; l++) {
     const DevLevel &L = ctx->lv[l - 1], &C = ctx->lv[l - 2];
-    if (l - 1 != top) {
-      launch_pdl(k_correction<T>, grid_for((int64_t)C.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, r, u, u1,
-                 C.view(l - 1), sg);
-      ctx->launches++;
-    }
+    launch_pdl(k_correction<T>, grid_for((int64_t)C.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, r, u, u1,
+               C.view(l - 1), sg);
+    ctx->launches++;
     launch_pdl(k_interp_push<T>, grid_for((int64_t)L.nch * 256, 256, kGridCap), 256, 0, ctx->stream, u, r, L.view(l),
                ctx->push_lv[l - 1], sw, sg, refined(l));
     ctx->launches++;

@@ -60,7 +60,7 @@ struct LevelView {
 
 // The reciprocal div_by takes for a divisor: 1 / d, or 0 (plain divisions) where d is so small
 // or large that an intermediate result could leave the normal range.
-inline double recip_of(double d) {
+__host__ __device__ inline double recip_of(double d) {
   const double m = d < 0 ? -d : d;
   return m > 1e-90 && m < 1e90 ? 1.0 / d : 0.0;
 }
@@ -92,8 +92,9 @@ struct OpParams {
   T rs;          // 1 / s, correctly rounded
   const double *c4;  // order 4, cylindrical: kCoef4 coefficients per radial index, or null (formed per cell)
 };
-// Order-4 coefficients of one radial index: am, ap, em, cc, ep (coeffs9) and the diagonal.
-constexpr int kCoef4 = 6;
+// Order-4 coefficients of one radial index: am, ap, em, cc, ep (coeffs9), the diagonal and its
+// reciprocal (recip_of), as one 64-byte row.
+constexpr int kCoef4 = 8;
 
 // a / d with rd = 1 / d correctly rounded: div_by in double, the plain quotient in float.
 __device__ __forceinline__ double quot(double a, double d, double rd) { return div_by(a, d, rd); }
@@ -197,6 +198,24 @@ __device__ __forceinline__ void coeffs9(int geom, int64_t ir, int64_t iz, double
   }
 }
 
+// A row of the coefficient table, and the 9 coefficients it stands for.
+struct Row4 {
+  double am, ap, em, cc, ep, diag, rdiag;
+  __device__ __forceinline__ Row4() {}
+  __device__ __forceinline__ explicit Row4(const double *t) {
+    const double2 *v = reinterpret_cast<const double2 *>(t);
+    const double2 a = v[0], b = v[1], c = v[2], d = v[3];
+    am = a.x, ap = a.y, em = b.x, cc = b.y, ep = c.x, diag = c.y, rdiag = d.x;
+  }
+};
+__device__ __forceinline__ void spread9(const Row4 &r, int geom, double c[9]) {
+  if (geom == 1) {
+    c[0] = r.am; c[1] = 4; c[2] = r.ap; c[3] = r.em; c[4] = r.cc; c[5] = r.ep; c[6] = r.am; c[7] = 4; c[8] = r.ap;
+  } else {
+    c[0] = r.am; c[1] = r.em; c[2] = r.am; c[3] = 4; c[4] = r.cc; c[5] = 4; c[6] = r.ap; c[7] = r.ep; c[8] = r.ap;
+  }
+}
+
 // The same from the table of this radial index (k_coef4, the same operations): forming the
 // coefficients takes five divisions, more than the rest of a cell's update.
 __device__ __forceinline__ void coeffs9(const double *c4, int geom, int64_t ir, int64_t iz, double c[9]) {
@@ -204,13 +223,7 @@ __device__ __forceinline__ void coeffs9(const double *c4, int geom, int64_t ir, 
     coeffs9(geom, ir, iz, c);
     return;
   }
-  const double *t = c4 + kCoef4 * (geom == 1 ? ir : iz);
-  const double am = t[0], ap = t[1], em = t[2], cc = t[3], ep = t[4];
-  if (geom == 1) {
-    c[0] = am; c[1] = 4; c[2] = ap; c[3] = em; c[4] = cc; c[5] = ep; c[6] = am; c[7] = 4; c[8] = ap;
-  } else {
-    c[0] = am; c[1] = em; c[2] = am; c[3] = 4; c[4] = cc; c[5] = 4; c[6] = ap; c[7] = ep; c[8] = ap;
-  }
+  spread9(Row4(c4 + kCoef4 * (geom == 1 ? ir : iz)), geom, c);
 }
 
 template <typename T>
@@ -246,6 +259,8 @@ static __global__ void k_coef4(double *__restrict__ tab, int n) {
   t[3] = c[4];
   t[4] = c[5];
   t[5] = diagelm4(1, i, 0);
+  t[6] = recip_of(t[5]);
+  t[7] = 0.0;
 }
 
 // 1-based global indices of local cell (x, y) of a block at 1-based coords (cr, cz)
@@ -376,10 +391,9 @@ __device__ __forceinline__ void push_ghosts(T *__restrict__ u, const PushView &p
   }
 }
 
-template <typename T, bool kPush>
-__device__ __forceinline__ void d_gs_colour_impl(T *__restrict__ u, const T *__restrict__ b, LevelView lv,
-                                                 OpParams<T> p, WTab<T> wt, int parity, PushView pv,
-                                                 unsigned sg) {
+template <typename T>
+__device__ __forceinline__ void d_gs_colour(T *__restrict__ u, const T *__restrict__ b, LevelView lv,
+                                            OpParams<T> p, WTab<T> wt, int parity) {
   const int64_t total = (int64_t)lv.nblk * 128;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -394,14 +408,7 @@ __device__ __forceinline__ void d_gs_colour_impl(T *__restrict__ u, const T *__r
     const T v = fma(p.s, b[(int64_t)bk.x * kSS + o], Lu);
     const T nv = fma(p.nwc, v, ub[o]);
     ub[o] = nv;
-    if (kPush) push_ghosts<T>(u, pv, sg, bi, x, y, nv);
   }
-}
-
-template <typename T>
-__device__ __forceinline__ void d_gs_colour(T *__restrict__ u, const T *__restrict__ b, LevelView lv,
-                                            OpParams<T> p, WTab<T> wt, int parity) {
-  d_gs_colour_impl<T, false>(u, b, lv, p, wt, parity, PushView{nullptr, nullptr, nullptr}, 0u);
 }
 
 // ---- residual (src/multigrid.jl:309-323, 349-354): r = -(b + Lu/s) ---------------
@@ -581,10 +588,41 @@ __global__ void __launch_bounds__(NT) k_reduce_sqrt(double *out,
 }
 
 // gauss_seidel!(..., FourColors{P1,P2}) (src/multigrid.jl:206-232): cells
-// (2 + 2a + p1, 2 + 2b + p2), u -= omega (Lu + s b) / c, unfused.
-template <typename T, bool kPush>
-__device__ __forceinline__ void d_gs4_impl(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p,
-                                           int p1, int p2, PushView pv, unsigned sg) {
+// (2 + 2a + p1, 2 + 2b + p2), u -= omega (Lu + s b) / c, unfused.  row4: the cell's
+// coefficient row in cylindrical geometry, from the table or (none built) formed here.
+template <typename T>
+__device__ __forceinline__ Row4 row4(const OpParams<T> &p, int64_t ir, int64_t iz) {
+  if (p.c4) return Row4(p.c4 + kCoef4 * (p.geom == 1 ? ir : iz));
+  Row4 r;
+  double c[9];
+  coeffs9(p.geom, ir, iz, c);
+  r.am = c[0];
+  r.ap = p.geom == 1 ? c[2] : c[6];
+  r.em = p.geom == 1 ? c[3] : c[1];
+  r.cc = c[4];
+  r.ep = p.geom == 1 ? c[5] : c[7];
+  r.diag = diagelm4(p.geom, ir, iz);
+  r.rdiag = 0.0;
+  return r;
+}
+// The update of the cell at uc in geometry GEOM.
+template <typename T, int GEOM>
+__device__ __forceinline__ T gs4_value(const T *uc, T bo, const OpParams<T> &p, const Row4 &r) {
+  double c[9];
+  if (GEOM == 0) coeffs9(0, 0, 0, c);
+  else spread9(r, GEOM, c);
+  T v = T(0);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) v = dadd<T>(v, dmul<T>(T(c[k]), uc[(k % 3 - 1) + kS * (k / 3 - 1)]));
+  const T Lu = quot(v, T(6), T(1) / T(6));
+  const T w = dmul<T>(p.omega, dadd<T>(Lu, dmul<T>(p.s, bo)));
+  const T upd = GEOM == 0 ? quot(w, T(-20.0 / 6.0), T(1.0 / (-20.0 / 6.0))) : quot(w, T(r.diag), T(r.rdiag));
+  return uc[0] - upd;
+}
+
+template <typename T>
+__device__ __forceinline__ void d_gs4(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p, int p1,
+                                      int p2) {
   const int64_t total = (int64_t)lv.nblk * 64;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -592,21 +630,14 @@ __device__ __forceinline__ void d_gs4_impl(T *__restrict__ u, const T *__restric
     const int x = 2 + 2 * (c & 7) + p1, y = 2 + 2 * (c >> 3) + p2;
     const int4 bk = lv.blocks[bi];
     T *ub = u + (int64_t)bk.x * kSS;
-    const int64_t ir = gidx(bk.y, x), iz = gidx(bk.z, y);
-    const T Lu = apply9<T>(ub, x, y, p.geom, ir, iz, p.c4);
     const int o = x + kS * y;
-    const T cdiag =
-        T(p.c4 && p.geom ? p.c4[kCoef4 * (p.geom == 1 ? ir : iz) + 5] : diagelm4(p.geom, ir, iz));
-    const T upd = dmul<T>(p.omega, dadd<T>(Lu, dmul<T>(p.s, b[(int64_t)bk.x * kSS + o]))) / cdiag;
-    const T nv = ub[o] - upd;
+    const Row4 r = p.geom ? row4(p, gidx(bk.y, x), gidx(bk.z, y)) : Row4();
+    const T bo = b[(int64_t)bk.x * kSS + o];
+    const T nv = p.geom == 1   ? gs4_value<T, 1>(ub + o, bo, p, r)
+                 : p.geom == 2 ? gs4_value<T, 2>(ub + o, bo, p, r)
+                               : gs4_value<T, 0>(ub + o, bo, p, r);
     ub[o] = nv;
-    if (kPush) push_ghosts<T>(u, pv, sg, bi, x, y, nv);
   }
-}
-
-template <typename T>
-__device__ __forceinline__ void d_gs4(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p, int p1, int p2) {
-  d_gs4_impl<T, false>(u, b, lv, p, p1, p2, PushView{nullptr, nullptr, nullptr}, 0u);
 }
 
 // rhs! over rhs_level! (src/multigrid.jl:363-388): q1 = R q on the valid cells.  Order
@@ -948,70 +979,75 @@ __global__ void k_interp_push(T *__restrict__ u, const T *__restrict__ e, LevelV
   d_interp_push<T>(u, e, lv, pv, sw, sg, refined);
 }
 
-// The coarse end of a fused V-cycle in one CTA: levels 1..top (each of at most
-// kLocalBlocks blocks), every step a body above over the CTA's threads with a CTA barrier
-// after it.  A step costs a barrier and L1 latencies (~0.6 us) where a launch costs ~3 us, and
-// levels of 1, 4 and 16 blocks have ~75 of them a cycle; above 16 blocks one SM's fp64 rate
-// is the longer of the two (a colour of 64 blocks is 2 us of it).
-constexpr int kLocalBlocks = 16, kLocalLevels = 12;
-template <typename T>
-struct LocalCycle {
-  LevelView lv[kLocalLevels + 2];  // levels 1..top + 1
-  PushView pv[kLocalLevels + 1];
-  OpParams<T> p[kLocalLevels + 2];
-  T *u, *b, *r, *u1;
-  Signs sg;
-  unsigned sw, refined, mref;      // boundary table as bits; per-level bits
-  WTab<T> wt;
-  const int2 *coord_of;
-  int top, inner, known, ndown, ntop, nup;  // inner: level top + 1 exists and has been restricted;
-                                            // known: else, whether level top's ghosts are filled
-};
-
-// gauss_seidel_iter! with ghost pushes, n sweeps.  known: the ghosts are what a fill would
-// make of the cells now (else, and where boundary corners mirror refinement ghosts, the
-// first colour is followed by a fill).
-template <typename T>
-__device__ __forceinline__ void local_gs(const LocalCycle<T> &L, int l, int n, bool known) {
-  const bool four = L.p[l].op == 2;
-  for (int i = 0; i < n; ++i)
-    for (int c = 0; c < (four ? 4 : 2); ++c) {
-      const bool plain = i == 0 && c == 0 && (!known || ((L.mref >> l) & 1));
-      if (four) d_gs4_impl<T, true>(L.u, L.b, L.lv[l], L.p[l], c >> 1, c & 1, L.pv[l], L.sw);
-      else d_gs_colour_impl<T, true>(L.u, L.b, L.lv[l], L.p[l], L.wt, c, L.pv[l], L.sw);
-      __syncthreads();
-      if (plain) {
-        d_fill_ghost<T>(L.u, L.lv[l], L.sg, 3);
-        __syncthreads();
-      }
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(1024, 1) k_vcycle_local(const __grid_constant__ LocalCycle<T> L) {
-  pdl_enter();
-  auto down = [&](int l) {  // after level l's restriction
-    d_fill_ghost<T>(L.u, L.lv[l - 1], L.sg, (L.refined >> (l - 1)) & 1 ? 7 : 3);
-    __syncthreads();
-    d_save_rhs<T>(L.u1, L.b, L.u, L.r, L.lv[l - 1], L.lv[l], L.coord_of, L.p[l - 1], L.wt);
-    __syncthreads();
+// The colour sweeps with their ghost pushes (PushView), the per-operation V-cycle's most
+// frequent kernels and a chain of latencies: block record, coefficients, cells, a dozen
+// dependent fp64 operations, then the push list and its entries.  All that comes from tables
+// -- everything but u and b -- is loaded before the wait for the previous kernel: a thread's
+// first cell (nearly always its only one) with up to two pushes.  u and b are not
+// __restrict__, so that their loads stay below it.  Up to ~16k cells a sweep the time does
+// not depend on the level's size: an order-4 sweep 1.7 us in a row of them (4.7 before, with
+// coefficients from nine fp64 divisions a cell and nothing ahead of the wait).
+template <typename T, bool FOUR, int GEOM>
+__global__ void __launch_bounds__(128) k_gs_push(T *u, const T *b, LevelView lv, OpParams<T> p, WTab<T> wt, int p1,
+                                                 int p2, PushView pv, unsigned sg) {
+  constexpr int N = FOUR ? 64 : 128;  // cells of a colour per block
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int total = lv.nblk * N, stride = gridDim.x * blockDim.x;  // a field holds fewer than 2^31 values here
+  struct Cell {
+    int at, e0, e1;
+    int2 d0, d1;
+    Row4 r;   // FOUR
+    W5<T> w;  // red-black
   };
-  if (L.inner) down(L.top + 1);
-  for (int l = L.top; l >= 2; --l) {
-    local_gs<T>(L, l, L.ndown, L.known || L.inner || l < L.top);
-    d_down<T>(L.u, L.r, L.b, L.lv[l], L.coord_of, L.p[l], L.wt);
-    __syncthreads();
-    down(l);
+  auto load = [&](int t) {
+    Cell q;
+    const int bi = t / N, c = t % N;
+    const int y = FOUR ? 2 + 2 * (c >> 3) + p2 : 2 + (c >> 3);
+    const int x = 2 + 2 * (c & 7) + (FOUR ? p1 : ((p1 ^ (y + 1)) & 1));
+    const int *off = pv.off + bi * 256 + (x - kG) + kM * (y - kG);
+    const int4 bk = lv.blocks[bi];
+    q.e0 = off[0];
+    q.e1 = off[1];
+    q.at = bk.x * kSS + x + kS * y;
+    if (q.e0 < q.e1) q.d0 = pv.ent[q.e0];
+    if (q.e0 + 1 < q.e1) q.d1 = pv.ent[q.e0 + 1];
+    if (FOUR) {
+      if (GEOM) q.r = row4(p, gidx(bk.y, x), gidx(bk.z, y));
+    } else {
+      q.w = weights<T>(wt, GEOM, bk.y, bk.z, x, y);
+    }
+    return q;
+  };
+  auto push = [&](int2 d, T v) {
+    if (d.y != 255) {  // mirrors on the way
+      const int k1 = d.y & 15, k2 = d.y >> 4;
+      if (k1 < 9) v = dmul<T>(T((int)((sg >> (2 * k1)) & 3u) - 1), v);
+      if (k2 < 9) v = dmul<T>(T((int)((sg >> (2 * k2)) & 3u) - 1), v);
+    }
+    u[d.x] = v;
+  };
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  Cell q;
+  if (t < total) q = load(t);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  while (t < total) {
+    T *uc = u + q.at;
+    const T bo = b[q.at];
+    T nv;
+    if (FOUR) {
+      nv = gs4_value<T, GEOM>(uc, bo, p, q.r);
+    } else {
+      const T v = fma(p.s, bo, apply5<T>(uc, 0, 0, q.w, p.centre));
+      nv = fma(p.nwc, v, uc[0]);
+    }
+    *uc = nv;
+    if (q.e0 < q.e1) push(q.d0, nv);
+    if (q.e0 + 1 < q.e1) push(q.d1, nv);
+    for (int e = q.e0 + 2; e < q.e1; ++e) push(pv.ent[e], nv);
+    if (total - t <= stride) break;
+    t += stride;
+    q = load(t);
   }
-  local_gs<T>(L, 1, L.ntop, L.known || L.inner || L.top > 1);
-  for (int l = 2; l <= L.top; ++l) {
-    d_correction<T>(L.r, L.u, L.u1, L.lv[l - 1], L.sg);
-    __syncthreads();
-    d_interp_push<T>(L.u, L.r, L.lv[l], L.pv[l], L.sw, L.sg, (L.refined >> l) & 1);
-    __syncthreads();
-    local_gs<T>(L, l, L.nup, true);
-  }
-  if (L.inner) d_correction<T>(L.r, L.u, L.u1, L.lv[L.top], L.sg);
 }
 
 // FMG's step up to level lf: level lf saved, and the correction of the level below it.
@@ -1021,21 +1057,6 @@ __global__ void k_fmg_step(T *__restrict__ e, T *__restrict__ u1, const T *__res
   pdl_enter();
   d_correction<T>(e, u, u1, lc, sg);
   d_copy_level<T>(u1, u, lf);
-}
-
-// The colour sweeps with their ghost pushes (PushView).
-template <typename T>
-__global__ void k_gs_colour_push(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p,
-                                 WTab<T> wt, int parity, PushView pv, unsigned sg) {
-  pdl_enter();
-  d_gs_colour_impl<T, true>(u, b, lv, p, wt, parity, pv, sg);
-}
-
-template <typename T>
-__global__ void k_gs4_push(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p, int p1, int p2,
-                           PushView pv, unsigned sg) {
-  pdl_enter();
-  d_gs4_impl<T, true>(u, b, lv, p, p1, p2, pv, sg);
 }
 
 }  // namespace srmg
