@@ -581,6 +581,10 @@ int srmg_ssprk3_stage_dev(srmg_ctx *ctx, double *out, const double *n, const dou
  *                      after it (bit-identical results; tables built once per tree from
  *                      the fill itself, trees whose fill the tables cannot express keep
  *                      the fill launches); 0 = a fill launch after every colour;
+ *   "coarse_cluster"   1 (default) = the coarse levels of an FP64 V-cycle on a 2D tree (up to
+ *                      256 blocks each, as many as fit) run in one thread-block cluster
+ *                      with their fields in shared memory (bit-identical results);
+ *                      0 = as the finer ones;
  *   "direct_level"     the level of the FP64 direct coarsest solve of mixed and
  *                      SRMG_MODE_FP64_DIRECT solves on the persistent kernel: 0 (default)
  *                      = level 2 for a lone tree whose level 2 holds 1..4 blocks and has no

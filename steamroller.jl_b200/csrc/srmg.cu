@@ -4,6 +4,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 #include <algorithm>
 #include <unordered_map>
 #include <vector>
@@ -109,6 +110,8 @@ void srmg::free_tree(srmg_ctx *ctx) {
   ctx->coef4 = DevBuf{};
   ctx->push_lv.clear();
   ctx->push_state = 0;
+  if (ctx->coarse.tab.p) cudaFree(ctx->coarse.tab.p);
+  ctx->coarse = CoarseTab{};
 }
 
 extern "C" void srmg_destroy(srmg_ctx *ctx) {
@@ -1077,16 +1080,37 @@ int srmg::L_diff(srmg_ctx *ctx, T *dst, const T *a1, const T *a2, int l) {
 
 // ------------------------------------------------------------------ V-cycle / FMG
 
+// Levels 1..top of a cycle with finest level lmax in one cluster; filled: level top's ghosts are
+// filled (else, on lmax == top, the caller's).
+static int coarse_levels(srmg_ctx *ctx, int top, double *u, double *b, double *r, double s, int op, double k2, int geom,
+                         const Signs &sg, int lmax, bool filled, int ndown, int ntop, int nup, double omega) {
+  CoarseCycle A;
+  memset(&A, 0, sizeof A);
+  for (int l = 1; l <= top; l++) A.p[l] = tabled(ctx, op_params<double>(op, geom, k2, level_scale(s, l), omega));
+  A.u = u;
+  A.b = b;
+  A.r = r;
+  A.sg = sg;
+  A.sw = sign_bits(sg);
+  A.wt = wtab<double>(ctx);
+  A.top = top;
+  A.inner = lmax > top;
+  A.known = filled;
+  A.ndown = ndown;
+  A.ntop = ntop;
+  A.nup = nup;
+  return coarse_launch(ctx, A, op == SRMG_OP_LAPLACIAN4, geom);
+}
+
 // The V-cycle on trees whose sweeps push their ghosts, with its steps fused (the same values
 // in u and in b; r and u1, scratch, end with other contents).  A level's ghosts stay what
 // a fill would make of them -- the sweeps and the prolongation push their cells' copies and
 // mirrors, refinement ghosts are interpolated once the parent level is final -- so of the
 // reference's fills only the one after the restriction remains, besides the one after the
 // first colour on the finest level (the caller's ghosts are not known) and on levels whose
-// boundary corners mirror refinement ghosts.  On the 2725-block order-4 tree a cycle is 190
-// kernels instead of 281 and 501 us instead of 990.  (Its coarse levels in one CTA, fields in shared memory, or in one
-// cluster, fields in global memory, were no faster than launches: a colour of 16 blocks is
-// bound by one SM's shared memory, 3.4 us, and one of a cluster by two trips to L2, 2.0 us.)
+// boundary corners mirror refinement ghosts.  The coarse levels run in one cluster
+// (srmg_coarse.cu).  On the 2725-block order-4 tree a cycle is 109 kernels instead of 281 and
+// 407 us instead of 990 (190 and 501 with launches down to level 1).
 template <typename T>
 static int vcycle_fused(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, double k2, int geom, const Signs &sg,
                         int lmax, int ndown, int ntop, int nup, double omega) {
@@ -1109,23 +1133,34 @@ static int vcycle_fused(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op
       }
     return SRMG_OK;
   };
-  for (int l = lmax; l > 1; l--) {
+  int top = 0;
+  if constexpr (std::is_same_v<T, double>)
+    if (ctx->use_coarse) top = coarse_top(ctx, lmax, four, geom);
+  for (int l = lmax; l > std::max(top, 1); l--) {
     const DevLevel &L = ctx->lv[l - 1], &C = ctx->lv[l - 2];
     RC(gs(l, ndown, filled || l < lmax));
     launch_pdl(k_down<T>, grid_for((int64_t)L.nch * 64, 128, kGridCap), 128, 0, ctx->stream, u, r, b, L.view(l),
                ctx->d_coord_of, par(l), wtab<T>(ctx));
     ctx->launches++;
+    if (l - 1 == top) break;  // the cluster takes it from here
     RC(L_fill_ghost<T>(ctx, u, l - 1, sg, 7));
     launch_pdl(k_save_rhs<T>, grid_for((int64_t)C.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, u1, b, u, r,
                C.view(l - 1), L.view(l), ctx->d_coord_of, par(l - 1), wtab<T>(ctx));
     ctx->launches++;
   }
-  RC(gs(1, ntop, filled || lmax > 1));
-  for (int l = 2; l <= lmax; l++) {
+  if (top >= 1) {
+    if constexpr (std::is_same_v<T, double>)
+      RC(coarse_levels(ctx, top, u, b, r, s, op, k2, geom, sg, lmax, filled, ndown, ntop, nup, omega));
+  } else {
+    RC(gs(1, ntop, filled || lmax > 1));
+  }
+  for (int l = std::max(top, 1) + 1; l <= lmax; l++) {
     const DevLevel &L = ctx->lv[l - 1], &C = ctx->lv[l - 2];
-    launch_pdl(k_correction<T>, grid_for((int64_t)C.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, r, u, u1,
-               C.view(l - 1), sg);
-    ctx->launches++;
+    if (l - 1 != top) {
+      launch_pdl(k_correction<T>, grid_for((int64_t)C.nblk * kSS, 256, kGridCap), 256, 0, ctx->stream, r, u, u1,
+                 C.view(l - 1), sg);
+      ctx->launches++;
+    }
     launch_pdl(k_interp_push<T>, grid_for((int64_t)L.nch * 256, 256, kGridCap), 256, 0, ctx->stream, u, r, L.view(l),
                ctx->push_lv[l - 1], sw, sg, refined(l));
     ctx->launches++;
@@ -1133,6 +1168,11 @@ static int vcycle_fused(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op
   }
   return SRMG_OK;
 }
+
+// Splitting the persistent kernel's V-cycle around the cluster costs two more launches (25 us),
+// and a level's ~6 phases there take 20 to 25 us, its steps in the cluster 10 to 14: worth it
+// from this many levels on.
+constexpr int kCoarseWorth = 3;
 
 template <typename T>
 int srmg::vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, double k2, int geom,
@@ -1151,10 +1191,33 @@ int srmg::vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, d
       ntop >= 1 && nup >= 1 && ctx->nlev <= 30 && !ctx->seq_rec) {
     ItemTabs tabs;
     const std::vector<ItemSpec> specs = uniform_items(ctx, s, op, k2, bc_of(sg).data());
+    int top = 0, L = lmax;
+    if constexpr (std::is_same_v<T, double>) {
+      if (ctx->use_coarse && unit_signs(sg) && !ctx->trace_on) {
+        RC(ensure_coarse(ctx));
+        while (L > 1 && ctx->lv[L - 1].nblk == 0) --L;
+        top = coarse_top(ctx, L, false, geom);
+        if (L > top && top < kCoarseWorth) top = 0;
+      }
+      if (top >= 1 && L <= top)
+        return coarse_levels(ctx, top, u, b, r, s, op, k2, geom, sg, L, false, ndown, ntop, nup, omega);
+    }
     RC(prepare_items(ctx, specs.data(), geom, omega, false, 0, 0.0, &tabs));
+    if constexpr (std::is_same_v<T, double>) {
+      if (top >= 1) {
+        EngineRun run;
+        run.leg = 1;
+        run.leg_top = top;
+        RC(engine_vcycle<T>(ctx, u, b, u1, r, tabs, geom, L, ndown, ntop, nup, &run));
+        RC(coarse_levels(ctx, top, u, b, r, s, op, k2, geom, sg, L, false, ndown, ntop, nup, omega));
+        run.leg = 2;
+        return engine_vcycle<T>(ctx, u, b, u1, r, tabs, geom, L, ndown, ntop, nup, &run);
+      }
+    }
     return engine_vcycle<T>(ctx, u, b, u1, r, tabs, geom, lmax, ndown, ntop, nup);
   }
   RC(ensure_gs_push(ctx, op));
+  if (ctx->use_coarse) RC(ensure_coarse(ctx));
   // every level down to 1 has blocks, and each block of levels 2.. is some child edge's fine block
   bool whole = ctx->nlev <= 30 && ndown >= 1 && ntop >= 1 && nup >= 1 && ctx->lv[0].nblk > 0;
   for (int l = 2; l <= lmax; l++)
@@ -1306,6 +1369,10 @@ extern "C" int srmg_set_option(srmg_ctx *ctx, const char *key, int64_t value) {
     ctx->use_gs_push = value != 0;
     drop_op_graphs(ctx);
   }
+  else if (!strcmp(key, "coarse_cluster")) {
+    ctx->use_coarse = value != 0;
+    drop_op_graphs(ctx);
+  }
   else if (!strcmp(key, "op_graphs")) {
     ctx->use_op_graphs = value != 0;
     if (!ctx->use_op_graphs) drop_op_graphs(ctx);
@@ -1370,7 +1437,8 @@ int srmg::vcycle_ops(srmg_ctx *ctx, double *u, double *b, double *r, double *u1,
   const bool seq = ctx->use_op_seq;
   if (!(ctx->use_op_graphs || seq) || ncycles <= 0 || cap != cudaStreamCaptureStatusNone)
     return run_vcycles(ctx, u, b, r, u1, s, op, k2, geom, bc, lmax, ndown, ntop, nup, omega, ncycles);
-  RC(ensure_gs_push(ctx, op));  // before the key: a graph bakes in whether the sweeps push
+  RC(ensure_gs_push(ctx, op));
+  if (ctx->use_coarse) RC(ensure_coarse(ctx));  // before the key: a graph bakes in whether the sweeps push
   std::vector<char> key;
   for (const void *p : {(const void *)u, (const void *)b, (const void *)r, (const void *)u1, (const void *)ctx->d_tree,
                         (const void *)ctx->stream})

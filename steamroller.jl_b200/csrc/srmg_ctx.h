@@ -51,6 +51,14 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
+// The coarse levels' tables for k_vcycle_coarse (srmg_coarse.cu): state 0 = not built for this
+// tree, 1 = built, -1 = not used on it.
+struct CoarseTab {
+  int state = 0, levels = 0, slots = 0, tabq = 0, pbase[kCoarseLevels + 2] = {};
+  int base[kCoarseLevels + 2] = {}, nblk[kCoarseLevels + 1] = {}, per[kCoarseLevels + 1] = {};
+  DevBuf tab;
+};
+
 // Operator of one item (an independent problem of the context's forest).
 struct ItemSpec {
   double s = 1.0;
@@ -122,6 +130,8 @@ struct srmg_ctx {
   srmg::DevBuf push_tab;
   std::vector<srmg::PushView> push_lv;      // per level, index l-1
   unsigned mref_levels = 0;                 // bit l: boundary corners of level l mirror refinement ghosts
+  bool use_coarse = true;                   // coarse levels of an FP64 V-cycle in one cluster
+  srmg::CoarseTab coarse;
   srmg::DevBuf coef4;                       // order-4 coefficients per radial index (BoxStencil trees)
   bool trace_on = false;
   srmg::DevBuf trace;        // %globaltimer stamps after every engine phase (CTA 0)

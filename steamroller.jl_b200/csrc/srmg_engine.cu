@@ -41,18 +41,20 @@ int engine_threads_of(const srmg_ctx *ctx) {
 }
 
 template <typename T>
-const void *engine_kernel(int threads) {
-  return threads == kEngineNarrow ? (const void *)k_engine_vcycle<T, kEngineNarrow>
-                                  : (const void *)k_engine_vcycle<T, kEngineWide>;
+const void *engine_kernel(int threads, bool legs) {
+  if constexpr (sizeof(T) == 8)
+    if (legs) return engine_legs_kernel(threads);
+  return threads == kEngineNarrow ? (const void *)k_engine_vcycle<T, kEngineNarrow, false>
+                                  : (const void *)k_engine_vcycle<T, kEngineWide, false>;
 }
 
 template <typename T>
-int engine_grid(srmg_ctx *ctx, int threads, int *grid) {
+int engine_grid(srmg_ctx *ctx, int threads, bool legs, int *grid) {
   if (ctx->num_sms == 0) CK(cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, ctx->device));
   const size_t smem = engine_smem_bytes<T>(threads);
-  CK(cudaFuncSetAttribute(engine_kernel<T>(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(engine_kernel<T>(threads, legs), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, engine_kernel<T>(threads), threads, smem));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, engine_kernel<T>(threads, legs), threads, smem));
   if (per_sm < 1) return fail(ctx, SRMG_ERR_CUDA, "engine kernel cannot be resident (occupancy 0)");
   *grid = ctx->num_sms * std::min(per_sm, 1);
   return SRMG_OK;
@@ -118,10 +120,11 @@ template <typename T>
 static int engine_launch(srmg_ctx *ctx, EngArgs<T> &A) {
   int grid = 0;
   const int threads = engine_threads_of(ctx);
-  RC(engine_grid<T>(ctx, threads, &grid));  // also raises the dynamic shared-memory limit
+  const bool legs = A.leg != 0;
+  RC(engine_grid<T>(ctx, threads, legs, &grid));  // also raises the dynamic shared-memory limit
   if (ctx->engine_ctas > 0 && ctx->engine_ctas < grid) grid = ctx->engine_ctas;
   void *args[] = {&A};
-  CK(cudaLaunchCooperativeKernel(engine_kernel<T>(threads), dim3(grid), dim3(threads), args,
+  CK(cudaLaunchCooperativeKernel(engine_kernel<T>(threads, legs), dim3(grid), dim3(threads), args,
                                  engine_smem_bytes<T>(threads), ctx->stream));
   ctx->launches++;
   return SRMG_OK;
@@ -154,6 +157,11 @@ int srmg::engine_vcycle(srmg_ctx *ctx, T *u, T *b, T *u1, T *e, const ItemTabs &
   A.nup = nup;
   A.local_top = engine_local_top(ctx, L);
   A.top = 1;
+  if (run->leg) {
+    A.leg = run->leg;
+    A.top = run->leg_top;
+    A.local_top = 0;
+  }
   if (run->direct && tabs.P) {
     A.it_P = tabs.P;
     if (tabs.top == 2 && L >= 2) {

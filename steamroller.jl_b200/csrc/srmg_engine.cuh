@@ -87,6 +87,7 @@ struct EngArgs {
   int ndown, ntop, nup;
   int local_top;     // levels 1..local_top run inside CTA 0
   int top;           // the coarsest level a V-cycle visits: 1, or 2 (a lone item's direct solve there)
+  int leg;           // 0 = the whole V-cycle, 1 = the descent to level top only, 2 = the ascent from it only
   int smooth_level;  // > 0: run smooth_n GS iterations on this level only (gauss_seidel_iter!)
   int smooth_n;
   int nitems;
@@ -1651,7 +1652,9 @@ constexpr size_t engine_smem_bytes(int threads) {
   return (size_t)(threads / 256) * sizeof(SlotSmem<T>);
 }
 
-template <typename T, int NT>
+// LEGS: one leg of a V-cycle (A.leg); its own instance, so that the registers of the whole
+// cycle's stay as they are (with the test in it a mixed solve took 1.2% longer).
+template <typename T, int NT, bool LEGS>
 __global__ void __launch_bounds__(NT, 1) k_engine_vcycle(const __grid_constant__ EngArgs<T> A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SlotSmem<T> *smem = reinterpret_cast<SlotSmem<T> *>(smem_raw);
@@ -1675,7 +1678,7 @@ __global__ void __launch_bounds__(NT, 1) k_engine_vcycle(const __grid_constant__
   slot_sync(slot);
   if (A.nitems == 1) {
     int used = 0;
-    for (int l = 1; l <= A.lmax; ++l) {
+    for (int l = LEGS ? A.top + 1 : 1; l <= A.lmax; ++l) {
       const bool loc = l <= A.local_top;
       if (loc && blockIdx.x != 0) continue;
       const int first = loc ? slot : blockIdx.x * nslots + slot, step = loc ? nslots : gridDim.x * nslots;
@@ -1825,10 +1828,11 @@ __global__ void __launch_bounds__(NT, 1) k_engine_vcycle(const __grid_constant__
 
   // One FAS V-cycle (src/multigrid.jl:60-106) on the current fields.
   auto vcycle_body = [&]() -> bool {
-    cur = 0;
-    // descending leg, down to the level above the coarsest one visited
     const int lt = A.top;
-    for (int l = L; l >= lt + 1; --l) {
+    // levels that the descent of an earlier launch left in the second buffer
+    cur = LEGS && A.leg == 2 && (A.ndown & 1) ? (2u << L) - (2u << lt) : 0;
+    // descending leg, down to the level above the coarsest one visited
+    for (int l = LEGS && A.leg == 2 ? lt : L; l >= lt + 1; --l) {
       const bool loc = l <= K;
       for (int it = 0; it < A.ndown; ++it) {
         bool ok = true;
@@ -1842,8 +1846,10 @@ __global__ void __launch_bounds__(NT, 1) k_engine_vcycle(const __grid_constant__
       if (runs(loc)) okr = ph_restrict<T>(A, l, fld(l), fld(l - 1), first_of(loc), step_of(loc), t, slot, S, pk);
       if (!sync(okr, loc, (l - 1) <= K)) return false;
     }
+    if (LEGS && A.leg == 1) return true;
     // coarsest level
-    if (A.it_P && lt == 2) {
+    if (LEGS) {
+    } else if (A.it_P && lt == 2) {
       // a lone item's direct solve on level 2, grid-wide (never CTA-local: local_top = 0)
       ph_direct2_rhs<T>(A, fld(2), 2, s_rhs, s_direct);
       const int n2 = 256 * A.it_lrange[1].y;

@@ -45,6 +45,12 @@ void free_tree(srmg_ctx *ctx);
 // where the sweeps of operator `op` do not push by rule (BoxStencil{3} or order 4).
 int ensure_gs_push(srmg_ctx *ctx, int op);
 int d3_ensure_push(srmg_ctx *ctx);
+// The coarse levels of an FP64 V-cycle in one cluster (srmg_coarse.cu): their tables (not while
+// the stream is capturing), how many levels from 1 up a cycle with finest level lmax gives it
+// (0: none), and the launch.
+int ensure_coarse(srmg_ctx *ctx);
+int coarse_top(const srmg_ctx *ctx, int lmax, bool four, int geom);
+int coarse_launch(srmg_ctx *ctx, CoarseCycle &A, bool four, int geom);
 void drop_op_graphs(srmg_ctx *ctx);
 // One cooperative launch of the sequencer over `nops` recorded operations (srmg_seq.cu).
 int seq_launch(srmg_ctx *ctx, const void *d_ops, int nops);
@@ -142,11 +148,13 @@ struct EngineRun {
   int inner = 1;                     // mixed: FP32 V-cycles per defect-correction step
   int max_cycles = 0;                // > 0: device-side loop until every item has converged
   double tol = 0.0;                  // relative to each item's leaf norm of b
+  int leg = 0, leg_top = 0;          // vcycle!: 1 = only the descent to level leg_top, 2 = only the ascent from it
 };
 template <typename T>
 int engine_vcycle(srmg_ctx *ctx, T *u, T *b, T *u1, T *e, const ItemTabs &tabs, int geom, int lmax,
                   int ndown, int ntop, int nup, const EngineRun *run = nullptr);
 int engine_check(srmg_ctx *ctx);
+const void *engine_legs_kernel(int threads);  // the persistent kernel for EngineRun::leg (FP64)
 template <typename T>
 int engine_smooth(srmg_ctx *ctx, T *u, const T *b, const ItemTabs &tabs, int geom, int level, int n);
 // Copy the per-item results of the last device loop ({norm, |b|, initial, cycles} per

@@ -69,12 +69,12 @@ __host__ __device__ inline double recip_of(double d) {
 // product a rd by the exact remainder.  The first makes q faithful (off by less than one
 // unit in the last place), so that by Markstein's theorem (IBM J. Res. Dev. 34, 1990) the
 // second gives the correctly rounded quotient, as long as nothing leaves the normal range;
-// there, and for zeros, infinities and NaN, the division itself is called.
+// there, and for infinities and NaN, the division itself is called.
 __device__ __forceinline__ double div_by(double a, double d, double rd) {
   // the exponent field: 2^-700 <= |a| < 2^700 (an integer test; the fp64 pipe is the bound),
   // and a reciprocal from recip_of
   if ((unsigned)((__double2hiint(a) & 0x7ff00000) - (323 << 20)) >= (1400u << 20) || __double2hiint(rd) == 0)
-    return __ddiv_rn(a, d);
+    return a == 0.0 && rd != 0.0 ? __dmul_rn(a, rd) : __ddiv_rn(a, d);
   double q = __dmul_rn(a, rd);
   q = fma(fma(-q, d, a), rd, q);
   return fma(fma(-q, d, a), rd, q);
@@ -277,9 +277,13 @@ __device__ __forceinline__ T lhs_apply(const T *ub, int x, int y, const OpParams
 }
 
 // ---- ghost fill (src/connectivity.jl:155-258) --------------------------------------
+// Tile X of a field: a block's values in a field in memory (srmg_coarse.cu has fields whose
+// tiles lie in the shared memories of a cluster).
 template <typename T>
-__device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelView &lv, const Signs &sg, int phase,
-                                                 int64_t t);
+__device__ __forceinline__ T *tile_of(T *u, int64_t X) { return u + X * kSS; }
+
+template <typename T, class F>
+__device__ __forceinline__ void fill_corner_cell(F u, const LevelView &lv, const Signs &sg, int phase, int64_t t);
 
 // One warp per block, a lane one cell of each face: lane -> (layer g = lane/16, position
 // k = lane%16).  The fill is a chain of dependent scattered loads (record, value, store), so
@@ -291,12 +295,13 @@ __device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelV
 // copy and boundary passes, a warp barrier, then interpolation -- a boundary corner mirrors
 // its own block's refinement ghosts as they were before the fill, and no pass reads
 // another block's ghosts of this level, so one launch does all three.
-template <typename T>
-__device__ __forceinline__ void d_fill_ghost(T *__restrict__ u, LevelView lv, Signs sg, int mask) {
+template <typename T, class F>
+__device__ __forceinline__ void d_fill_ghost(F u, LevelView lv, Signs sg, int mask, int cta = blockIdx.x,
+                                             int ctas = gridDim.x) {
   const int lane = threadIdx.x & 31;
   const int g = lane >> 4, k = lane & 15;
-  const int stride = gridDim.x * (blockDim.x >> 5);
-  for (int bi = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); bi < lv.nblk; bi += stride) {
+  const int stride = ctas * (blockDim.x >> 5);
+  for (int bi = cta * (blockDim.x >> 5) + (threadIdx.x >> 5); bi < lv.nblk; bi += stride) {
     int type[4], src[4];
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
@@ -304,7 +309,7 @@ __device__ __forceinline__ void d_fill_ghost(T *__restrict__ u, LevelView lv, Si
       type[f] = r.x;
       src[f] = r.y;
     }
-    T *ub = u + (int64_t)lv.blocks[bi].x * kSS;
+    T *ub = tile_of(u, lv.blocks[bi].x);
     T v[4];
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
@@ -313,7 +318,7 @@ __device__ __forceinline__ void d_fill_ghost(T *__restrict__ u, LevelView lv, Si
         // _fill_ghost_copy! (src/connectivity.jl:184-198): ghost <- neighbour's valid
         // cell M positions away along the face normal.
         const int sx = f == 0 ? x + kM : f == 1 ? x - kM : x, sy = f == 2 ? y + kM : f == 3 ? y - kM : y;
-        if (mask & 1) v[f] = u[(int64_t)src[f] * kSS + sx + kS * sy];
+        if (mask & 1) v[f] = tile_of(u, src[f])[sx + kS * sy];
       } else if (type[f] == FACE_BOUNDARY) {
         // fill_ghost_bnd! (src/connectivity.jl:217-231), mirrorghost (src/blockfield.jl:513-521)
         const int mx = f == 0 ? 2 * kG - 1 - x : f == 1 ? 2 * (kG + kM) - 1 - x : x;
@@ -340,7 +345,7 @@ __device__ __forceinline__ void d_fill_ghost(T *__restrict__ u, LevelView lv, Si
         // the coarse source cell and the 0/1 child offsets per dimension.
         const int x = f == 0 ? g : f == 1 ? 18 + g : 2 + k, y = f == 2 ? g : f == 3 ? 18 + g : 2 + k;
         const int4 fi = lv.faces[4 * bi + f];
-        const T *cb = u + (int64_t)fi.y * kSS;
+        const T *cb = tile_of(u, fi.y);
         const int sbr = fi.z, sbz = fi.w;
         const int jr = f == 0 ? 1 + 8 * sbr : f == 1 ? 2 + 8 * (sbr - 1) : 2 + 8 * (sbr - 1) + (k >> 1);
         const int jz = f == 2 ? 1 + 8 * sbz : f == 3 ? 2 + 8 * (sbz - 1) : 2 + 8 * (sbz - 1) + (k >> 1);
@@ -605,16 +610,20 @@ __device__ __forceinline__ Row4 row4(const OpParams<T> &p, int64_t ir, int64_t i
   r.rdiag = 0.0;
   return r;
 }
-// The update of the cell at uc in geometry GEOM.
+// apply9 at the cell at uc in geometry GEOM, and the cell's update.
 template <typename T, int GEOM>
-__device__ __forceinline__ T gs4_value(const T *uc, T bo, const OpParams<T> &p, const Row4 &r) {
+__device__ __forceinline__ T sum9(const T *uc, const Row4 &r) {
   double c[9];
   if (GEOM == 0) coeffs9(0, 0, 0, c);
   else spread9(r, GEOM, c);
   T v = T(0);
 #pragma unroll
   for (int k = 0; k < 9; ++k) v = dadd<T>(v, dmul<T>(T(c[k]), uc[(k % 3 - 1) + kS * (k / 3 - 1)]));
-  const T Lu = quot(v, T(6), T(1) / T(6));
+  return quot(v, T(6), T(1) / T(6));
+}
+template <typename T, int GEOM>
+__device__ __forceinline__ T gs4_value(const T *uc, T bo, const OpParams<T> &p, const Row4 &r) {
+  const T Lu = sum9<T, GEOM>(uc, r);
   const T w = dmul<T>(p.omega, dadd<T>(Lu, dmul<T>(p.s, bo)));
   const T upd = GEOM == 0 ? quot(w, T(-20.0 / 6.0), T(1.0 / (-20.0 / 6.0))) : quot(w, T(r.diag), T(r.rdiag));
   return uc[0] - upd;
@@ -687,12 +696,12 @@ __global__ void k_rhs(T *__restrict__ q1, const T *__restrict__ q, LevelView lv,
 // source -- the neighbour's valid cell, or the mirrored valid cell -- with the same
 // operations as the face pass, instead of reading it.  Interpolation (mask 4) follows: the
 // boundary pass reads a refinement face's ghosts as they were before this fill.
-template <typename T>
-__device__ __forceinline__ T face_ghost_value(const T *__restrict__ u, const T *ub, const LevelView &lv,
+template <typename T, class F>
+__device__ __forceinline__ T face_ghost_value(F u, const T *ub, const LevelView &lv,
                                               const Signs &sg, int bi, int f, int x, int y) {
   const int4 ff = lv.faces[4 * bi + f];
   if (ff.x == FACE_NEIGHBOR) {  // as the copy pass of d_fill_ghost
-    const T *src = u + (int64_t)ff.y * kSS;
+    const T *src = tile_of(u, ff.y);
     int sx = x, sy = y;
     if (f == 0) sx = x + kM; else if (f == 1) sx = x - kM;
     else if (f == 2) sy = y + kM; else sy = y - kM;
@@ -707,9 +716,8 @@ __device__ __forceinline__ T face_ghost_value(const T *__restrict__ u, const T *
   return ub[x + kS * y];  // a refinement face: not written by the copy and boundary passes
 }
 
-template <typename T>
-__device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelView &lv, const Signs &sg, int mask,
-                                                 int64_t t) {
+template <typename T, class F>
+__device__ __forceinline__ void fill_corner_cell(F u, const LevelView &lv, const Signs &sg, int mask, int64_t t) {
   {
     const int bi = (int)(t >> 4), q = (int)((t >> 2) & 3), cell = (int)(t & 3);
     const int4 fi = lv.cfaces[4 * bi + q];
@@ -721,9 +729,9 @@ __device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelV
     const int fr = 2 * (q & 1) - 1, fz = 2 * (q >> 1) - 1;  // ghost direction
     const int ir = cell & 1, iz = cell >> 1;
     const int x = (fr < 0 ? 0 : kM + kG) + ir, y = (fz < 0 ? 0 : kM + kG) + iz;
-    T *ub = u + (int64_t)lv.blocks[bi].x * kSS;
+    T *ub = tile_of(u, lv.blocks[bi].x);
     if (type == FACE_NEIGHBOR) {
-      const T *src = u + (int64_t)fi.y * kSS;
+      const T *src = tile_of(u, fi.y);
       ub[x + kS * y] = src[(x - kM * fr) + kS * (y - kM * fz)];
     } else if (type == FACE_BOUNDARY) {
       const int b0 = fi.z, b1 = fi.w;
@@ -741,7 +749,7 @@ __device__ __forceinline__ void fill_corner_cell(T *__restrict__ u, const LevelV
       }
       ub[x + kS * y] = dmul<T>(a, src);
     } else {
-      const T *cb = u + (int64_t)fi.y * kSS;
+      const T *cb = tile_of(u, fi.y);
       const int sbr = fi.z, sbz = fi.w;
       // subblockbnd(subblock, -face): the last cell of the subblock along a dimension
       // where the ghost lies below, the first where it lies above
@@ -792,10 +800,10 @@ __device__ __forceinline__ void d_down(T *__restrict__ u, T *__restrict__ r, con
 // fill_ghost! of it, refinement ghosts interpolated from the parent level of e (already
 // filled): what copying or subtracting the whole blocks and filling them would leave, cell
 // by cell.
-template <typename T>
-__device__ __forceinline__ T filled_diff(const T *__restrict__ a, const T *__restrict__ a1, const T *e,
-                                         const LevelView &lv, const Signs &sg, int bi, int64_t blk, int x, int y) {
-  auto diff = [&](int64_t X, int o) { return dadd<T>(a[X * kSS + o], -a1[X * kSS + o]); };
+template <typename T, class F, class E>
+__device__ __forceinline__ T filled_diff(F a, F a1, E e, const LevelView &lv, const Signs &sg, int bi, int64_t blk,
+                                         int x, int y) {
+  auto diff = [&](int64_t X, int o) { return dadd<T>(tile_of(a, X)[o], -tile_of(a1, X)[o]); };
   const int fr = x < kG ? -1 : x >= kG + kM ? 1 : 0, fz = y < kG ? -1 : y >= kG + kM ? 1 : 0;
   const int o = x + kS * y;
   if (!fr && !fz) return diff(blk, o);
@@ -830,7 +838,7 @@ __device__ __forceinline__ T filled_diff(const T *__restrict__ a, const T *__res
     return dmul<T>(T(sg.v[(1 + b0) + 3 * (1 + b1)]), v);
   }
   if (fi.x == FACE_REFBND) {
-    const T *cb = e + (int64_t)fi.y * kSS;
+    const T *cb = tile_of(e, fi.y);
     const int jr = fr < 0 ? 1 + 8 * fi.z : fr > 0 ? 2 + 8 * (fi.z - 1) : 2 + 8 * (fi.z - 1) + ((x - kG) >> 1);
     const int jz = fz < 0 ? 1 + 8 * fi.w : fz > 0 ? 2 + 8 * (fi.w - 1) : 2 + 8 * (fi.w - 1) + ((y - kG) >> 1);
     const int ir = x & 1, iz = y & 1, q = jr + kS * jz;  // both ghost pairs start at an even index
@@ -1049,6 +1057,27 @@ __global__ void __launch_bounds__(128) k_gs_push(T *u, const T *b, LevelView lv,
     q = load(t);
   }
 }
+
+// The coarse end of a V-cycle as one cluster runs it (srmg_coarse.cu): up to kCoarseCtas blocks
+// per level and CTA slot, kCoarsePer slots a level.
+constexpr int kCoarseLevels = 12, kCoarseCtas = 16, kCoarsePer = 16, kCoarseThreads = 512;
+constexpr int kCoarseSmem = 227 * 1024;
+struct CoarseCycle {
+  OpParams<double> p[kCoarseLevels + 1];
+  double *u, *b, *r;
+  Signs sg;
+  WTab<double> wt;
+  unsigned sw;                // the boundary table as bits
+  int top, inner, known;      // inner: level top + 1 exists and has been restricted (residual in r);
+                              // known: else, whether level top's ghosts are filled
+  int ndown, ntop, nup;
+  // the tree's tables, set by coarse_launch
+  const int4 *tab;
+  int slots, levels, tabq, corners;
+  unsigned refined, mref;     // per-level bits
+  int base[kCoarseLevels + 2], nblk[kCoarseLevels + 1], per[kCoarseLevels + 1];  // slots of level l: base[l]..
+  int pbase[kCoarseLevels + 2];                                                  // pushes of level l: pbase[l]..
+};
 
 // FMG's step up to level lf: level lf saved, and the correction of the level below it.
 template <typename T>
