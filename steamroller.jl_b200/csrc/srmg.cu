@@ -1110,7 +1110,7 @@ static int coarse_levels(srmg_ctx *ctx, int top, double *u, double *b, double *r
 // first colour on the finest level (the caller's ghosts are not known) and on levels whose
 // boundary corners mirror refinement ghosts.  The coarse levels run in one cluster
 // (srmg_coarse.cu).  On the 2725-block order-4 tree a cycle is 109 kernels instead of 281 and
-// 407 us instead of 990 (190 and 501 with launches down to level 1).
+// 373 us instead of 990 (190 and ~460 with launches down to level 1).
 template <typename T>
 static int vcycle_fused(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, double k2, int geom, const Signs &sg,
                         int lmax, int ndown, int ntop, int nup, double omega) {

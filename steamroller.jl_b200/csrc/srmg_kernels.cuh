@@ -960,28 +960,28 @@ __global__ void k_gs4(T *__restrict__ u, const T *__restrict__ b, LevelView lv, 
 }
 
 template <typename T>
-__global__ void k_down(T *__restrict__ u, T *__restrict__ r, const T *__restrict__ b, LevelView lv,
+__global__ void __launch_bounds__(256, 1) k_down(T *__restrict__ u, T *__restrict__ r, const T *__restrict__ b, LevelView lv,
                        const int2 *__restrict__ coord_of, OpParams<T> p, WTab<T> wt) {
   pdl_enter();
   d_down<T>(u, r, b, lv, coord_of, p, wt);
 }
 
 template <typename T>
-__global__ void k_save_rhs(T *__restrict__ u1, T *__restrict__ b, const T *__restrict__ u, const T *__restrict__ r,
+__global__ void __launch_bounds__(256, 1) k_save_rhs(T *__restrict__ u1, T *__restrict__ b, const T *__restrict__ u, const T *__restrict__ r,
                            LevelView lc, LevelView lf, const int2 *__restrict__ coord_of, OpParams<T> pc, WTab<T> wt) {
   pdl_enter();
   d_save_rhs<T>(u1, b, u, r, lc, lf, coord_of, pc, wt);
 }
 
 template <typename T>
-__global__ void k_correction(T *__restrict__ e, const T *__restrict__ u, const T *__restrict__ u1, LevelView lv,
+__global__ void __launch_bounds__(256, 1) k_correction(T *__restrict__ e, const T *__restrict__ u, const T *__restrict__ u1, LevelView lv,
                              Signs sg) {
   pdl_enter();
   d_correction<T>(e, u, u1, lv, sg);
 }
 
 template <typename T>
-__global__ void k_interp_push(T *__restrict__ u, const T *__restrict__ e, LevelView lv, PushView pv, unsigned sw,
+__global__ void __launch_bounds__(256, 1) k_interp_push(T *__restrict__ u, const T *__restrict__ e, LevelView lv, PushView pv, unsigned sw,
                               Signs sg, bool refined) {
   pdl_enter();
   d_interp_push<T>(u, e, lv, pv, sw, sg, refined);
@@ -991,19 +991,20 @@ __global__ void k_interp_push(T *__restrict__ u, const T *__restrict__ e, LevelV
 // frequent kernels and a chain of latencies: block record, coefficients, cells, a dozen
 // dependent fp64 operations, then the push list and its entries.  All that comes from tables
 // -- everything but u and b -- is loaded before the wait for the previous kernel: a thread's
-// first cell (nearly always its only one) with up to two pushes.  u and b are not
+// first cell (nearly always its only one) with its pushes.  u and b are not
 // __restrict__, so that their loads stay below it.  Up to ~16k cells a sweep the time does
 // not depend on the level's size: an order-4 sweep 1.7 us in a row of them (4.7 before, with
 // coefficients from nine fp64 divisions a cell and nothing ahead of the wait).
 template <typename T, bool FOUR, int GEOM>
-__global__ void __launch_bounds__(128) k_gs_push(T *u, const T *b, LevelView lv, OpParams<T> p, WTab<T> wt, int p1,
+__global__ void __launch_bounds__(128, 1) k_gs_push(T *u, const T *b, LevelView lv, OpParams<T> p, WTab<T> wt, int p1,
                                                  int p2, PushView pv, unsigned sg) {
   constexpr int N = FOUR ? 64 : 128;  // cells of a colour per block
+  constexpr int kAhead = 3;           // a cell by a block's corner has that many pushes
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int total = lv.nblk * N, stride = gridDim.x * blockDim.x;  // a field holds fewer than 2^31 values here
   struct Cell {
     int at, e0, e1;
-    int2 d0, d1;
+    int2 d[kAhead];
     Row4 r;   // FOUR
     W5<T> w;  // red-black
   };
@@ -1017,8 +1018,9 @@ __global__ void __launch_bounds__(128) k_gs_push(T *u, const T *b, LevelView lv,
     q.e0 = off[0];
     q.e1 = off[1];
     q.at = bk.x * kSS + x + kS * y;
-    if (q.e0 < q.e1) q.d0 = pv.ent[q.e0];
-    if (q.e0 + 1 < q.e1) q.d1 = pv.ent[q.e0 + 1];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (q.e0 + k < q.e1) q.d[k] = pv.ent[q.e0 + k];
     if (FOUR) {
       if (GEOM) q.r = row4(p, gidx(bk.y, x), gidx(bk.z, y));
     } else {
@@ -1049,9 +1051,10 @@ __global__ void __launch_bounds__(128) k_gs_push(T *u, const T *b, LevelView lv,
       nv = fma(p.nwc, v, uc[0]);
     }
     *uc = nv;
-    if (q.e0 < q.e1) push(q.d0, nv);
-    if (q.e0 + 1 < q.e1) push(q.d1, nv);
-    for (int e = q.e0 + 2; e < q.e1; ++e) push(pv.ent[e], nv);
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (q.e0 + k < q.e1) push(q.d[k], nv);
+    for (int e = q.e0 + kAhead; e < q.e1; ++e) push(pv.ent[e], nv);
     if (total - t <= stride) break;
     t += stride;
     q = load(t);
