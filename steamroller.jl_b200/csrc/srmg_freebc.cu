@@ -18,7 +18,7 @@
 // x_1) and C_k = 2 Re(e^{-i pi k / 2n} V_k); DST-III(X)[k] = (-1)^k DCT-III(X'')[k] with
 // X''_j = X_{n-1-j}, and DCT-III through the inverse reordering of an unnormalised
 // inverse FFT of W^{-k} (X''_k - i X''_{n-k}).  For n <= 8192 the gather, both FFTs
-// (radix-2 stages, two per pass over shared memory) and the steps between them run in
+// (radix-2 stages, four per pass over shared memory) and the steps between them run in
 // one CTA in shared memory; above, a
 // four-step n = n1 n2 split (n2 column FFTs with twiddles, then n1 row FFTs) per
 // transform, twiddles from a table of e^{-2 pi i k / n}.  Other n run as direct
@@ -109,7 +109,7 @@ __global__ void k_twiddles(double2 *tw, int64_t n) {
 }
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_double2(fma(-a.y, b.y, a.x * b.x), fma(a.y, b.x, a.x * b.y));
 }
 
 // `count` forward FFTs of length len (a power of two, <= kFftMaxLocal), one per CTA
@@ -237,12 +237,12 @@ __global__ void k_dst3_post(double *__restrict__ b, const double2 *__restrict__ 
 
 // ---- the whole transform in one CTA (n a power of two, n <= kFftMaxLocal) -----------
 
-constexpr int kLocalThreads = 1024;
+constexpr int kLocalThreads = 512;  // 16 complex values a thread in registers
 
-// Shared-memory index of element i: one pad element after every eight, so that the
-// power-of-two strides of the butterflies and of the twiddle reads fall on different
-// banks (16-byte elements, a quarter-warp of 8 threads per 128-byte wavefront).
-__device__ __forceinline__ int spad(int i) { return i + (i >> 3); }
+// Shared-memory index of element i, padded so that the accesses of a quarter-warp (8 elements
+// of 16 bytes, a 128-byte wavefront) fall on different banks: runs, the strides of 16 of the
+// last pass, those of 16 to 128 of the twiddles, and bit-reversed runs.
+__host__ __device__ constexpr int spad(int i) { return i + (i >> 4) + (i >> 7) + (i >> 9); }
 
 // Decimation in time: a' = a + w c, c' = a - w c.
 __device__ __forceinline__ void bfly_dit(double2 &a, double2 &c, double2 w) {
@@ -259,80 +259,61 @@ __device__ __forceinline__ void bfly_dif(double2 &a, double2 &c, double2 w) {
 }
 
 // In-place radix-2 FFTs over buf (padded, spad) with the twiddles W^k = e^{-2 pi i k / n},
-// k < n / 2, in shared memory (padded), two stages per pass over shared memory.
-// Decimation in frequency takes natural order to bit-reversed order: stages
-// half = n/2, n/4, ..., 1, a thread holding e_q = g + pos + q H/2 (q = 0..3, g a
-// multiple of 2H, pos < H/2) for the stage pair (H, H/2): (e0, e2) with W_{2H}^pos,
-// (e1, e3) with W_{2H}^(pos + H/2), then (e0, e1) and (e2, e3) with W_H^pos.
-__device__ __forceinline__ void local_fft_dif(double2 *buf, const double2 *stw, int n, int logn) {
-  int H = n / 2;
-  for (; H >= 2; H >>= 2) {
-    const int q = H / 2, t1 = n / (2 * H), t2 = n / H;
-    for (int idx = threadIdx.x; idx < n / 4; idx += blockDim.x) {
-      const int pos = idx & (q - 1), e0 = (idx - pos) * 4 + pos;
-      double2 a0 = buf[spad(e0)], a1 = buf[spad(e0 + q)], a2 = buf[spad(e0 + 2 * q)], a3 = buf[spad(e0 + 3 * q)];
-      bfly_dif(a0, a2, stw[spad(pos * t1)]);
-      bfly_dif(a1, a3, stw[spad((pos + q) * t1)]);
-      const double2 w2 = stw[spad(pos * t2)];
-      bfly_dif(a0, a1, w2);
-      bfly_dif(a2, a3, w2);
-      buf[spad(e0)] = a0;
-      buf[spad(e0 + q)] = a1;
-      buf[spad(e0 + 2 * q)] = a2;
-      buf[spad(e0 + 3 * q)] = a3;
+// k < n / 2, in shared memory (padded), LOG stages per pass over shared memory, up to four: a
+// thread holds the 2^LOG elements g + pos + q S (q = 0..2^LOG - 1, g a multiple of 2^LOG S,
+// pos < S) that those stages mix.  On one SM the passes are bound by shared-memory
+// instructions and their barriers, so that the fewer passes win: 4096 points in 3 passes
+// a transform instead of 6 (the same butterflies) and padded, the kernel 30 -> 17 us.
+// Decimation in frequency takes natural order to bit-reversed order, stages of half =
+// 2^(LOG-1) S, ..., S; decimation in time bit-reversed to natural, half = S, ..., 2^(LOG-1) S.
+// A stage's butterfly (i, i + half) takes W_{2 half}^(i mod half).
+template <int LOG, bool DIF>
+__device__ __forceinline__ void fft_pass(double2 *buf, const double2 *stw, int n, int S) {
+  constexpr int R = 1 << LOG;
+  for (int idx = threadIdx.x; idx < n / R; idx += blockDim.x) {
+    const int pos = idx & (S - 1), e0 = (idx - pos) * R + pos;
+    double2 a[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) a[q] = buf[spad(e0 + q * S)];
+#pragma unroll
+    for (int k = 0; k < LOG; ++k) {
+      const int hq = DIF ? R >> (k + 1) : 1 << k;  // half / S
+      const int t = n / (2 * hq * S);              // twiddle step
+#pragma unroll
+      for (int j = 0; j < R / 2; ++j) {
+        if (j >= hq) break;
+        const double2 w = stw[spad((pos + j * S) * t)];
+#pragma unroll
+        for (int q = 0; q < R; q += 1) {
+          if (q % (2 * hq) != j) continue;
+          if (DIF) bfly_dif(a[q], a[q + hq], w);
+          else bfly_dit(a[q], a[q + hq], w);
+        }
+      }
     }
-    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < R; ++q) buf[spad(e0 + q * S)] = a[q];
   }
-  if (H == 1) {  // an odd stage count ends with one radix-2 stage (twiddle 1)
-    for (int idx = threadIdx.x; idx < n / 2; idx += blockDim.x) {
-      double2 a = buf[spad(2 * idx)], c = buf[spad(2 * idx + 1)];
-      bfly_dif(a, c, stw[0]);
-      buf[spad(2 * idx)] = a;
-      buf[spad(2 * idx + 1)] = c;
-    }
-    __syncthreads();
-  }
+  __syncthreads();
 }
 
-// Decimation in time takes bit-reversed order to natural order: stages half = 1, 2,
-// ..., n/2 (the butterflies of k_fft), a thread holding g + pos + {0, h, 2h, 3h} (g a
-// multiple of 4h, pos < h) for the stage pair (h, 2h): (0, h) and (2h, 3h) with
-// W_{2h}^pos, then (0, 2h) with W_{4h}^pos and (h, 3h) with W_{4h}^(pos + h).
-__device__ __forceinline__ void local_fft_dit(double2 *buf, const double2 *stw, int n, int logn) {
-  int half = 1;
-  if (logn & 1) {  // one radix-2 stage first when the stage count is odd
-    for (int idx = threadIdx.x; idx < n / 2; idx += blockDim.x) {
-      double2 a = buf[spad(2 * idx)], c = buf[spad(2 * idx + 1)];
-      bfly_dit(a, c, stw[0]);
-      buf[spad(2 * idx)] = a;
-      buf[spad(2 * idx + 1)] = c;
-    }
-    __syncthreads();
-    half = 2;
-  }
-  for (; half < n; half <<= 2) {
-    const int t1 = n / (2 * half), t2 = n / (4 * half);
-    for (int idx = threadIdx.x; idx < n / 4; idx += blockDim.x) {
-      const int pos = idx & (half - 1), i = (idx - pos) * 4 + pos;
-      double2 a0 = buf[spad(i)], a1 = buf[spad(i + half)], a2 = buf[spad(i + 2 * half)],
-              a3 = buf[spad(i + 3 * half)];
-      const double2 w1 = stw[spad(pos * t1)];
-      bfly_dit(a0, a1, w1);
-      bfly_dit(a2, a3, w1);
-      bfly_dit(a0, a2, stw[spad(pos * t2)]);
-      bfly_dit(a1, a3, stw[spad((pos + half) * t2)]);
-      buf[spad(i)] = a0;
-      buf[spad(i + half)] = a1;
-      buf[spad(i + 2 * half)] = a2;
-      buf[spad(i + 3 * half)] = a3;
-    }
-    __syncthreads();
-  }
+template <bool DIF>
+__device__ __forceinline__ void local_fft(double2 *buf, const double2 *stw, int n, int logn) {
+  // the last pass of the one and the first of the other take what is left over of the stages
+  const int rest = logn & 3;
+  auto odd = [&] {
+    if (rest == 1) fft_pass<1, DIF>(buf, stw, n, 1);
+    else if (rest == 2) fft_pass<2, DIF>(buf, stw, n, 1);
+    else if (rest == 3) fft_pass<3, DIF>(buf, stw, n, 1);
+  };
+  if (!DIF) odd();
+#pragma unroll 1
+  for (int k = 0; k < logn >> 2; ++k) fft_pass<4, DIF>(buf, stw, n, DIF ? n >> (4 * (k + 1)) : 1 << (rest + 4 * k));
+  if (DIF) odd();
 }
 
-// Dynamic shared memory of k_dst_local: n + n/8 padded complex values and n/2 + n/16
-// padded twiddles (27 n bytes, 216 KB at n = 8192).
-constexpr int local_smem_bytes(int n) { return (int)sizeof(double2) * (n + n / 8 + n / 2 + n / 16); }
+// Dynamic shared memory of k_dst_local: the padded transform and twiddles (211 KB at n = 8192).
+constexpr int local_smem_bytes(int n) { return (int)sizeof(double2) * (spad(n) + spad(n / 2)); }
 
 // b = DST-III(f .* DST-II(getouter!(u))) h / 2^(level-1) / 2 in one CTA.  The gather
 // and the Makhoul reordering load the first FFT's input in natural order; that FFT
@@ -341,41 +322,75 @@ constexpr int local_smem_bytes(int n) { return (int)sizeof(double2) * (n + n / 8
 // (decimation in time) wants it, at the bit-reversed positions of m and n - m; that FFT
 // leaves natural order for the output reordering.  No permutation pass.
 __global__ void __launch_bounds__(kLocalThreads, 1)
-    k_dst_local(double *__restrict__ b, const FbcSrc *__restrict__ src, const double *__restrict__ u, double h,
+    k_dst_local(double *b, const FbcSrc *__restrict__ src, const double *u, double h, double rh,
                 const double2 *__restrict__ tw, const double2 *__restrict__ hw, const double *__restrict__ f, int n,
                 int logn, double p2) {
   extern __shared__ double2 sm[];
   double2 *buf = sm, *stw = sm + spad(n);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (int k = threadIdx.x; k < n / 2; k += blockDim.x) stw[spad(k)] = tw[k];
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    const double x = outer_value(src, u, h, j);
-    buf[spad((int)makhoul_pos(j, n))] = make_double2((j & 1) ? -x : x, 0.0);
-  }
-  __syncthreads();
-  local_fft_dif(buf, stw, n, logn);
-  auto brev = [&](int i) { return (int)(__brev((unsigned)i) >> (32 - logn)); };
-  for (int m = threadIdx.x; m <= n / 2; m += blockDim.x) {
-    const int mm = n - m;  // the partner position (m = 0 has none, m = n / 2 is its own)
-    const int am = spad(brev(m));
-    const double2 hm = hw[m];
-    const double cm = dct2_at(buf[am], hm);
-    if (m == 0) {
-      buf[am] = dst3_in(__dmul_rn(f[n - 1], cm), 0.0, hm);
-      continue;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // getouter!, several positions of a thread in flight: u / (h 2^-k), its reciprocal 2^k / h
+  constexpr int G = 8;
+  for (int j0 = threadIdx.x; j0 < n; j0 += G * blockDim.x) {
+    FbcSrc sj[G];
+    double x[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int j = j0 + g * blockDim.x;
+      if (j < n) sj[g] = src[j];
+      else sj[g].off = -1;
     }
-    const int amm = spad(brev(mm));
-    const double2 hmm = hw[mm];
-    const double cmm = dct2_at(buf[amm], hmm);
-    const double2 vm = dst3_in(__dmul_rn(f[n - 1 - m], cm), __dmul_rn(f[m - 1], cmm), hm);
-    if (mm != m) buf[amm] = dst3_in(__dmul_rn(f[n - 1 - mm], cmm), __dmul_rn(f[mm - 1], cm), hmm);
-    buf[am] = vm;
+#pragma unroll
+    for (int g = 0; g < G; ++g) x[g] = sj[g].off >= 0 ? u[sj[g].off] : 0.0;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int j = j0 + g * blockDim.x;
+      if (j >= n) break;
+      const double two = (double)((int64_t)1 << max(sj[g].level - 1, 0));
+      const double v = sj[g].off >= 0 ? div_by(x[g], h / two, __dmul_rn(rh, two)) : 0.0;
+      buf[spad((int)makhoul_pos(j, n))] = make_double2((j & 1) ? -v : v, 0.0);
+    }
   }
   __syncthreads();
-  local_fft_dit(buf, stw, n, logn);
+  local_fft<true>(buf, stw, n, logn);
+  auto brev = [&](int i) { return (int)(__brev((unsigned)i) >> (32 - logn)); };
+  constexpr int B = 4;  // values of m a thread has in flight
+  for (int m0 = threadIdx.x; m0 <= n / 2; m0 += B * blockDim.x) {
+    double2 h0[B], h1[B];
+    double f0[B], f1[B];  // f[n - 1 - m] and f[m - 1], the partner's the other way round
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      const int m = m0 + k * blockDim.x;
+      if (m > n / 2) break;
+      h0[k] = hw[m];
+      f0[k] = f[n - 1 - m];
+      if (m > 0) h1[k] = hw[n - m], f1[k] = f[m - 1];
+    }
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      const int m = m0 + k * blockDim.x, mm = n - m;  // the partner position (m = 0 has none, m = n / 2 is its own)
+      if (m > n / 2) break;
+      const int am = spad(brev(m));
+      const double cm = dct2_at(buf[am], h0[k]);
+      if (m == 0) {
+        buf[am] = dst3_in(__dmul_rn(f0[k], cm), 0.0, h0[k]);
+        continue;
+      }
+      const int amm = spad(brev(mm));
+      const double cmm = dct2_at(buf[amm], h1[k]);
+      const double2 vm = dst3_in(__dmul_rn(f0[k], cm), __dmul_rn(f1[k], cmm), h0[k]);
+      if (mm != m) buf[amm] = dst3_in(__dmul_rn(f1[k], cmm), __dmul_rn(f0[k], cm), h1[k]);
+      buf[am] = vm;
+    }
+  }
+  __syncthreads();
+  local_fft<false>(buf, stw, n, logn);
   for (int j = threadIdx.x; j < n / 2; j += blockDim.x) {
     const double ye = buf[spad(j)].x, yo = buf[spad(n - 1 - j)].x;  // as k_dst3_post
-    b[2 * j] = ye * h / p2 / 2.0;
-    b[2 * j + 1] = -yo * h / p2 / 2.0;
+    const double half = 0.5 / p2;  // a power of two
+    b[2 * j] = __dmul_rn(__dmul_rn(ye, h), half);
+    b[2 * j + 1] = __dmul_rn(__dmul_rn(-yo, h), half);
   }
 }
 
@@ -429,40 +444,58 @@ __device__ __forceinline__ double seg_mean(const double *b, int64_t first, int64
   for (int64_t m = 0; m < count; ++m) v = __dadd_rn(v, b[first + m]);
   return v / (double)count;
 }
+// By kMeanLanes lanes of a warp (the calling group's lane g of it), every one of them with the
+// result: on the coarsest level a cell's mean is of 256 values and more, and a sum by one
+// thread was the kernel's length (13.6 us, 4.9 by the lanes, on the 1.5M-cell channel tree).
+constexpr int kMeanLanes = 8;
+__device__ __forceinline__ double seg_mean(const double *b, int64_t first, int64_t count, int g) {
+  double v = 0.0;
+  for (int64_t m = g; m < count; m += kMeanLanes) v = __dadd_rn(v, b[first + m]);
+  const unsigned group = 0xffu << (threadIdx.x & 24);
+#pragma unroll
+  for (int o = kMeanLanes / 2; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_xor_sync(group, v, o));
+  return v / (double)count;
+}
 
 // factor(CylindricalGeometry{D}, J, delta) with delta along D (src/geometry.jl:27-29)
 __device__ __forceinline__ double cyl_factor(int64_t J) { return fabs(1.0 + 1.0 / (double)(2 * J - 1)); }
 
-// setouter! (src/freebc.jl:157-219) over every level in one launch: one thread per cell
+// setouter! (src/freebc.jl:157-219) over every level in one launch: kMeanLanes lanes per cell
 // of the outer valid column of each listed block (the blocks at the level's outer
-// extent, or with a boundary face at +dim).  The thread adds the boundary source
+// extent, or with a boundary face at +dim).  The first of them adds the boundary source
 // (src/freebc.jl:157-176) when the block's +dim face is a boundary, then -- for the
 // first and last cell of the column -- the refinement-boundary corrections that land
 // on it (src/freebc.jl:178-219), walking the connectivity's direction order (`order`
 // lists face codes: 0..3 star faces, 4..7 the corners).  Each cell belongs to one
-// block and one thread, so its additions happen in the reference's order: the level's
+// block and one group of lanes, so its additions happen in the reference's order: the level's
 // boundary sources before its refinement corrections, those in direction order.
-__global__ void k_setouter_all(double *__restrict__ q, const double *__restrict__ b, const LevelView *__restrict__ lvs,
+__global__ void __launch_bounds__(128, 1) k_setouter_all(double *q, const double *b, const LevelView *__restrict__ lvs,
                                const int2 *__restrict__ ent, int nent, int dim, int level, long long root_dim,
                                double s, int4 order_lo, int4 order_hi, int norder) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int order[8] = {order_lo.x, order_lo.y, order_lo.z, order_lo.w, order_hi.x, order_hi.y, order_hi.z, order_hi.w};
   const int fidx = dim == 1 ? 1 : 3;
-  const int64_t total = (int64_t)nent * kM;
+  const int64_t total = (int64_t)nent * kM * kMeanLanes;
+  const int g = threadIdx.x % kMeanLanes;
+  bool waited = false;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int e = (int)(t / kM), i = (int)(t % kM);
+    const int e = (int)(t / (kM * kMeanLanes)), i = (int)(t / kMeanLanes % kM);
     const int l = ent[e].x, bi = ent[e].y;
     const LevelView &lv = lvs[l - 1];
     const int4 bk = lv.blocks[bi];
+    const int outer = lv.faces[4 * bi + fidx].x;
+    if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+    waited = true;
     const int cd = dim == 1 ? bk.y : bk.z, co = dim == 1 ? bk.z : bk.y;
     const int64_t fl = (int64_t)1 << (l - 1);
     const double sl = s / (double)(fl * fl);
     const int64_t p = (int64_t)1 << (level - l);
     const int64_t Jd = (int64_t)kM * (cd - 1) + kM;
-    if (lv.faces[4 * bi + fidx].x == FACE_BOUNDARY) {
+    if (outer == FACE_BOUNDARY) {
       const int64_t i0 = (int64_t)(co - 1) * kM;
-      const double bmean = seg_mean(b, p * (i0 + i), p);
+      const double bmean = seg_mean(b, p * (i0 + i), p, g);
       double *qc = q + (int64_t)bk.x * kSS + cell_off(dim, kG + kM - 1, kG + i);
-      *qc = *qc + 2.0 * cyl_factor(Jd) * bmean / sl;
+      if (g == 0) *qc = *qc + 2.0 * cyl_factor(Jd) * bmean / sl;
     }
     if ((i != 0 && i != kM - 1) || cd != (int)(root_dim << (l - 1))) continue;
     for (int r = 0; r < norder; ++r) {
@@ -487,9 +520,9 @@ __global__ void k_setouter_all(double *__restrict__ q, const double *__restrict_
       // 0-based first element: dir = 1 reads b[p j + 1 : p (j + 2)], otherwise
       // b[p (j - 3) : p (j - 1) - 1] (1-based, as written in the reference)
       const int64_t first = dir == 1 ? p * j : p * (j - 3) - 1;
-      const double bmean = seg_mean(b, first, 2 * p);
+      const double bmean = seg_mean(b, first, 2 * p, g);
       double *qc = q + (int64_t)bk.x * kSS + cell_off(dim, kG + kM - 1, i1 - 1);
-      *qc = *qc + 2.0 * 0.25 * cyl_factor(J1d) * bmean / sl;
+      if (g == 0) *qc = *qc + 2.0 * 0.25 * cyl_factor(J1d) * bmean / sl;
     }
   }
 }
@@ -700,8 +733,8 @@ extern "C" int srmg_freebc_dev(srmg_ctx *ctx, double *q, const double *u, int64_
     // gather, DST-II, times f, DST-III: one CTA
     int logn = 0;
     while (((int64_t)1 << logn) < n) ++logn;
-    k_dst_local<<<1, kLocalThreads, local_smem_bytes((int)n), ctx->stream>>>(b, fbc_src(ctx), u, h, fbc_tw(ctx), fbc_hw(ctx), fbc_f(ctx), (int)n,
-                                                          logn, p2);
+    launch_pdl(k_dst_local, 1, kLocalThreads, local_smem_bytes((int)n), ctx->stream, b, fbc_src(ctx), u, h, recip_of(h),
+               fbc_tw(ctx), fbc_hw(ctx), fbc_f(ctx), (int)n, logn, p2);
     ctx->launches++;
   } else if (fbc_pow2(n) && !ctx->fbc_direct) {
     double2 *w0 = fbc_work(ctx, 0), *w1 = fbc_work(ctx, 1), *w2 = fbc_work(ctx, 2);
@@ -727,9 +760,8 @@ extern "C" int srmg_freebc_dev(srmg_ctx *ctx, double *q, const double *u, int64_
   const int4 olo = make_int4(ord[0], ord[1], ord[2], ord[3]);
   const int4 ohi = nord == 8 ? make_int4(ord[4], ord[5], ord[6], ord[7]) : make_int4(0, 0, 0, 0);
   if (ctx->fbc_nent > 0) {
-    k_setouter_all<<<gridfor((int64_t)ctx->fbc_nent * kM, 128), 128, 0, ctx->stream>>>(
-        q, b, fbc_lvs(ctx), fbc_ent(ctx), ctx->fbc_nent, dim, level, (long long)ctx->fbc_root[dim - 1], s, olo, ohi,
-        nord);
+    launch_pdl(k_setouter_all, gridfor((int64_t)ctx->fbc_nent * kM * kMeanLanes, 128), 128, 0, ctx->stream, q, b, fbc_lvs(ctx),
+               fbc_ent(ctx), ctx->fbc_nent, dim, level, (long long)ctx->fbc_root[dim - 1], s, olo, ohi, nord);
     ctx->launches++;
   }
   if (b_out) CK(cudaMemcpyAsync(b_out, b, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
