@@ -8,8 +8,11 @@
 // step is a cluster barrier (0.3 us), a stencil from shared memory (0.2) and those stores (0.2)
 // away from the next: latency all the way.  Two FP64 V-cycles (2, 4, 2) on the uniform tree of
 // 1 to 256 blocks, whole in the cluster: 231 -> 146 us; order 4 on the 2725-block tree, levels
-// of 1 to 64 blocks here: 164 -> 87 us of a cycle; full multigrid on the 400k-cell channel
-// tree: 1507 -> 1161 us.  The same with the fields in global memory took 2.0 us a colour.
+// of 1 to 64 blocks here: 164 -> 78 us of a cycle; full multigrid on the 400k-cell channel
+// tree: 1507 -> 1150 us.  The same with the fields in global memory took 2.0 us a colour.
+// 256 threads a CTA: a barrier costs more with more warps (512: 87 us of that cycle, 1024 on
+// the uniform tree 86 us a cycle instead of 73), and so do several cells a thread at a time
+// (two 82 us, four 92).
 #include <algorithm>
 
 #include "srmg_ctx.h"
@@ -199,8 +202,8 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_vcycle_coarse(const __gri
   };
   // gauss_seidel_iter! with ghost pushes, n sweeps.  known: the ghosts are what a fill would
   // make of the cells now (else, and where boundary corners mirror refinement ghosts, the
-  // first colour is followed by a fill).  A thread takes up to two cells at a time, what comes
-  // from tables loaded before the wait; the pushes follow from a list of their own, a thread
+  // first colour is followed by a fill).  What comes from tables is loaded before
+  // the wait; the pushes follow from a list of their own, a thread
   // each: at the cells, most lanes would wait for the few that have some, twice the time of
   // the rest.  A level of one block keeps to CTA 0's own barriers.
   auto gs = [&](int l, int n, bool known) {
@@ -244,21 +247,16 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_vcycle_coarse(const __gri
 #pragma unroll 1
       for (int c = 0; c < kColours; ++c) {
         int t = tid;
-        Cell k0, k1;
-        if (t < total) k0 = load(t, c);
-        if (t + kCoarseThreads < total) k1 = load(t + kCoarseThreads, c);
+        Cell k;
+        if (t < total) k = load(t, c);
         const int *run = head + 8 * (l - 1) + (FOUR ? kind(c) : 2 * c);
         const int i0 = run[0] + tid, i1 = run[FOUR ? 1 : 2];
         const int2 e = i0 < i1 ? ent[i0] : int2();
         wait();
         while (t < total) {
-          const bool two = t + kCoarseThreads < total;
-          const T v0 = value(k0);
-          if (two) su[k1.at] = value(k1);
-          su[k0.at] = v0;
-          t += 2 * kCoarseThreads;
-          if (t < total) k0 = load(t, c);
-          if (t + kCoarseThreads < total) k1 = load(t + kCoarseThreads, c);
+          su[k.at] = value(k);
+          t += kCoarseThreads;
+          if (t < total) k = load(t, c);
         }
         __syncthreads();
         push(i0, i1, e);

@@ -74,9 +74,9 @@ int srmg::engine_local_top(srmg_ctx *ctx, int lmax) {
 }
 
 // Launch state shared by every engine launch: tree tables, item tables, barrier and
-// error words, the frozen flags (zeroed) and norm scratch.
+// error words, the frozen flags (zeroed, but for a cycle's second leg) and norm scratch.
 template <typename T>
-static int engine_common(srmg_ctx *ctx, EngArgs<T> &A, T *u, const ItemTabs &tabs, int geom) {
+static int engine_common(srmg_ctx *ctx, EngArgs<T> &A, T *u, const ItemTabs &tabs, int geom, int leg = 0) {
   memset(&A, 0, sizeof A);
   A.u = u;
   {
@@ -112,7 +112,11 @@ static int engine_common(srmg_ctx *ctx, EngArgs<T> &A, T *u, const ItemTabs &tab
     RC(ensure(ctx, ctx->trace, kTraceMax * sizeof(long long)));
     A.trace = (long long *)ctx->trace.p;
   }
-  CK(cudaMemsetAsync(ctx->sync.p, 0, sync_bytes, ctx->stream));
+  if (leg == 2) {  // a counter of its own: the error word of the first leg stays
+    A.bar += 16;
+  } else {
+    CK(cudaMemsetAsync(ctx->sync.p, 0, sync_bytes, ctx->stream));
+  }
   return SRMG_OK;
 }
 
@@ -142,7 +146,7 @@ int srmg::engine_vcycle(srmg_ctx *ctx, T *u, T *b, T *u1, T *e, const ItemTabs &
     if (ctx->nblk_host[l - 1] > 0) L = l;
   if (L == 0) return SRMG_OK;
   EngArgs<T> A;
-  RC(engine_common<T>(ctx, A, u, tabs, geom));
+  RC(engine_common<T>(ctx, A, u, tabs, geom, run->leg));
   A.b = b;
   // Tolerance-driven solves run on the engine's own copy of b (FP64: a copy of the
   // caller's b; mixed: the FP32 defect), whose ghost cells then carry the neighbours'

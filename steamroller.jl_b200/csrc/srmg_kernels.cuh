@@ -1063,7 +1063,7 @@ __global__ void __launch_bounds__(128, 1) k_gs_push(T *u, const T *b, LevelView 
 
 // The coarse end of a V-cycle as one cluster runs it (srmg_coarse.cu): up to kCoarseCtas blocks
 // per level and CTA slot, kCoarsePer slots a level.
-constexpr int kCoarseLevels = 12, kCoarseCtas = 16, kCoarsePer = 16, kCoarseThreads = 512;
+constexpr int kCoarseLevels = 12, kCoarseCtas = 16, kCoarsePer = 16, kCoarseThreads = 256;
 constexpr int kCoarseSmem = 227 * 1024;
 struct CoarseCycle {
   OpParams<double> p[kCoarseLevels + 1];
