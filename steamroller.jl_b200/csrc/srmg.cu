@@ -1080,10 +1080,11 @@ int srmg::L_diff(srmg_ctx *ctx, T *dst, const T *a1, const T *a2, int l) {
 
 // ------------------------------------------------------------------ V-cycle / FMG
 
-// Levels 1..top of a cycle with finest level lmax in one cluster; filled: level top's ghosts are
-// filled (else, on lmax == top, the caller's).
+// Levels 1..top of a cycle with finest level lmax in one cluster (ncycles of them, where lmax ==
+// top); filled: level top's ghosts are filled (else, on lmax == top, the caller's).
 static int coarse_levels(srmg_ctx *ctx, int top, double *u, double *b, double *r, double s, int op, double k2, int geom,
-                         const Signs &sg, int lmax, bool filled, int ndown, int ntop, int nup, double omega) {
+                         const Signs &sg, int lmax, bool filled, int ndown, int ntop, int nup, double omega,
+                         int ncycles = 1) {
   CoarseCycle A;
   memset(&A, 0, sizeof A);
   for (int l = 1; l <= top; l++) A.p[l] = tabled(ctx, op_params<double>(op, geom, k2, level_scale(s, l), omega));
@@ -1099,6 +1100,7 @@ static int coarse_levels(srmg_ctx *ctx, int top, double *u, double *b, double *r
   A.ndown = ndown;
   A.ntop = ntop;
   A.nup = nup;
+  A.ncycles = ncycles;
   return coarse_launch(ctx, A, op == SRMG_OP_LAPLACIAN4, geom);
 }
 
@@ -1176,9 +1178,10 @@ constexpr int kCoarseWorth = 3;
 
 template <typename T>
 int srmg::vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, double k2, int geom,
-                     const Signs &sg, int lmax, int ndown, int ntop, int nup, double omega) {
+                     const Signs &sg, int lmax, int ndown, int ntop, int nup, double omega, int ncycles, int *ran) {
   if (lmax == 0) lmax = ctx->nlev;
   if (lmax < 1 || lmax > ctx->nlev) return fail(ctx, SRMG_ERR_BADARG, "lmax %d out of range", lmax);
+  if (ran) *ran = 1;
   // The persistent engine runs the whole cycle in one launch; r carries the coarse
   // corrections there.  Sweep counts of zero keep the per-operation kernels.
   // Bulk copies need 16-byte aligned block tiles.
@@ -1199,8 +1202,11 @@ int srmg::vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, d
         top = coarse_top(ctx, L, false, geom);
         if (L > top && top < kCoarseWorth) top = 0;
       }
-      if (top >= 1 && L <= top)
-        return coarse_levels(ctx, top, u, b, r, s, op, k2, geom, sg, L, false, ndown, ntop, nup, omega);
+      if (top >= 1 && L <= top) {
+        if (ran) *ran = ncycles;
+        return coarse_levels(ctx, top, u, b, r, s, op, k2, geom, sg, L, false, ndown, ntop, nup, omega,
+                             ran ? ncycles : 1);
+      }
     }
     RC(prepare_items(ctx, specs.data(), geom, omega, false, 0, 0.0, &tabs));
     if constexpr (std::is_same_v<T, double>) {
@@ -1256,9 +1262,9 @@ int srmg::vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, d
   return SRMG_OK;
 }
 template int srmg::vcycle_dev<double>(srmg_ctx *, double *, double *, double *, double *, double, int,
-                                      double, int, const Signs &, int, int, int, int, double);
+                                      double, int, const Signs &, int, int, int, int, double, int, int *);
 template int srmg::vcycle_dev<float>(srmg_ctx *, float *, float *, float *, float *, double, int,
-                                     double, int, const Signs &, int, int, int, int, double);
+                                     double, int, const Signs &, int, int, int, int, double, int, int *);
 
 static int finest_level(srmg_ctx *ctx) {
   int lmax = 0;
@@ -1532,8 +1538,8 @@ extern "C" int srmg_vcycle_dev(srmg_ctx *ctx, double *u, double *b, double *r, d
     return SRMG_OK;
   }
   const Signs sg = make_signs(bc);
-  for (int c = 0; c < ncycles; c++)
-    RC(vcycle_dev<double>(ctx, u, b, r, u1, s, op, k2, geom, sg, lmax, ndown, ntop, nup, omega));
+  for (int c = 0, ran = 1; c < ncycles; c += ran)
+    RC(vcycle_dev<double>(ctx, u, b, r, u1, s, op, k2, geom, sg, lmax, ndown, ntop, nup, omega, ncycles - c, &ran));
   CK(cudaGetLastError());
   return SRMG_OK;
 }

@@ -7,7 +7,7 @@
 // stay in one CTA, ghosts go to the neighbour's CTA by stores into its shared memory, and a
 // step is a cluster barrier (0.3 us), a stencil from shared memory (0.2) and those stores (0.2)
 // away from the next: latency all the way.  Two FP64 V-cycles (2, 4, 2) on the uniform tree of
-// 1 to 256 blocks, whole in the cluster: 231 -> 146 us; order 4 on the 2725-block tree, levels
+// 1 to 256 blocks, whole in the cluster: 231 -> 130 us (one launch; 146 as two); order 4 on the 2725-block tree, levels
 // of 1 to 64 blocks here: 164 -> 78 us of a cycle; full multigrid on the 400k-cell channel
 // tree: 1507 -> 1150 us.  The same with the fields in global memory took 2.0 us a colour.
 // 256 threads a CTA: a barrier costs more with more warps (512: 87 us of that cycle, 1024 on
@@ -285,59 +285,63 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_vcycle_coarse(const __gri
   };
   if (L.inner) arrive_at(top);
 #pragma unroll 1
-  for (int l = top; l >= 2; --l) {
-    gs(l, L.ndown, L.known || L.inner || l < top);
-    step([&] {
-      const OpParams<T> p = L.p[l];
-      for (int t = tid; t < own(l) * 64; t += kCoarseThreads) {
-        const int q = L.base[l] + (t >> 6), kx = t & 7, ky = (t >> 3) & 7;
-        const int4 ch = child[q];
-        T f = T(0), g = T(0);
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int x = 2 + 2 * kx + i, y = 2 + 2 * ky + j, o = x + kS * y;
-            f = dadd<T>(f, su[q * kSS + o]);
-            g = dadd<T>(g, -(sb[q * kSS + o] + quot(lhs(p, q, x, y), p.s, p.rs)));
-          }
-        const int o = (2 + 8 * (ch.z - 1) + kx) + kS * (2 + 8 * (ch.w - 1) + ky);
-        tile_of(fu, ch.y)[o] = dmul<T>(f, T(0.25));
-        tile_of(fe, ch.y)[o] = dmul<T>(g, T(0.25));
-      }
-    });
-    arrive_at(l - 1);
-  }
-  gs(1, L.ntop, L.known || L.inner || top > 1);
+  for (int cyc = 0; cyc < L.ncycles; ++cyc) {
+    const bool known = L.known || L.inner || cyc > 0;  // level top's ghosts
 #pragma unroll 1
-  for (int l = 2; l <= top; ++l) {
-    step([&] {
-      const LevelView lc = view(l - 1);
-      for (int t = tid; t < lc.nblk * kSS; t += kCoarseThreads) {
-        const int bi = t / kSS, o = t % kSS;
-        se[(L.base[l - 1] + bi) * kSS + o] = filled_diff<T>(fu, f1, fe, lc, L.sg, bi, lc.blocks[bi].x, o % kS, o / kS);
-      }
-    });
-    step([&] {
-      for (int t = tid; t < own(l) * 256; t += kCoarseThreads) {
-        const int q = L.base[l] + (t >> 8), dx = t & 15, dy = (t >> 4) & 15;
-        const int4 ch = child[q];
-        const int ir = dx & 1, iz = dy & 1;
-        const T *cb = tile_of(fe, ch.y) + 2 + 8 * (ch.z - 1) + (dx >> 1) + kS * (2 + 8 * (ch.w - 1) + (dy >> 1));
-        T v = dmul<T>(T(0.5), cb[0]);
-        v = dadd<T>(v, dmul<T>(T(0.25), cb[2 * ir - 1]));
-        v = dadd<T>(v, dmul<T>(T(0.25), cb[kS * (2 * iz - 1)]));
-        T *d = su + q * kSS + (2 + dx) + kS * (2 + dy);
-        v = dadd<T>(v, *d);
-        *d = v;
-      }
-      const int i = head[8 * (l - 1)] + tid, end = head[8 * (l - 1) + 4];
-      const int2 first = i < end ? ent[i] : int2();
-      __syncthreads();
-      push(i, end, first);
-      if ((L.refined >> l) & 1) d_fill_ghost<T>(fu, view(l), L.sg, 4, 0, 1);
-    });
-    gs(l, L.nup, true);
+    for (int l = top; l >= 2; --l) {
+      gs(l, L.ndown, known || l < top);
+      step([&] {
+        const OpParams<T> p = L.p[l];
+        for (int t = tid; t < own(l) * 64; t += kCoarseThreads) {
+          const int q = L.base[l] + (t >> 6), kx = t & 7, ky = (t >> 3) & 7;
+          const int4 ch = child[q];
+          T f = T(0), g = T(0);
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const int x = 2 + 2 * kx + i, y = 2 + 2 * ky + j, o = x + kS * y;
+              f = dadd<T>(f, su[q * kSS + o]);
+              g = dadd<T>(g, -(sb[q * kSS + o] + quot(lhs(p, q, x, y), p.s, p.rs)));
+            }
+          const int o = (2 + 8 * (ch.z - 1) + kx) + kS * (2 + 8 * (ch.w - 1) + ky);
+          tile_of(fu, ch.y)[o] = dmul<T>(f, T(0.25));
+          tile_of(fe, ch.y)[o] = dmul<T>(g, T(0.25));
+        }
+      });
+      arrive_at(l - 1);
+    }
+    gs(1, L.ntop, known || top > 1);
+#pragma unroll 1
+    for (int l = 2; l <= top; ++l) {
+      step([&] {
+        const LevelView lc = view(l - 1);
+        for (int t = tid; t < lc.nblk * kSS; t += kCoarseThreads) {
+          const int bi = t / kSS, o = t % kSS;
+          se[(L.base[l - 1] + bi) * kSS + o] = filled_diff<T>(fu, f1, fe, lc, L.sg, bi, lc.blocks[bi].x, o % kS, o / kS);
+        }
+      });
+      step([&] {
+        for (int t = tid; t < own(l) * 256; t += kCoarseThreads) {
+          const int q = L.base[l] + (t >> 8), dx = t & 15, dy = (t >> 4) & 15;
+          const int4 ch = child[q];
+          const int ir = dx & 1, iz = dy & 1;
+          const T *cb = tile_of(fe, ch.y) + 2 + 8 * (ch.z - 1) + (dx >> 1) + kS * (2 + 8 * (ch.w - 1) + (dy >> 1));
+          T v = dmul<T>(T(0.5), cb[0]);
+          v = dadd<T>(v, dmul<T>(T(0.25), cb[2 * ir - 1]));
+          v = dadd<T>(v, dmul<T>(T(0.25), cb[kS * (2 * iz - 1)]));
+          T *d = su + q * kSS + (2 + dx) + kS * (2 + dy);
+          v = dadd<T>(v, *d);
+          *d = v;
+        }
+        const int i = head[8 * (l - 1)] + tid, end = head[8 * (l - 1) + 4];
+        const int2 first = i < end ? ent[i] : int2();
+        __syncthreads();
+        push(i, end, first);
+        if ((L.refined >> l) & 1) d_fill_ghost<T>(fu, view(l), L.sg, 4, 0, 1);
+      });
+      gs(l, L.nup, true);
+    }
   }
   cluster_wait();
   if (L.inner) {  // the correction of level top, for the prolongation of the next
@@ -428,7 +432,8 @@ int srmg::ensure_coarse(srmg_ctx *ctx) {
   auto add = [&](int l, int src, int x, int y, int dst, int cell, int k1, int k2) {
     const int mask = (1 << kSlotBits) - 1;
     list[((size_t)(l - 1) * kCoarseCtas + (src >> kSlotBits)) * 4 + kKindAt[2 * (x & 1) + (y & 1)]].push_back(
-        make_int2(cell | (dst & mask) << 9 | (dst >> kSlotBits) << 15, (x + kS * y) | (src & mask) << 9 | k1 << 15 | k2 << 19));
+        make_int2(cell | (dst & mask) << 9 | (dst >> kSlotBits) << 15,
+                  (x + kS * y) | (src & mask) << 9 | k1 << 15 | k2 << 19));
   };
   for (int l = 1; l <= (int)H.size(); l++) {
     const Host &h = H[l - 1];
@@ -452,7 +457,8 @@ int srmg::ensure_coarse(srmg_ctx *ctx) {
     for (int k = 0; k < 4 * nb; k++) {
       const int me = pos[h.blk[k / 4].x], f = k % 4, type = h.face[k].x;
       if (type != FACE_NEIGHBOR && type != FACE_BOUNDARY) continue;
-      if (type == FACE_NEIGHBOR && (h.face[k].y < 0 || h.face[k].y >= ctx->max_blk || pos[h.face[k].y] < 0)) return SRMG_OK;
+      if (type == FACE_NEIGHBOR && (h.face[k].y < 0 || h.face[k].y >= ctx->max_blk || pos[h.face[k].y] < 0))
+        return SRMG_OK;
       for (int g = 0; g < kG; g++)
         for (int i = 0; i < kM; i++) {
           const int x = f == 0 ? g : f == 1 ? kG + kM + g : kG + i, y = f == 2 ? g : f == 3 ? kG + kM + g : kG + i;
@@ -572,7 +578,9 @@ int srmg::coarse_launch(srmg_ctx *ctx, CoarseCycle &A, bool four, int geom) {
   const CoarseKernel k = coarse_kernel(four, geom);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  CK(coarse_config(k, (int)smem_bytes(C.base[A.top + 1], C.base[A.top], A.inner, A.top, A.pbase[A.top + 1], four, geom), &cfg, attr));
+  const int64_t smem =
+      smem_bytes(C.base[A.top + 1], C.base[A.top], A.inner, A.top, A.pbase[A.top + 1], four, geom);
+  CK(coarse_config(k, (int)smem, &cfg, attr));
   cfg.stream = ctx->stream;
   CK(cudaLaunchKernelEx(&cfg, k, A));
   ctx->launches++;

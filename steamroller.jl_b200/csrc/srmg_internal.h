@@ -104,9 +104,10 @@ template <typename T> int L_interp_add(srmg_ctx *ctx, T *u, const T *u1, int l);
 template <typename T> int L_copy(srmg_ctx *ctx, T *dst, const T *src, int l);
 template <typename T> int L_diff(srmg_ctx *ctx, T *dst, const T *a1, const T *a2, int l);
 
+// One V-cycle; with `ran`, as many of `ncycles` as run in one launch, their number in *ran.
 template <typename T>
 int vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, double k2, int geom,
-               const Signs &sg, int lmax, int ndown, int ntop, int nup, double omega);
+               const Signs &sg, int lmax, int ndown, int ntop, int nup, double omega, int ncycles = 1, int *ran = nullptr);
 template <typename T>
 int leafnorm_dev(srmg_ctx *ctx, const T *u, const T *b, double s, int op, double k2, int geom,
                  int mode, int slot);

@@ -1073,7 +1073,7 @@ struct CoarseCycle {
   unsigned sw;                // the boundary table as bits
   int top, inner, known;      // inner: level top + 1 exists and has been restricted (residual in r);
                               // known: else, whether level top's ghosts are filled
-  int ndown, ntop, nup;
+  int ndown, ntop, nup, ncycles;
   // the tree's tables, set by coarse_launch
   const int4 *tab;
   int slots, levels, tabq, corners;
