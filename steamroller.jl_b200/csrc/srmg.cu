@@ -110,8 +110,9 @@ void srmg::free_tree(srmg_ctx *ctx) {
   ctx->coef4 = DevBuf{};
   ctx->push_lv.clear();
   ctx->push_state = 0;
-  if (ctx->coarse.tab.p) cudaFree(ctx->coarse.tab.p);
+  const DevBuf tab = ctx->coarse.tab;  // kept for the next tree
   ctx->coarse = CoarseTab{};
+  ctx->coarse.tab = tab;
 }
 
 extern "C" void srmg_destroy(srmg_ctx *ctx) {
@@ -119,6 +120,7 @@ extern "C" void srmg_destroy(srmg_ctx *ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   free_tree(ctx);
+  if (ctx->coarse.tab.p) cudaFree(ctx->coarse.tab.p);
   for (auto &b : ctx->f64) if (b.p) cudaFree(b.p);
   for (auto &b : ctx->f32) if (b.p) cudaFree(b.p);
   if (ctx->part.p) cudaFree(ctx->part.p);
@@ -575,6 +577,8 @@ int srmg::build_tree(srmg_ctx *ctx, int nlev, const int64_t *npairs, const srmg_
   ctx->nleaf = (int)leafblk.size();
   ctx->it_lrange_host = lrange;
   ctx->nitems = nitems;
+  for (int l = 0; l < nlev && l < kCoarseLevels && (int)hb[l].size() <= kCoarseCtas * kCoarsePer; l++)
+    ctx->coarse.tree.push_back({hb[l], hf[l], corners ? hcf[l] : std::vector<int4>(), hc[l]});
   ctx->l1_blocks = hb[0];
   ctx->l1_faces = hf[0];
   ctx->l2_blocks = nlev >= 2 ? hb[1] : std::vector<int4>();

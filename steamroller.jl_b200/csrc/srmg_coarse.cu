@@ -396,47 +396,42 @@ int srmg::ensure_coarse(srmg_ctx *ctx) {
   CK(cudaStreamIsCapturing(ctx->stream, &cap));
   if (cap != cudaStreamCaptureStatusNone) return SRMG_OK;
   CoarseTab &C = ctx->coarse;
+  if (ctx->has_corners && ctx->push_state == 0) return SRMG_OK;
   C.state = -1;
   if (ctx->has_corners && ctx->push_state != 1) return SRMG_OK;
-  struct Host { std::vector<int4> blk, face, corner, child; };
-  std::vector<Host> H;
+  const std::vector<CoarseTab::Level> &T = C.tree;
+  int levels = 0;
   std::vector<int> pos((size_t)ctx->max_blk, -1);
   int slots = 0;
-  auto fetch = [&](std::vector<int4> &v, const int4 *d, size_t n) {
-    v.resize(n);
-    return n == 0 || cudaMemcpy(v.data(), d, n * sizeof(int4), cudaMemcpyDeviceToHost) == cudaSuccess;
-  };
-  while ((int)H.size() < ctx->nlev && (int)H.size() < kCoarseLevels) {
-    const int l = (int)H.size() + 1;
+  for (int l = 1; l <= (int)T.size(); l++) {
     const DevLevel &L = ctx->lv[l - 1];
+    const CoarseTab::Level &h = T[l - 1];
     const int per = (L.nblk + kCoarseCtas - 1) / kCoarseCtas;
     if (L.nblk < 1 || per > kCoarsePer || slots + per > (1 << kSlotBits) || (l > 1 && L.nch != L.nblk)) break;
-    Host h;
-    if (!fetch(h.blk, L.blocks, L.nblk) || !fetch(h.face, L.faces, 4 * (size_t)L.nblk) ||
-        !fetch(h.corner, L.cfaces, L.cfaces ? 4 * (size_t)L.nblk : 0) || !fetch(h.child, L.child, l > 1 ? L.nch : 0))
-      return fail(ctx, SRMG_ERR_CUDA, "coarse levels: %s", cudaGetErrorString(cudaGetLastError()));
-    for (int bi = 0; bi < L.nblk; bi++) {
-      if (h.blk[bi].x < 0 || h.blk[bi].x >= ctx->max_blk) return SRMG_OK;
-      pos[h.blk[bi].x] = pos_of(bi / per, slots + bi % per);
-    }
+    for (int bi = 0; bi < L.nblk; bi++) pos[h.blk[bi].x] = pos_of(bi / per, slots + bi % per);
     C.nblk[l] = L.nblk;
     C.per[l] = per;
     C.base[l] = slots;
     slots += per;
     C.base[l + 1] = slots;
-    H.push_back(std::move(h));
+    levels = l;
   }
-  if (H.empty()) return SRMG_OK;
+  if (levels == 0) return SRMG_OK;
   // the pushes: of the star's faces by rule, of a BoxStencil tree from its push tables
-  std::vector<std::vector<int2>> list((size_t)H.size() * kCoarseCtas * 4);  // by level, CTA, kind
+  // Counted first, then placed: bin (level, CTA, kind).
+  const int mask = (1 << kSlotBits) - 1;
+  std::vector<int> bin((size_t)levels * kCoarseCtas * 4, 0);
+  struct Push { int bin; int2 word; };
+  std::vector<Push> list;
+  list.reserve((size_t)slots * kCoarseCtas * 144);
   auto add = [&](int l, int src, int x, int y, int dst, int cell, int k1, int k2) {
-    const int mask = (1 << kSlotBits) - 1;
-    list[((size_t)(l - 1) * kCoarseCtas + (src >> kSlotBits)) * 4 + kKindAt[2 * (x & 1) + (y & 1)]].push_back(
-        make_int2(cell | (dst & mask) << 9 | (dst >> kSlotBits) << 15,
-                  (x + kS * y) | (src & mask) << 9 | k1 << 15 | k2 << 19));
+    const int k = ((l - 1) * kCoarseCtas + (src >> kSlotBits)) * 4 + kKindAt[2 * (x & 1) + (y & 1)];
+    bin[k]++;
+    list.push_back({k, make_int2(cell | (dst & mask) << 9 | (dst >> kSlotBits) << 15,
+                                 (x + kS * y) | (src & mask) << 9 | k1 << 15 | k2 << 19)});
   };
-  for (int l = 1; l <= (int)H.size(); l++) {
-    const Host &h = H[l - 1];
+  for (int l = 1; l <= levels; l++) {
+    const CoarseTab::Level &h = T[l - 1];
     const int nb = ctx->lv[l - 1].nblk;
     if (ctx->has_corners) {
       const PushView &pv = ctx->push_lv[l - 1];
@@ -471,38 +466,41 @@ int srmg::ensure_coarse(srmg_ctx *ctx) {
     }
   }
   C.pbase[1] = 0;
-  for (int l = 1; l <= (int)H.size(); l++) {
-    size_t most = 0;
+  for (int l = 1; l <= levels; l++) {
+    int most = 0;
     for (int cta = 0; cta < kCoarseCtas; cta++) {
-      size_t n = 0;
-      for (int k = 0; k < 4; k++) n += list[((size_t)(l - 1) * kCoarseCtas + cta) * 4 + k].size();
-      most = std::max(most, n);
+      const int *n = &bin[((l - 1) * kCoarseCtas + cta) * 4];
+      most = std::max(most, n[0] + n[1] + n[2] + n[3]);
     }
-    C.pbase[l + 1] = C.pbase[l] + (int)((most + 1) / 2 * 2);
+    C.pbase[l + 1] = C.pbase[l] + (most + 1) / 2 * 2;
   }
-  C.levels = (int)H.size();
+  C.levels = levels;
   C.slots = slots;
   C.tabq = slots * kSlotQ + 2 * C.levels + C.pbase[C.levels + 1] / 2;
   std::vector<int4> img((size_t)kCoarseCtas * C.tabq, make_int4(0, 0, 0, 0));
+  std::vector<int2 *> fillp(bin.size());
   for (int l = 1; l <= C.levels; l++)
     for (int cta = 0; cta < kCoarseCtas; cta++) {
-      int4 *T = img.data() + (size_t)cta * C.tabq + slots * kSlotQ;
-      int *head = reinterpret_cast<int *>(T + 2 * (l - 1));
-      int2 *ent = reinterpret_cast<int2 *>(T + 2 * C.levels);
+      int4 *T4 = img.data() + (size_t)cta * C.tabq + slots * kSlotQ;
+      int *head = reinterpret_cast<int *>(T4 + 2 * (l - 1));
+      int2 *ent = reinterpret_cast<int2 *>(T4 + 2 * C.levels);
       int n = C.pbase[l];
       for (int k = 0; k < 4; k++) {
+        const int b = ((l - 1) * kCoarseCtas + cta) * 4 + k;
         head[k] = n;
-        for (const int2 &e : list[((size_t)(l - 1) * kCoarseCtas + cta) * 4 + k]) ent[n++] = e;
+        fillp[b] = ent + n;
+        n += bin[b];
       }
       head[4] = n;
     }
-  for (int l = 1; l <= (int)H.size(); l++) {
-    const Host &h = H[l - 1];
+  for (const Push &e : list) *fillp[e.bin]++ = e.word;
+  for (int l = 1; l <= levels; l++) {
+    const CoarseTab::Level &h = T[l - 1];
     for (size_t bi = 0; bi < h.blk.size(); bi++) {
       const int p = pos[h.blk[bi].x], s = p & ((1 << kSlotBits) - 1);
-      int4 *T = img.data() + (size_t)(p >> kSlotBits) * C.tabq;
-      int4 *blk = T + s, *child = T + slots + s, *face = T + 2 * slots + 4 * s, *corner = T + 6 * slots + 4 * s;
-      *blk = make_int4(p, h.blk[bi].y, h.blk[bi].z, 0);
+      int4 *T4 = img.data() + (size_t)(p >> kSlotBits) * C.tabq;
+      int4 *blk = T4 + s, *child = T4 + slots + s, *face = T4 + 2 * slots + 4 * s, *corner = T4 + 6 * slots + 4 * s;
+      *blk = make_int4(p, h.blk[bi].y, h.blk[bi].z, h.blk[bi].w);  // w: the quadrants with finer blocks
       *child = make_int4(h.blk[bi].x, 0, 0, 0);
       auto placed = [&](int4 f) {
         if (f.x == FACE_NEIGHBOR || f.x == FACE_REFBND) f.y = f.y >= 0 && f.y < ctx->max_blk ? pos[f.y] : -1;
@@ -516,34 +514,27 @@ int srmg::ensure_coarse(srmg_ctx *ctx) {
       }
     }
   }
-  // parents, and the quadrants of a block with finer blocks on them
-  for (int l = 2; l <= (int)H.size() + 1 && l <= ctx->nlev; l++) {
-    const bool in = l <= (int)H.size();
-    std::vector<int4> edges;
-    if (!in && !fetch(edges, ctx->lv[l - 1].child, ctx->lv[l - 1].nch))
-      return fail(ctx, SRMG_ERR_CUDA, "coarse levels: %s", cudaGetErrorString(cudaGetLastError()));
-    for (const int4 &e : in ? H[l - 1].child : edges) {
-      if (e.y < 0 || e.y >= ctx->max_blk || pos[e.y] < 0) return SRMG_OK;
-      const int pc = pos[e.y];
-      img[(size_t)(pc >> kSlotBits) * C.tabq + (pc & ((1 << kSlotBits) - 1))].w |= 1 << ((e.z - 1) + 2 * (e.w - 1));
-      if (!in) continue;
-      const int pf = pos[e.x];
-      if (pf < 0) return SRMG_OK;
-      int4 &c = img[(size_t)(pf >> kSlotBits) * C.tabq + slots + (pf & ((1 << kSlotBits) - 1))];
+  for (int l = 2; l <= levels; l++)  // parents
+    for (const int4 &e : T[l - 1].child) {
+      const int pc = pos[e.y], pf = pos[e.x];
+      if (pc < 0 || pf < 0) return SRMG_OK;
+      int4 &c = img[(size_t)(pf >> kSlotBits) * C.tabq + slots + (pf & mask)];
       c.y = pc, c.z = e.z, c.w = e.w;
     }
-  }
   // the GPU must have room for a cluster of this size
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[2];
-  const CoarseKernel k = coarse_kernel(ctx->has_corners, 1);
-  int clusters = 0;
-  const cudaError_t able = coarse_config(k, kCoarseSmem, &cfg, attr);
-  cfg.numAttrs = 1;
-  if (able != cudaSuccess || cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
-    (void)cudaGetLastError();
-    return SRMG_OK;
+  int &able = ctx->coarse_able[ctx->has_corners];
+  if (able == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    const CoarseKernel k = coarse_kernel(ctx->has_corners, 1);
+    int clusters = 0;
+    cudaError_t e = coarse_config(k, kCoarseSmem, &cfg, attr);
+    cfg.numAttrs = 1;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, k, &cfg);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    able = e == cudaSuccess && clusters >= 1 ? 1 : -1;
   }
+  if (able < 0) return SRMG_OK;
   RC(ensure(ctx, C.tab, img.size() * sizeof(int4)));
   CK(cudaMemcpy(C.tab.p, img.data(), img.size() * sizeof(int4), cudaMemcpyHostToDevice));
   C.state = 1;

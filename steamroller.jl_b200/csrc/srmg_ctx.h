@@ -54,6 +54,9 @@ struct DevBuf {
 // The coarse levels' tables for k_vcycle_coarse (srmg_coarse.cu): state 0 = not built for this
 // tree, 1 = built, -1 = not used on it.
 struct CoarseTab {
+  // what the tables are built from, kept from the upload: the levels from 1 up that may fit
+  struct Level { std::vector<int4> blk, face, corner, child; };
+  std::vector<Level> tree;
   int state = 0, levels = 0, slots = 0, tabq = 0, pbase[kCoarseLevels + 2] = {};
   int base[kCoarseLevels + 2] = {}, nblk[kCoarseLevels + 1] = {}, per[kCoarseLevels + 1] = {};
   DevBuf tab;
@@ -132,6 +135,7 @@ struct srmg_ctx {
   unsigned mref_levels = 0;                 // bit l: boundary corners of level l mirror refinement ghosts
   bool use_coarse = true;                   // coarse levels of an FP64 V-cycle in one cluster
   srmg::CoarseTab coarse;
+  int coarse_able[2] = {0, 0};              // whether the GPU has room for its cluster: 0 = not asked, 1, -1 (order 2, 4)
   srmg::DevBuf coef4;                       // order-4 coefficients per radial index (BoxStencil trees)
   bool trace_on = false;
   srmg::DevBuf trace;        // %globaltimer stamps after every engine phase (CTA 0)

@@ -87,7 +87,6 @@ struct EngArgs {
   int ndown, ntop, nup;
   int local_top;     // levels 1..local_top run inside CTA 0
   int top;           // the coarsest level a V-cycle visits: 1, or 2 (a lone item's direct solve there)
-  int leg;           // 0 = the whole V-cycle, 1 = the descent to level top only, 2 = the ascent from it only
   int smooth_level;  // > 0: run smooth_n GS iterations on this level only (gauss_seidel_iter!)
   int smooth_n;
   int nitems;
@@ -115,6 +114,7 @@ struct EngArgs {
   double *bpart_b;         // the same for b^2
   double *inorm;           // per item: {norm, |b|, initial norm, V-cycles run}
   double *out;             // out[0] V-cycles run by the launch
+  int leg;  // 0 = the whole V-cycle, 1 = the descent to level top only, 2 = the ascent from it only
 };
 
 __device__ __forceinline__ int item_of(int4 bk) { return bk.w >> 8; }
