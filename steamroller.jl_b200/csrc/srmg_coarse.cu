@@ -373,7 +373,8 @@ CoarseKernel coarse_kernel(bool four, int geom) {
 
 cudaError_t coarse_config(CoarseKernel k, int smem, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at) {
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // the same limit on every launch: another thread's may be about to need more
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoarseSmem);
   cfg->gridDim = dim3(kCoarseCtas);
   cfg->blockDim = dim3(kCoarseThreads);
   cfg->dynamicSmemBytes = smem;
