@@ -57,6 +57,15 @@ int srmg::ensure(srmg_ctx *ctx, DevBuf &b, size_t bytes) {
   return SRMG_OK;
 }
 
+// On the context's (non-blocking) stream and complete on return: a plain cudaMemcpy runs on the
+// legacy stream, which nothing orders with it, and may return before a pageable source has
+// arrived -- while kernels read their tables ahead of their wait for the previous kernel.
+int srmg::upload(srmg_ctx *ctx, void *dst, const void *src, size_t bytes) {
+  CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return SRMG_OK;
+}
+
 // ------------------------------------------------------------------ context
 
 extern "C" int srmg_create(srmg_ctx **out, int D, int M, int G, int device) {
@@ -536,9 +545,7 @@ int srmg::build_tree(srmg_ctx *ctx, int nlev, const int64_t *npairs, const srmg_
   void *d = nullptr;
   if (cudaMalloc(&d, off) != cudaSuccess) return fail(ctx, SRMG_ERR_NOMEM, "tree allocation of %zu bytes", off);
   ctx->d_tree = d;
-  // on the context's (non-blocking) stream, so that its later work is ordered after it
-  CK(cudaMemcpyAsync(d, host.data(), off, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  RC(upload(ctx, d, host.data(), off));
   char *base = (char *)d;
   ctx->nlev = nlev;
   ctx->lv.resize(nlev);
@@ -783,6 +790,7 @@ int srmg::ensure_gs_push(srmg_ctx *ctx, int op) {
     RC(ensure(ctx, ctx->coef4, (size_t)ctx->wtab_n * kCoef4 * sizeof(double)));
     k_coef4<<<(ctx->wtab_n + 127) / 128, 128, 0, ctx->stream>>>((double *)ctx->coef4.p, ctx->wtab_n);
     CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(ctx->stream));  // a table as the others: there whatever stream reads it next
   }
   const int64_t nf = ctx->max_blk * kSS;
   if (nf <= 0 || nf >= ((int64_t)1 << 31)) return SRMG_OK;
@@ -918,7 +926,7 @@ int srmg::ensure_gs_push(srmg_ctx *ctx, int op) {
     for (const Ent &e : ents[l - 1]) ent[fillp[e.key]++] = make_int2(e.dest, e.sg);
   }
   RC(ensure(ctx, ctx->push_tab, bytes));
-  CK(cudaMemcpy(ctx->push_tab.p, stage.data(), bytes, cudaMemcpyHostToDevice));
+  RC(upload(ctx, ctx->push_tab.p, stage.data(), bytes));
   ctx->push_lv.assign(ctx->nlev, PushView{nullptr, nullptr, nullptr});
   for (int l = 1; l <= ctx->nlev; l++) {
     const int nb = ctx->lv[l - 1].nblk;

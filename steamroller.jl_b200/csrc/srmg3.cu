@@ -923,7 +923,7 @@ int ensure_push3(srmg_ctx *ctx) {
     for (const Ent &e : ents[l - 1]) ent[fillp[e.key]++] = make_int2(e.dest, e.sg);
   }
   RC(ensure(ctx, ctx->push_tab, bytes));
-  CK(cudaMemcpy(ctx->push_tab.p, stage.data(), bytes, cudaMemcpyHostToDevice));
+  RC(upload(ctx, ctx->push_tab.p, stage.data(), bytes));
   ctx->push_lv.assign(ctx->nlev, PushView{nullptr, nullptr});
   char *base = static_cast<char *>(ctx->push_tab.p);
   for (int l = 1; l <= ctx->nlev; l++)
@@ -1319,8 +1319,7 @@ extern "C" int srmg_set_tree3(srmg_ctx *ctx, int nlev, const int64_t *npairs, co
   if (cudaMalloc(&d, host.size()) != cudaSuccess)
     return fail(ctx, SRMG_ERR_NOMEM, "tree allocation of %zu bytes", host.size());
   ctx->d_tree = d;
-  CK(cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  RC(upload(ctx, d, host.data(), host.size()));
   char *base = (char *)d;
   ctx->nlev = nlev;
   ctx->lv3.assign(nlev, Dev3Level{});

@@ -537,7 +537,7 @@ int srmg::ensure_coarse(srmg_ctx *ctx) {
   }
   if (able < 0) return SRMG_OK;
   RC(ensure(ctx, C.tab, img.size() * sizeof(int4)));
-  CK(cudaMemcpy(C.tab.p, img.data(), img.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  RC(upload(ctx, C.tab.p, img.data(), img.size() * sizeof(int4)));
   C.state = 1;
   return SRMG_OK;
 }

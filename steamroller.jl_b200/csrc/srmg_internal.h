@@ -33,6 +33,7 @@ void launch_pdl(void (*kernel)(KArgs...), int64_t grid, int threads, size_t smem
 }
 int cuda_check(srmg_ctx *c, cudaError_t e, const char *what);
 int ensure(srmg_ctx *ctx, DevBuf &b, size_t bytes);
+int upload(srmg_ctx *ctx, void *dst, const void *src, size_t bytes);
 int check_call(srmg_ctx *ctx, int64_t nblk_alloc, int op, int geom, const int8_t *bc);
 // check_call for the entry points that also run on three-dimensional trees (3^D-entry
 // boundary table, Cartesian geometry there); check_call refuses D = 3 contexts.
