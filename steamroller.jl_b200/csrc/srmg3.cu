@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "srmg3_sweep.h"
 #include "srmg_ctx.h"
 #include "srmg_engine.cuh"
 #include "srmg_internal.h"
@@ -422,9 +423,10 @@ template <int MODE>
 __global__ void __launch_bounds__(128, 1) k3_gs_push(double *u, const double *b, Level3View L, Op3 p, int P1, int P2,
                                                   PushView pv, unsigned long long sw, const __grid_constant__ Signs27 sg) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  constexpr int N = MODE == 2 ? 1024 : 2048;  // cells of a colour per block
-  constexpr int kAhead = 7;                   // a cell by a block's corner has that many pushes
-  const int total = L.nblk * N, stride = gridDim.x * blockDim.x;  // a field holds fewer than 2^31 values
+  using Index = typename Sweep3<MODE>::Index;
+  constexpr int N = Sweep3<MODE>::kCells;
+  constexpr int kAhead = 7;  // a cell by a block's corner has that many pushes
+  const Index total = Sweep3<MODE>::total(L.nblk), stride = (Index)gridDim.x * blockDim.x;
   struct Cell {
     int x, y, z;
     int64_t base;
@@ -433,9 +435,9 @@ __global__ void __launch_bounds__(128, 1) k3_gs_push(double *u, const double *b,
     int2 d[kAhead];
   };
   auto side = [](int q) { return q < kG + 2 ? -1 : q >= kG + kM - 2 ? 1 : 0; };
-  auto load = [&](int t) {
+  auto load = [&](Index t) {
     Cell q;
-    const int bi = t / N, c = t % N;
+    const int bi = (int)(t / N), c = (int)(t % N);
     if (MODE == 2) {
       q.z = kG + c / 64;
       q.x = kG + 2 * (c % 8) + ((P1 + q.z + 1) & 1);
@@ -462,7 +464,7 @@ __global__ void __launch_bounds__(128, 1) k3_gs_push(double *u, const double *b,
     }
     return q;
   };
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  Index t = blockIdx.x * (Index)blockDim.x + threadIdx.x;
   Cell q;
   if (t < total) q = load(t);
   asm volatile("griddepcontrol.wait;" ::: "memory");
