@@ -233,11 +233,15 @@ extern "C" int srmg_get_trace(srmg_ctx *ctx, int64_t *out, int max_entries) {
   return k;
 }
 
-// Reads the engine's error word (after the stream has been synchronised by the caller).
+// Reads the engine's error word (after the stream has been synchronised by the caller).  A word
+// that has been reported is cleared: the next call need not launch a persistent kernel, which
+// would zero it, and its own work has not failed.
 int srmg::engine_check(srmg_ctx *ctx) {
   if (!ctx->sync.p) return SRMG_OK;
   int err = 0;
   CK(cudaMemcpy(&err, (char *)ctx->sync.p + 128, sizeof(int), cudaMemcpyDeviceToHost));
-  if (err) return fail(ctx, SRMG_ERR_TIMEOUT, "engine barrier timed out (error word %d)", err);
-  return SRMG_OK;
+  if (!err) return SRMG_OK;
+  CK(cudaMemsetAsync((char *)ctx->sync.p + 128, 0, sizeof(int), ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return fail(ctx, SRMG_ERR_TIMEOUT, "engine barrier timed out (error word %d)", err);
 }
