@@ -536,7 +536,10 @@ int srmg::ensure_coarse(srmg_ctx *ctx) {
     able = e == cudaSuccess && clusters >= 1 ? 1 : -1;
   }
   if (able < 0) return SRMG_OK;
-  RC(ensure(ctx, C.tab, img.size() * sizeof(int4)));
+  if (ensure(ctx, C.tab, img.size() * sizeof(int4))) {  // no memory for them: cycles run as without
+    (void)cudaGetLastError();
+    return SRMG_OK;
+  }
   RC(upload(ctx, C.tab.p, img.data(), img.size() * sizeof(int4)));
   C.state = 1;
   return SRMG_OK;
