@@ -71,9 +71,10 @@ __host__ __device__ inline double recip_of(double d) {
 // second gives the correctly rounded quotient, as long as nothing leaves the normal range;
 // there, and for infinities and NaN, the division itself is called.
 __device__ __forceinline__ double div_by(double a, double d, double rd) {
-  // the exponent field: 2^-700 <= |a| < 2^700 (an integer test; the fp64 pipe is the bound),
-  // and a reciprocal from recip_of
-  if ((unsigned)((__double2hiint(a) & 0x7ff00000) - (323 << 20)) >= (1400u << 20) || __double2hiint(rd) == 0)
+  // the exponent field: 2^-700 <= |a| < 2^670 (an integer test; the fp64 pipe is the bound),
+  // and a reciprocal from recip_of.  A cell size passes recip_of on level 1 and is below 1e-90
+  // by up to 2^-29 on the finest level: |a / d| < 2^(670 + 299 + 29) stays normal.
+  if ((unsigned)((__double2hiint(a) & 0x7ff00000) - (323 << 20)) >= (1370u << 20) || __double2hiint(rd) == 0)
     return a == 0.0 && rd != 0.0 ? __dmul_rn(a, rd) : __ddiv_rn(a, d);
   double q = __dmul_rn(a, rd);
   q = fma(fma(-q, d, a), rd, q);
