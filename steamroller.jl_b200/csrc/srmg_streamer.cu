@@ -74,7 +74,8 @@ __device__ __forceinline__ double min_quotient(double md, double a, double b) {
 
 // Cell sizes of a level: h = h1 / 2^(l-1), its reciprocal and (h h / D) / 4.  Scaling by powers
 // of two is exact, so the host forms the level-1 quotients once and the kernels need no
-// division for them.
+// division for them (dt1 < 0: some level's square or quotient could leave the normal range, and
+// the limit is formed per block).
 struct CellSize {
   double h1, rh1, dt1;
 };
@@ -171,7 +172,7 @@ k_streamer_flux(double *__restrict__ flux, double *__restrict__ maxdt_blk, doubl
     const double *n = sm + (j % kRing) * kTileSet, *ea = n + kSS, *eb = n + 2 * kSS;
     double *fb = flux + (int64_t)X * 2 * kSSV;
     const double h = mul(cs.h1, pow2(1 - lb.y)), rh = mul(cs.rh1, pow2(lb.y - 1));  // h /= 1 << (level - 1)
-    const double dt = mul(cs.dt1, pow2(2 - 2 * lb.y));
+    const double dt = cs.dt1 >= 0.0 ? mul(cs.dt1, pow2(2 - 2 * lb.y)) : dvd(dvd(mul(h, h), tr.D), 4.0);
     md = BLK ? fmin(INFINITY, dt) : fmin(md, dt);
     if (act) {
       fb[rx + kSV * ry] = face_flux(load_face(eb, ea, n, 0, rx, ry), tr, h, rh, r3, r6, md);
@@ -312,7 +313,8 @@ bool aligned16(std::initializer_list<const void *> ps) {
 CellSize cell_size(double h, const srmg_transport &tr) {
   volatile double hh = h * h;
   volatile double q = hh / tr.D;
-  return CellSize{h, recip_of(h), q / 4.0};
+  auto safe = [](double v) { return v > 1e-200 && v < 1e200; };  // levels scale by 2^-58 at most
+  return CellSize{h, recip_of(h), safe(hh) && safe(q) ? q / 4.0 : -1.0};
 }
 
 int check_transport(srmg_ctx *ctx, const srmg_transport *tr, const char *who) {
