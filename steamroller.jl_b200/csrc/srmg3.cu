@@ -353,38 +353,38 @@ __device__ __forceinline__ void d3_copy(double *__restrict__ dst, const double *
 
 // The per-operation kernels: each one body, launched alone or run by the sequencer.
 __global__ void k3_fill(double *__restrict__ u, Level3View L, Signs27 sg, int phase) {
-  pdl_enter();
+  pdl_enter(u);
   d3_fill(u, L, sg, phase);
 }
 __global__ void k3_gs_rb(double *__restrict__ u, const double *__restrict__ b, Level3View L, Op3 p, int parity) {
-  pdl_enter();
+  pdl_enter(u, b);
   d3_gs_rb(u, b, L, p, parity);
 }
 __global__ void k3_gs4(double *__restrict__ u, const double *__restrict__ b, Level3View L, Op3 p, int P1, int P2) {
-  pdl_enter();
+  pdl_enter(u, b);
   d3_gs4(u, b, L, p, P1, P2);
 }
 __global__ void k3_residual(double *__restrict__ r, const double *__restrict__ u, const double *__restrict__ b,
                             Level3View L, Op3 p) {
-  pdl_enter();
+  pdl_enter(r, u, b);
   d3_residual(r, u, b, L, p);
 }
 __global__ void k3_postrestrict(double *__restrict__ bf, const double *__restrict__ u, const double *__restrict__ r,
                                 Level3View L, Op3 pc) {
-  pdl_enter();
+  pdl_enter(bf, u, r);
   d3_postrestrict(bf, u, r, L, pc);
 }
 __global__ void k3_restrict(double *__restrict__ u, Level3View L) {
-  pdl_enter();
+  pdl_enter(u);
   d3_restrict(u, L);
 }
 __global__ void k3_interp_add(double *__restrict__ u, const double *__restrict__ u1, Level3View L) {
-  pdl_enter();
+  pdl_enter(u, u1);
   d3_interp_add(u, u1, L);
 }
 __global__ void k3_copy(double *__restrict__ dst, const double *__restrict__ a1, const double *__restrict__ a2,
                         Level3View L) {
-  pdl_enter();
+  pdl_enter(dst, a1, a2);
   d3_copy(dst, a1, a2, L);
 }
 
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(128, 1) k3_gs_push(double *u, const double *b,
 // one pass, eight lanes a coarse cell (the order-4 residual is a chain of 19 additions, and a
 // level of 8 blocks has 4096 coarse cells: one thread a cell left most of the chip idle).
 __global__ void __launch_bounds__(128) k3_down(double *u, double *r, const double *b, Level3View L, Op3 p) {
-  pdl_enter();
+  pdl_enter(u, r, b);
   const int64_t total = (int64_t)L.nch * 4096;  // a multiple of the warp
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int e = (int)(t / 4096), c = (int)(t % 4096) / 8, i = (int)(t % 8);
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(128) k3_down(double *u, double *r, const doubl
 // The saved copy of the coarse level lc and its FAS right-hand side under the children of lf.
 __global__ void __launch_bounds__(128) k3_save_rhs(double *u1, double *b, const double *u, const double *r,
                                                    Level3View lc, Level3View lf, Op3 pc) {
-  pdl_enter();
+  pdl_enter(u1, b, u, r);
   d3_postrestrict(b, u, r, lf, pc);
   d3_copy(u1, u, nullptr, lc);
 }
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(128) k3_save_rhs(double *u1, double *b, const 
 // that d3_fill would copy, mirror or interpolate it from.
 __global__ void __launch_bounds__(128) k3_correction(double *e, const double *u, const double *u1, Level3View L,
                                                      const __grid_constant__ Signs27 sg) {
-  pdl_enter();
+  pdl_enter(e, u, u1);
   const int64_t total = (int64_t)L.nblk * S3;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int bi = (int)(t / S3), c = (int)(t % S3), x = c % S, y = (c / S) % S, z = c / S2;
@@ -576,7 +576,7 @@ template <bool RULE>
 __global__ void __launch_bounds__(128) k3_interp_push(double *u, const double *e, Level3View L, PushView pv,
                                                       unsigned long long sw, const __grid_constant__ Signs27 sg,
                                                       bool refined) {
-  pdl_enter();
+  pdl_enter(u, e);
   const int64_t total = (int64_t)L.nch * 4096;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int k = (int)(t / 4096), c = (int)(t % 4096);
@@ -685,7 +685,7 @@ bool seq3_push(srmg_ctx *ctx, int kind, int i0, int i1, double *a, const double 
 // rhs! (src/multigrid.jl:363-388): identity at order 2, the 7-point right-hand side
 // (centre 6) / 12 at order 4 (src/laplacian.jl:322-337)
 __global__ void k3_rhs(double *__restrict__ q1, const double *__restrict__ q, Level3View L, int op) {
-  pdl_enter();
+  pdl_enter(q1, q);
   const int64_t total = (int64_t)L.nblk * 4096;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int bi = (int)(t / 4096), c = (int)(t % 4096);
@@ -715,7 +715,7 @@ template <int NT>
 __global__ void __launch_bounds__(NT) k3_leafsq(double *__restrict__ part, const double *__restrict__ u,
                                                 const double *__restrict__ b, Level3View L, Op3 p, double wl,
                                                 int mode) {
-  pdl_enter();
+  pdl_enter(part, u, b);
   double acc = 0.0;
   const int64_t total = (int64_t)L.nblk * 4096;
   for (int64_t t = blockIdx.x * (int64_t)NT + threadIdx.x; t < total; t += (int64_t)gridDim.x * NT) {

@@ -14,6 +14,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <initializer_list>
 
 namespace srmg {
 
@@ -32,12 +33,15 @@ constexpr int kNormChunk = 4;
 constexpr int kItemRec = 5;
 
 // Top of a kernel launched by launch_pdl: lets the next kernel's blocks be scheduled, then
-// waits for the previous kernel on the stream to complete.  (A load through a const
-// __restrict__ pointer may be moved above the wait unless its address comes from a load that
-// cannot; in these kernels it comes from the tree's tables.)
-__device__ __forceinline__ void pdl_enter() {
+// waits for the previous kernel on the stream to complete.  fields: the kernel's pointers to
+// memory that other kernels write.  The compiler may move an access through a __restrict__
+// parameter above the wait (nothing else in the kernel, the wait included, can touch what it
+// points to), so the pointers pass through an empty asm after it: what follows depends on that.
+template <typename... P>
+__device__ __forceinline__ void pdl_enter(P &...fields) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  (void)std::initializer_list<int>{([](auto &p) { asm volatile("" : "+l"(p)::"memory"); }(fields), 0)...};
 }
 
 // Face numbering (the four StarStencil directions): 0 = -r, 1 = +r, 2 = -z, 3 = +z.
@@ -543,7 +547,7 @@ template <typename T, int NT>
 __global__ void __launch_bounds__(NT) k_leafsq(double *__restrict__ part, const T *__restrict__ u,
                                                const T *__restrict__ b, LevelView lv,
                                                OpParams<T> p, WTab<T> wt, double wl, int mode) {
-  pdl_enter();
+  pdl_enter(part, u, b);
   double acc = 0.0;
   const int64_t total = (int64_t)lv.nblk * 256;
   for (int64_t t = blockIdx.x * (int64_t)NT + threadIdx.x; t < total; t += (int64_t)gridDim.x * NT) {
@@ -574,12 +578,11 @@ __global__ void __launch_bounds__(NT) k_leafsq(double *__restrict__ part, const 
   }
 }
 
-// Final fixed-order reduction of n partials into out[0] (sqrt applied).  part is not
-// __restrict__: its loads must stay below pdl_enter().
+// Final fixed-order reduction of n partials into out[0] (sqrt applied).
 template <int NT>
 __global__ void __launch_bounds__(NT) k_reduce_sqrt(double *out,
                                                     const double *part, int n) {
-  pdl_enter();
+  pdl_enter(out, part);
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += NT) acc += part[i];
   __shared__ double sh[NT / 32];
@@ -656,7 +659,7 @@ __device__ __forceinline__ void d_gs4(T *__restrict__ u, const T *__restrict__ b
 // (0,-1), (-1,0), (0,0), (1,0), (0,1), then divided by 12.
 template <typename T>
 __global__ void k_rhs(T *__restrict__ q1, const T *__restrict__ q, LevelView lv, int op, int geom) {
-  pdl_enter();
+  pdl_enter(q1, q);
   const int64_t total = (int64_t)lv.nblk * 256;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -903,21 +906,21 @@ __device__ __forceinline__ void d_save_rhs(T *__restrict__ u1, T *__restrict__ b
 // same bodies also run as the operations of one cooperative launch (srmg_seq.cu).
 template <typename T>
 __global__ void __launch_bounds__(256, 6) k_fill_ghost(T *__restrict__ u, LevelView lv, Signs sg, int mask) {
-  pdl_enter();
+  pdl_enter(u);
   d_fill_ghost<T>(u, lv, sg, mask);
 }
 
 template <typename T>
 __global__ void k_gs_colour(T *__restrict__ u, const T *__restrict__ b, LevelView lv,
                             OpParams<T> p, WTab<T> wt, int parity) {
-  pdl_enter();
+  pdl_enter(u, b);
   d_gs_colour<T>(u, b, lv, p, wt, parity);
 }
 
 template <typename T>
 __global__ void k_residual(T *__restrict__ r, const T *__restrict__ u, const T *__restrict__ b,
                            LevelView lv, OpParams<T> p, WTab<T> wt) {
-  pdl_enter();
+  pdl_enter(r, u, b);
   d_residual<T>(r, u, b, lv, p, wt);
 }
 
@@ -925,66 +928,66 @@ template <typename T>
 __global__ void k_postrestrict(T *__restrict__ bf, const T *__restrict__ u, const T *__restrict__ r,
                                LevelView lv, const int2 *__restrict__ coord_of, OpParams<T> p,
                                WTab<T> wt) {
-  pdl_enter();
+  pdl_enter(bf, u, r);
   d_postrestrict<T>(bf, u, r, lv, coord_of, p, wt);
 }
 
 template <typename T>
 __global__ void k_restrict(T *__restrict__ u, LevelView lv) {
-  pdl_enter();
+  pdl_enter(u);
   d_restrict<T>(u, lv);
 }
 
 template <typename T>
 __global__ void k_interp_add(T *__restrict__ u, const T *__restrict__ u1, LevelView lv) {
-  pdl_enter();
+  pdl_enter(u, u1);
   d_interp_add<T>(u, u1, lv);
 }
 
 template <typename T>
 __global__ void k_copy_level(T *__restrict__ dst, const T *__restrict__ src, LevelView lv) {
-  pdl_enter();
+  pdl_enter(dst, src);
   d_copy_level<T>(dst, src, lv);
 }
 
 template <typename T>
 __global__ void k_diff_level(T *__restrict__ dst, const T *__restrict__ a1, const T *a2,
                              LevelView lv) {
-  pdl_enter();
+  pdl_enter(dst, a1, a2);
   d_diff_level<T>(dst, a1, a2, lv);
 }
 
 template <typename T>
 __global__ void k_gs4(T *__restrict__ u, const T *__restrict__ b, LevelView lv, OpParams<T> p, int p1, int p2) {
-  pdl_enter();
+  pdl_enter(u, b);
   d_gs4<T>(u, b, lv, p, p1, p2);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256, 1) k_down(T *__restrict__ u, T *__restrict__ r, const T *__restrict__ b, LevelView lv,
                        const int2 *__restrict__ coord_of, OpParams<T> p, WTab<T> wt) {
-  pdl_enter();
+  pdl_enter(u, r, b);
   d_down<T>(u, r, b, lv, coord_of, p, wt);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256, 1) k_save_rhs(T *__restrict__ u1, T *__restrict__ b, const T *__restrict__ u, const T *__restrict__ r,
                            LevelView lc, LevelView lf, const int2 *__restrict__ coord_of, OpParams<T> pc, WTab<T> wt) {
-  pdl_enter();
+  pdl_enter(u1, b, u, r);
   d_save_rhs<T>(u1, b, u, r, lc, lf, coord_of, pc, wt);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256, 1) k_correction(T *__restrict__ e, const T *__restrict__ u, const T *__restrict__ u1, LevelView lv,
                              Signs sg) {
-  pdl_enter();
+  pdl_enter(e, u, u1);
   d_correction<T>(e, u, u1, lv, sg);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256, 1) k_interp_push(T *__restrict__ u, const T *__restrict__ e, LevelView lv, PushView pv, unsigned sw,
                               Signs sg, bool refined) {
-  pdl_enter();
+  pdl_enter(u, e);
   d_interp_push<T>(u, e, lv, pv, sw, sg, refined);
 }
 
@@ -1087,7 +1090,7 @@ struct CoarseCycle {
 template <typename T>
 __global__ void k_fmg_step(T *__restrict__ e, T *__restrict__ u1, const T *__restrict__ u, LevelView lf, LevelView lc,
                            Signs sg) {
-  pdl_enter();
+  pdl_enter(e, u1, u);
   d_correction<T>(e, u, u1, lc, sg);
   d_copy_level<T>(u1, u, lf);
 }
