@@ -451,6 +451,12 @@ int srmg::build_tree(srmg_ctx *ctx, int nlev, const int64_t *npairs, const srmg_
           return fail(ctx, SRMG_ERR_BADTREE, "neighbour edge between two items");
       }
     }
+  // the ids in use, ascending, where some below the largest are not
+  std::vector<int> used;
+  for (int64_t b = 0; b < max_blk; b++)
+    if (binfo[b].w) used.push_back((int)b);
+  const int nused = (int)used.size();
+  if (nused == max_blk) used.clear();
   std::vector<std::vector<int4>> hr(nlev);
   for (int l = 0; l < nlev; l++) {
     hr[l].resize(5 * hb[l].size());
@@ -514,6 +520,7 @@ int srmg::build_tree(srmg_ctx *ctx, int nlev, const int64_t *npairs, const srmg_
   const size_t ochunk = take(std::max<size_t>(chunks.size(), 1) * sizeof(int4));
   const size_t oitch = take(itch.size() * sizeof(int2));
   const size_t oleaf = take(std::max<size_t>(leafblk.size(), 1) * sizeof(int2));
+  const size_t oused = take(used.size() * sizeof(int));
   std::vector<char> host(off, 0);
   for (int l = 0; l < nlev; l++) {
     memcpy(host.data() + orr[l], hr[l].data(), hr[l].size() * sizeof(int4));
@@ -539,6 +546,7 @@ int srmg::build_tree(srmg_ctx *ctx, int nlev, const int64_t *npairs, const srmg_
   memcpy(host.data() + ochunk, chunks.data(), chunks.size() * sizeof(int4));
   memcpy(host.data() + oitch, itch.data(), itch.size() * sizeof(int2));
   memcpy(host.data() + oleaf, leafblk.data(), leafblk.size() * sizeof(int2));
+  memcpy(host.data() + oused, used.data(), used.size() * sizeof(int));
 
   CK(cudaStreamSynchronize(ctx->stream));
   free_tree(ctx);
@@ -582,6 +590,8 @@ int srmg::build_tree(srmg_ctx *ctx, int nlev, const int64_t *npairs, const srmg_
   ctx->nchunk = (int)chunks.size();
   ctx->d_leaf = (int2 *)(base + oleaf);
   ctx->nleaf = (int)leafblk.size();
+  ctx->d_used = used.empty() ? nullptr : (int *)(base + oused);
+  ctx->nused = nused;
   ctx->it_lrange_host = lrange;
   ctx->nitems = nitems;
   for (int l = 0; l < nlev && l < kCoarseLevels && (int)hb[l].size() <= kCoarseCtas * kCoarsePer; l++)

@@ -161,6 +161,8 @@ struct srmg_ctx {
   int nchunk = 0;
   int2 *d_leaf = nullptr;               // blocks with a leaf cell: {0-based id, level}
   int nleaf = 0;
+  int *d_used = nullptr;                // the 0-based ids that blocks have, ascending; null: 0..nused-1
+  int nused = 0;
   srmg::DevBuf cnn_work[3];             // learned warm start: db, candidate guess, samples
   int cnn_active_ppm = 0;               // > 0: network only on blocks with g energy >= ppm 1e-6 x max
   int cnn_last_active = 0;              // active blocks of the last prediction (when read back)

@@ -33,19 +33,20 @@ constexpr int kSV = kS + 1;
 constexpr int kSSV = kSV * kSV;
 
 // q = dot(n, (-1, +1)) = (-1 n_e) + (1 n_ion) on the valid cells of every block of the tree
-// (info[X].w, the level, is 0 for an id that no block has): the products by +-1 are
+// (used: the blocks' ids, null where they are 0..nblk-1): the products by +-1 are
 // exact, so q is n_ion - n_e rounded once, as the reference computes it.  One launch for all
 // levels, a thread per cell (V = double) or cell pair (V = double2, 16-byte aligned fields): a
 // pure stream of 24 bytes a cell.  A launch per level with 8-byte accesses took 129 us
 // on 51877 blocks (49 us of bytes).
 template <typename V>
 __global__ void __launch_bounds__(256) k_netcharge(double *__restrict__ q, const double *__restrict__ ne,
-                                                   const double *__restrict__ nion, const int4 *__restrict__ info,
-                                                   int64_t nblk) {
+                                                   const double *__restrict__ nion, const int *__restrict__ used,
+                                                   int nblk) {
   constexpr int W = sizeof(V) / sizeof(double), NR = kM / W;  // cells a thread, threads a row
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t X = t / (kM * NR);
-  if (X >= nblk || info[X].w == 0) return;
+  const int64_t k0 = t / (kM * NR);
+  if (k0 >= nblk) return;
+  const int64_t X = used ? used[k0] : k0;
   const int c = (int)(t % (kM * NR));
   const int64_t o = X * kSS + kS * (2 + c / NR) + 2 + W * (c % NR);
   V a = *reinterpret_cast<const V *>(ne + o), b = *reinterpret_cast<const V *>(nion + o);
@@ -63,14 +64,15 @@ __global__ void __launch_bounds__(256) k_netcharge(double *__restrict__ q, const
 // upper faces too), and no warp waits for another.  |E| at the cell: sqrt((0 + s_1 s_1 / 4)
 // + s_2 s_2 / 4), s_d = f[I, d] + f[I + e_d, d], every operation rounded on its own (no fused
 // multiply-add; the quarter is exact either way), as in the reference.  One launch for
-// all levels (info: block coordinates, child mask, level, 0 for no block): a launch per
+// all levels (info: block coordinates, child mask, level; used as in k_netcharge): a launch per
 // level was 287 us on 51877 blocks, 650 MB of traffic (99 us).
 // CTAs stream blocks through a ring of u tiles (cp.async, three blocks ahead).
 constexpr int kEfRing = 4;
 template <int CH>
 __global__ void __launch_bounds__(256, 5) k_efield(double *__restrict__ e, double *__restrict__ eabs,
                                                    const double *__restrict__ u, const int4 *__restrict__ info,
-                                                   int nblk, double h1, double rh1, double e0r, double e0z) {
+                                                   const int *__restrict__ used, int nblk, double h1,
+                                                   double rh1, double e0r, double e0z) {
   __shared__ __align__(16) double tile[kEfRing][kSS];
   const int lane = threadIdx.x & 31, cx = lane & 15, p = threadIdx.x >> 5;
   const int x = 2 + cx, y0 = 2 + 2 * p, y = y0 + (lane >> 4);
@@ -78,19 +80,19 @@ __global__ void __launch_bounds__(256, 5) k_efield(double *__restrict__ e, doubl
   // the lane's extra face (any face of the tile where it has none)
   const int eo = ez ? x + kS * (y0 + 2) : 18 + kS * (y0 + (lane & 1)), el = eo - (ez ? kS : 1);
   auto fetch = [&](int j) {
-    const int64_t X = blockIdx.x + (int64_t)j * gridDim.x;
-    if (X < nblk) cp_tile<CH>(tile[j % kEfRing], u + X * kSS, kSS);
+    const int64_t k = blockIdx.x + (int64_t)j * gridDim.x;
+    if (k < nblk) cp_tile<CH>(tile[j % kEfRing], u + (used ? used[k] : k) * kSS, kSS);
     cp_async_commit();
   };
   for (int j = 0; j < kEfRing - 1; ++j) fetch(j);
   for (int j = 0;; ++j) {
-    const int64_t X = blockIdx.x + (int64_t)j * gridDim.x;
-    if (X >= nblk) break;
+    const int64_t k = blockIdx.x + (int64_t)j * gridDim.x;
+    if (k >= nblk) break;
+    const int64_t X = used ? used[k] : k;
     const int level = info[X].w;
     cp_async_wait<kEfRing - 2>();
     __syncthreads();  // the tile is here, and no thread reads the last one's any more
     fetch(j + kEfRing - 1);
-    if (level == 0) continue;  // no such block
     const double *ub = tile[j % kEfRing];
     double *eb = e + X * (2 * kSSV);
     const double hl = __dmul_rn(h1, __hiloint2double((1024 - level) << 20, 0));   // h / 2^(level - 1)
@@ -121,12 +123,12 @@ extern "C" int srmg_netcharge_dev(srmg_ctx *ctx, double *q, const double *ne, co
                                   int64_t nblk_alloc) {
   RC(check_call(ctx, nblk_alloc, 0, 0, nullptr));
   if (!q || !ne || !nion) return fail(ctx, SRMG_ERR_BADARG, "srmg_netcharge: null field");
-  const int64_t n = ctx->max_blk;
+  const int64_t n = ctx->nused;
   if (n > 0) {
     const bool pairs = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(ne) |
                          reinterpret_cast<uintptr_t>(nion)) & 15) == 0;
-    if (pairs) k_netcharge<double2><<<(unsigned)((n + 1) / 2), 256, 0, ctx->stream>>>(q, ne, nion, ctx->d_info, n);
-    else k_netcharge<double><<<(unsigned)n, 256, 0, ctx->stream>>>(q, ne, nion, ctx->d_info, n);
+    if (pairs) k_netcharge<double2><<<(unsigned)((n + 1) / 2), 256, 0, ctx->stream>>>(q, ne, nion, ctx->d_used, n);
+    else k_netcharge<double><<<(unsigned)n, 256, 0, ctx->stream>>>(q, ne, nion, ctx->d_used, n);
     ctx->launches++;
   }
   CK(cudaGetLastError());
@@ -145,10 +147,11 @@ extern "C" int srmg_electric_field_dev(srmg_ctx *ctx, double *e, double *eabs, c
   RC(check_call(ctx, nblk_alloc, 0, 0, nullptr));
   if (!e || !eabs || !u || !e0) return fail(ctx, SRMG_ERR_BADARG, "srmg_electric_field: null argument");
   if (!(h > 0.0) || !std::isfinite(h)) return fail(ctx, SRMG_ERR_BADARG, "srmg_electric_field: h must be > 0");
-  if (ctx->max_blk > 0) {
-    const int grid = (int)std::min<int64_t>(ctx->max_blk, 148 * 5);
+  if (ctx->nused > 0) {
+    const int grid = std::min(ctx->nused, 148 * 5);
     const auto kern = (reinterpret_cast<uintptr_t>(u) & 15) == 0 ? k_efield<16> : k_efield<8>;
-    kern<<<grid, 256, 0, ctx->stream>>>(e, eabs, u, ctx->d_info, (int)ctx->max_blk, h, recip_of(h), e0[0], e0[1]);
+    kern<<<grid, 256, 0, ctx->stream>>>(e, eabs, u, ctx->d_info, ctx->d_used, ctx->nused, h, recip_of(h), e0[0],
+                                        e0[1]);
     ctx->launches++;
   }
   CK(cudaGetLastError());

@@ -203,13 +203,13 @@ k_streamer_flux(double *__restrict__ flux, double *__restrict__ maxdt_blk, doubl
 // (block, face, k) sets the coarse block's face k (0..7) of the half `subblock` covers to the
 // mean of the two fine faces 2k, 2k + 1: f = ((0 + f_2k) + f_2k+1) / 2.
 __global__ void k_restrict_flux(double *__restrict__ flux, const int4 *__restrict__ faceb,
-                                const int4 *__restrict__ info, int64_t nblk) {
+                                const int *__restrict__ used, int nblk) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t X = t >> 5;
-  if (X >= nblk) return;
+  if ((t >> 5) >= nblk) return;
+  const int64_t X = used ? used[t >> 5] : t >> 5;
   const int f = (int)(t >> 3) & 3, k = (int)(t & 7);
   const int4 fi = faceb[4 * X + f];
-  if (fi.x != FACE_REFBND || info[X].w == 0) return;
+  if (fi.x != FACE_REFBND) return;
   const int d = f >> 1;  // the face's dimension: 0 for -r/+r, 1 for -z/+z
   const int fine_n = (f & 1) ? 2 + kM : 2, coarse_n = (f & 1) ? 2 : 2 + kM;  // normal face index
   const int sb = d == 0 ? fi.z >> 8 : fi.z & 255;  // the tangential half
@@ -349,8 +349,8 @@ extern "C" int srmg_streamer_flux_dev(srmg_ctx *ctx, double *flux, double *maxdt
     ctx->launches++;
   }
   if (ctx->refbnd_levels) {
-    k_restrict_flux<<<(unsigned)((ctx->max_blk * 32 + 255) / 256), 256, 0, ctx->stream>>>(flux, ctx->d_faceb,
-                                                                                          ctx->d_info, ctx->max_blk);
+    k_restrict_flux<<<(unsigned)(((int64_t)ctx->nused * 32 + 255) / 256), 256, 0, ctx->stream>>>(
+        flux, ctx->d_faceb, ctx->d_used, ctx->nused);
     ctx->launches++;
   }
   CK(cudaGetLastError());
