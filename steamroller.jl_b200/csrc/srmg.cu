@@ -1126,6 +1126,22 @@ static int coarse_levels(srmg_ctx *ctx, int top, double *u, double *b, double *r
   return coarse_launch(ctx, A, op == SRMG_OP_LAPLACIAN4, geom);
 }
 
+// Which levels go to the cluster, from timing every cut of trees of 1 to 1024 blocks a level at
+// (1, 1, 1) to (3, 5, 3) sweeps.  A level costs the cluster, which has 16 SMs for it, 10 us for
+// up to 16 blocks, 17 for 64 and 30 for 256 (order 2, two sweeps down and two up).
+// Against launches, 22 to 24 us a level of any of these sizes: up to kCoarseSmall blocks (5 a
+// CTA; levels of 1..64, 256: 77 us with the first four in it, 84 with all, 116 with none;
+// 8, 32, 128, 512: 82, 84 with the 128 too), but level 1 alone has to have sweeps enough to pay
+// for the way there and back, unless it is small (64 blocks, one sweep: 21 us, 18 launched).
+// Against the persistent kernel, 20 to 32 us a level: all of a tree that fits, the way out costing
+// nothing there -- but for a single sweep on levels so large that the phases win (64 and 256
+// blocks, (1, 1, 1): 48.4 us, 46.4 as phases).  A cycle split around the cluster has two more
+// launches, 25 us: worth it from kCoarseSweeps sweeps on small levels (3, 12, 48, then 192 and
+// 768 blocks, 5 sweeps: 95.5 us, 100.3 as phases, 108.7 with the 192 too; 16, 64, then 256 and
+// 1024, 3 sweeps: 95.4 us, 88.7), and from kCoarseSweepsBig with levels up to kCoarseBig (8, 32,
+// 128, then 512, 12 sweeps: 107 us, 116; 5 sweeps: 87.5 us, 81.5).
+constexpr int kCoarseFew = 32, kCoarseSmall = 80, kCoarseBig = 128, kCoarseSweeps = 5, kCoarseSweepsBig = 12;
+
 // The V-cycle on trees whose sweeps push their ghosts, with its steps fused (the same values
 // in u and in b; r and u1, scratch, end with other contents).  A level's ghosts stay what
 // a fill would make of them -- the sweeps and the prolongation push their cells' copies and
@@ -1159,7 +1175,10 @@ static int vcycle_fused(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op
   };
   int top = 0;
   if constexpr (std::is_same_v<T, double>)
-    if (ctx->use_coarse) top = coarse_top(ctx, lmax, four, geom);
+    if (ctx->use_coarse) {
+      top = coarse_top(ctx, lmax, four, geom, kCoarseSmall);
+      if (top == 1 && ntop == 1 && ctx->lv[0].nblk > kCoarseFew) top = 0;
+    }
   for (int l = lmax; l > std::max(top, 1); l--) {
     const DevLevel &L = ctx->lv[l - 1], &C = ctx->lv[l - 2];
     RC(gs(l, ndown, filled || l < lmax));
@@ -1193,11 +1212,6 @@ static int vcycle_fused(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op
   return SRMG_OK;
 }
 
-// Splitting the persistent kernel's V-cycle around the cluster costs two more launches (25 us),
-// and a level's ~6 phases there take 20 to 25 us, its steps in the cluster 10 to 14: worth it
-// from this many levels on.
-constexpr int kCoarseWorth = 3;
-
 template <typename T>
 int srmg::vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, double k2, int geom,
                      const Signs &sg, int lmax, int ndown, int ntop, int nup, double omega, int ncycles, int *ran) {
@@ -1221,8 +1235,15 @@ int srmg::vcycle_dev(srmg_ctx *ctx, T *u, T *b, T *r, T *u1, double s, int op, d
       if (ctx->use_coarse && unit_signs(sg) && !ctx->trace_on) {
         RC(ensure_coarse(ctx));
         while (L > 1 && ctx->lv[L - 1].nblk == 0) --L;
-        top = coarse_top(ctx, L, false, geom);
-        if (L > top && top < kCoarseWorth) top = 0;
+        auto sweeps = [&](int t) { return (t - 1) * (ndown + nup) + ntop; };
+        top = coarse_top(ctx, L, false, geom, kCoarseCtas * kCoarsePer);
+        if (top == L) {
+          if (sweeps(L) <= 3 && coarse_top(ctx, L, false, geom, kCoarseBig) < L) top = 0;
+        } else {
+          top = coarse_top(ctx, L, false, geom, kCoarseBig);
+          if (sweeps(top) < kCoarseSweepsBig) top = coarse_top(ctx, L, false, geom, kCoarseSmall);
+          if (top < 2 || sweeps(top) < kCoarseSweeps) top = 0;
+        }
       }
       if (top >= 1 && L <= top) {
         if (ran) *ran = ncycles;

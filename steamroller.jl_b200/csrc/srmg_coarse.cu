@@ -545,11 +545,14 @@ int srmg::ensure_coarse(srmg_ctx *ctx) {
   return SRMG_OK;
 }
 
-// The levels from 1 up that a cycle with finest level lmax runs in the cluster.
-int srmg::coarse_top(const srmg_ctx *ctx, int lmax, bool four, int geom) {
+// The levels from 1 up that a cycle with finest level lmax can run in the cluster, of up to
+// `most` blocks each.
+int srmg::coarse_top(const srmg_ctx *ctx, int lmax, bool four, int geom, int most) {
   const CoarseTab &C = ctx->coarse;
   if (C.state != 1) return 0;
-  for (int t = std::min(lmax, C.levels); t >= 1; t--)
+  int levels = 0;
+  while (levels < std::min(lmax, C.levels) && C.nblk[levels + 1] <= most) ++levels;
+  for (int t = levels; t >= 1; t--)
     if (smem_bytes(C.base[t + 1], C.base[t], t < lmax, t, C.pbase[t + 1], four, geom) <= kCoarseSmem) return t;
   return 0;
 }

@@ -47,10 +47,10 @@ void free_tree(srmg_ctx *ctx);
 int ensure_gs_push(srmg_ctx *ctx, int op);
 int d3_ensure_push(srmg_ctx *ctx);
 // The coarse levels of an FP64 V-cycle in one cluster (srmg_coarse.cu): their tables (not while
-// the stream is capturing), how many levels from 1 up a cycle with finest level lmax gives it
-// (0: none), and the launch.
+// the stream is capturing), how many levels from 1 up, of up to `most` blocks each, a cycle with
+// finest level lmax can give it (0: none), and the launch.
 int ensure_coarse(srmg_ctx *ctx);
-int coarse_top(const srmg_ctx *ctx, int lmax, bool four, int geom);
+int coarse_top(const srmg_ctx *ctx, int lmax, bool four, int geom, int most);
 int coarse_launch(srmg_ctx *ctx, CoarseCycle &A, bool four, int geom);
 void drop_op_graphs(srmg_ctx *ctx);
 // One cooperative launch of the sequencer over `nops` recorded operations (srmg_seq.cu).
