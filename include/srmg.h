@@ -133,7 +133,11 @@ int srmg_set_tree3(srmg_ctx *ctx, int nlev,
 /* ---- the ccall boundary: HOST pointers (Julia-owned arrays) --------------------- */
 
 /* `ncycles` x vcycle! (src/multigrid.jl:60-106) on host arrays of nblk_alloc blocks.
- * u is in/out exactly as in the reference, ghosts included.  b: its leaf cells are
+ * u is in/out exactly as in the reference, ghosts included; its ghosts are to be filled on
+ * entry (as after fill_ghost! on every level, or an earlier cycle), as the reference's callers
+ * have them.  Where they are not, the first sweep of the finest level reads them as they are,
+ * and a persistent kernel also takes the neighbours' edge cells of that sweep's first colour
+ * from them, so that the result depends on which kernels run the cycle.  b: its leaf cells are
  * never written; the reference leaves the FAS right-hand side in the covered cells of
  * the coarse levels, which none of its callers reads (derivs! re-restricts q before
  * every solve, src/streamer.jl:313-318, and vcycle! overwrites those cells before it
@@ -581,10 +585,13 @@ int srmg_ssprk3_stage_dev(srmg_ctx *ctx, double *out, const double *n, const dou
  *                      after it (bit-identical results; tables built once per tree from
  *                      the fill itself, trees whose fill the tables cannot express keep
  *                      the fill launches); 0 = a fill launch after every colour;
- *   "coarse_cluster"   1 (default) = the coarse levels of an FP64 V-cycle on a 2D tree (up to
- *                      256 blocks each, as many as fit) run in one thread-block cluster
- *                      with their fields in shared memory (bit-identical results);
- *                      0 = as the finer ones;
+ *   "coarse_cluster"   1 (default) = the coarse levels of an FP64 V-cycle on a 2D tree (as many
+ *                      as fit and gain by it; a tree that fits runs there whole, with up to
+ *                      256 blocks a level) run in one thread-block cluster with their
+ *                      fields in shared memory; 0 = as the finer ones.  Results are
+ *                      bit-identical to the per-operation path's always, and to the
+ *                      persistent kernel's from a u whose ghosts are filled (see
+ *                      srmg_vcycle);
  *   "direct_level"     the level of the FP64 direct coarsest solve of mixed and
  *                      SRMG_MODE_FP64_DIRECT solves on the persistent kernel: 0 (default)
  *                      = level 2 for a lone tree whose level 2 holds 1..4 blocks and has no
