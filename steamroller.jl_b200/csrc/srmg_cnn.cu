@@ -350,7 +350,8 @@ k_cnn_loss(const float *__restrict__ y, const float *__restrict__ t, const __nv_
       gr += wm * srho[cy + 1][cx + 2];
       rweights(geom, ir0, cx - 1, wm, wp);
       if (cx >= 2) gr += wp * srho[cy + 1][cx];
-      gr += srho[cy + 2][cx + 1] + srho[cy][cx + 1];
+      gr += srho[cy + 2][cx + 1];
+      gr += srho[cy][cx + 1];
       g += (float)(2.0 * invr) * lambda * gr;
     }
     dy[k] = g;
@@ -439,16 +440,22 @@ k_cnn_dx(const float *__restrict__ dy, const __nv_bfloat16 *__restrict__ wt,
 // Weight gradients of all layers in one launch.  CTA b belongs to one layer l (the CTAs
 // shared out by the layers' work, DwParts) and sums over its samples
 //   dW[tap][co][ci] += sum_p dz_l[p][co] * A_l[p + off(tap)][ci],  db[co] += sum_p dz_l[p][co]
-// into partials [cta][9][32][32] and [cta][32].  15 warps: warp = (pixel fifth kg, tap row
+// into partials [cta][9][32][32] and [cta][32].  15 warps: warp = (fifth kg of the pixels, tap row
 // dy), three taps x 32 co x 32 ci a warp, so that one dz fragment serves three taps and both
 // of a tap's ci halves (8 ldmatrix per 24 mma; one warp per (tap, co half) took 3 per
-// 4).  db is one more mma against a matrix of ones.  The next sample's tiles arrive by
+// 4).  mma.sync truncates as it accumulates, and the error grows with the chain: a chain ends
+// after kPart samples (kFlush in the first and last layer, whose registers have room for the
+// sums beside) and goes to sums of rounded additions.  Sums of one sign over 6000 samples:
+// dW_1..4 off by 5e-7 to 1.2e-6 of the sum and dW_5 by 1.6e-7, 2.0e-5 to 5.5e-5 with a chain
+// over all of a CTA's samples (1024 samples: 5e-7 to 1.1e-6 and 2.0e-7, 1.9e-6 to 5.9e-6).  db
+// is summed from the fragments by rounded additions, per sample and then over the samples
+// (7.6e-8; by one more mma against ones 2e-5 to 7e-5).  The next sample's tiles arrive by
 // cp.async while this one is summed.  mma.sync bounds it; a launch per layer without the
 // copies in flight, with a serial db sum, took 6 x 55 us at 1024 samples.
 constexpr int kDwThreads = 15 * 32;
+constexpr int kFlush = 4, kPart = 16;
 constexpr int kDwStage = kTileBytes + kNP * kC * 2;
-constexpr int kDwSmem = 2 * kDwStage;
-static_assert(9 * kWMat * 4 + kC * 4 <= kDwStage, "the partial sums reuse a stage");
+constexpr int kDwSmem = 2 * kDwStage + 9 * kWMat * 4 + kC * 4;  // two stages and the CTA's sums
 struct DwParts {
   int first[kL + 1];  // CTAs first[l] .. first[l + 1] - 1 work on layer l
 };
@@ -493,18 +500,41 @@ __device__ __forceinline__ void dw_layer(unsigned char *sm, int l, int part, int
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float acc[3][MH][NT][4], accb[MH][4];
-#pragma unroll
-  for (int m = 0; m < MH; ++m) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) accb[m][j] = 0.f;
+  constexpr bool kShort = MH == 1 || NT == 1;  // the layers with fewer CTAs
+  float acc[3][MH][NT][4], sum[kShort ? 3 : 1][MH][NT][4];
+  float db[2] = {0.f, 0.f};  // co half dyr / 2 (dyr 1: none)
+  float *red = reinterpret_cast<float *>(sm + 2 * kDwStage), *redb = red + 9 * kWMat;  // zero
+  auto each = [&](auto fn) {  // over acc
 #pragma unroll
     for (int d = 0; d < 3; ++d)
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
+      for (int m = 0; m < MH; ++m)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[d][m][nt][j] = 0.f;
-  }
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) fn(d, m, nt, j);
+  };
+  each([&](int d, int m, int nt, int j) {
+    acc[d][m][nt][j] = 0.f;
+    if (kShort) sum[d][m][nt][j] = 0.f;
+  });
+  int since = 0;
+  auto flush = [&] {  // kShort: to the registers beside
+    each([&](int d, int m, int nt, int j) {
+      sum[d][m][nt][j] += acc[d][m][nt][j];
+      acc[d][m][nt][j] = 0.f;
+    });
+  };
+  auto put = [&] {  // to the CTA's sums, the five pixel fifths in order
+    for (int k = 0; k < 5; ++k) {
+      if (kg == k)
+        each([&](int d, int m, int nt, int j) {
+          red[(dyr * 3 + d) * kWMat + (m * 16 + g + (j >> 1) * 8) * kC + nt * 8 + 2 * t4 + (j & 1)] += acc[d][m][nt][j];
+          acc[d][m][nt][j] = 0.f;
+        });
+      __syncthreads();
+    }
+  };
   const int mt = lane >> 3, r = lane & 7;
   int st = 0;
   if (part < n) load(part, 0);
@@ -517,8 +547,9 @@ __device__ __forceinline__ void dw_layer(unsigned char *sm, int l, int part, int
     }
     __syncthreads();
     const uint32_t a_s = sm_s + st * kDwStage, z_s = a_s + kTileBytes;
+    float dbs[2] = {0.f, 0.f};  // this sample's
 #pragma unroll 1
-    for (int k0 = kg * 80; k0 < kg * 80 + 80; k0 += 16) {
+    for (int k0 = kg * 16; k0 < kNP; k0 += 80) {  // every fifth 16 pixels: no chain has only the rim
       // A operand (rows co, k = pixels) from dz [p][co] by transposed ldmatrix: matrices (co
       // 0-7, p 0-7), (co 8-15, p 0-7), (co 0-7, p 8-15), (co 8-15, p 8-15)
       uint32_t a[MH][4];
@@ -543,36 +574,39 @@ __device__ __forceinline__ void dw_layer(unsigned char *sm, int l, int part, int
           for (int nt = 0; nt < NT; ++nt)
             mma16816(acc[d][m][nt], a[m][0], a[m][1], a[m][2], a[m][3], b[2 * nt], b[2 * nt + 1]);
       }
-      if (dyr == 1) {
 #pragma unroll
-        for (int m = 0; m < MH; ++m)
-          mma16816(accb[m], a[m][0], a[m][1], a[m][2], a[m][3], 0x3F803F80u, 0x3F803F80u);
-      }
-    }
-    __syncthreads();  // the stage is free for the load after next
-  }
-  // the five pixel fifths in order
-  float *red = reinterpret_cast<float *>(sm), *redb = red + 9 * kWMat;
-  for (int k = 0; k < 5; ++k) {
-    if (kg == k) {
+      for (int m = 0; m < MH; ++m)
+        if (dyr == 2 * m) {
 #pragma unroll
-      for (int m = 0; m < MH; ++m) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float *o = red + (dyr * 3 + d) * kWMat + (m * 16 + g + (j >> 1) * 8) * kC + nt * 8 + 2 * t4 + (j & 1);
-              *o = k ? *o + acc[d][m][nt][j] : acc[d][m][nt][j];
-            }
-        if (dyr == 1 && t4 == 0) {
-          float *o = redb + m * 16 + g;
-          o[0] = k ? o[0] + accb[m][0] : accb[m][0];
-          o[8] = k ? o[8] + accb[m][2] : accb[m][2];
+          for (int j = 0; j < 4; ++j)  // co g (j even) or g + 8, two pixels
+            dbs[j & 1] += __uint_as_float(a[m][j] << 16) + __uint_as_float(a[m][j] & 0xffff0000u);
         }
-      }
     }
+    db[0] += dbs[0];
+    db[1] += dbs[1];
+    ++since;
+    if constexpr (kShort)
+      if (since % kFlush == 0) flush();
+    __syncthreads();  // the stage is free for the load after next
+    if constexpr (!kShort)
+      if (since % kPart == 0) put();
+  }
+  if constexpr (kShort) {
+    flush();
+    each([&](int d, int m, int nt, int j) { acc[d][m][nt][j] = sum[d][m][nt][j]; });
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int o = 1; o <= 2; o <<= 1) db[j] += __shfl_xor_sync(0xffffffffu, db[j], o);
+  put();
+  for (int k = 0; k < 5; ++k) {
+#pragma unroll
+    for (int m = 0; m < MH; ++m)
+      if (kg == k && dyr == 2 * m && t4 == 0) {
+        redb[m * 16 + g] += db[0];
+        redb[m * 16 + g + 8] += db[1];
+      }
     __syncthreads();
   }
   for (int i = threadIdx.x; i < 9 * kWMat; i += blockDim.x)
@@ -921,14 +955,15 @@ int cnn_fwd_train(srmg_cnn *net, const __nv_bfloat16 *x, int n) {
 }
 
 // The layers' shares of the weight-gradient CTAs: one CTA per SM, by the layers' work per
-// sample (the first layer has 2 input channels, the last one output channel).
+// sample (the first layer has 2 input channels, the last one output channel and its flushes:
+// the backward pass at 1024 samples takes 331 us, with 0.6 instead of 0.7 17 us more).
 DwParts dw_parts(int nsm, int n) {
-  static const double work[kL] = {0.4, 1, 1, 1, 1, 0.6};
+  static const double work[kL] = {0.4, 1, 1, 1, 1, 0.7};
   DwParts p;
   p.first[0] = 0;
   double done = 0.0;
   for (int l = 0; l < kL; ++l) {
-    done += work[l] / 5.0;
+    done += work[l] / 5.1;
     const int to = l == kL - 1 ? nsm : (int)std::lround(done * nsm);
     p.first[l + 1] = p.first[l] + std::max(1, std::min(n, to - p.first[l]));
   }
