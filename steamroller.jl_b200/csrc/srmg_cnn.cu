@@ -454,6 +454,7 @@ k_cnn_dx(const float *__restrict__ dy, const __nv_bfloat16 *__restrict__ wt,
 // copies in flight, with a serial db sum, took 6 x 55 us at 1024 samples.
 constexpr int kDwThreads = 15 * 32;
 constexpr int kFlush = 4, kPart = 16;
+constexpr int kBwdSamples = 8192;
 constexpr int kDwStage = kTileBytes + kNP * kC * 2;
 constexpr int kDwSmem = 2 * kDwStage + 9 * kWMat * 4 + kC * 4;  // two stages and the CTA's sums
 struct DwParts {
@@ -630,8 +631,9 @@ k_cnn_dw(DwParts parts, const float *__restrict__ dy, const __nv_bfloat16 *__res
 
 // Fixed-order sum of the per-CTA partials into the gradient (master layout), all layers in
 // one launch, a thread per parameter (16 CTAs a layer were latency-bound: 6 x 37 us).
+// add: to the gradient of the samples before.
 __global__ void k_cnn_reduce(DwParts parts, const float *__restrict__ dw_part, const float *__restrict__ db_part,
-                             float *__restrict__ grad) {
+                             float *__restrict__ grad, bool add) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nparams()) return;
   int l = 0;
@@ -650,7 +652,7 @@ __global__ void k_cnn_reduce(DwParts parts, const float *__restrict__ dw_part, c
   float s = 0.f;
 #pragma unroll 8
   for (int k = parts.first[l]; k < parts.first[l + 1]; ++k) s += src[(int64_t)k * stride];
-  grad[i] = s;
+  grad[i] = add ? grad[i] + s : s;
 }
 
 #include "srmg_cnn_tc.cuh"
@@ -942,7 +944,7 @@ int cnn_fwd_train(srmg_cnn *net, const __nv_bfloat16 *x, int n) {
   RC(ensure(ctx, net->xc, (size_t)n * kNP * 4));
   RC(ensure(ctx, net->acts, (kL - 1) * layer));
   RC(ensure(ctx, net->signs, (size_t)(kL - 1) * n * kNP * 4));
-  RC(ensure(ctx, net->dz, (kL - 1) * layer));
+  RC(ensure(ctx, net->dz, (size_t)std::min(n, kBwdSamples) * (kL - 1) * kNP * kC * 2));
   RC(ensure(ctx, net->y, (size_t)n * 256 * 4));
   RC(ensure(ctx, net->dy, (size_t)n * 256 * 4));
   RC(ensure(ctx, net->dwp, (size_t)net->nsm * 9 * kWMat * 4));
@@ -970,20 +972,27 @@ DwParts dw_parts(int nsm, int n) {
   return p;
 }
 
-// Backward from the output gradient held in net->dy (n samples of the last forward).
+// Backward from the output gradient held in net->dy (n samples of the last forward), up to
+// kBwdSamples at a time: their gradients of all five layers are in memory together (1 GB),
+// and with those of a whole large batch a training step would need more than the 205 KB a
+// sample that activations and two layers' gradients take (140 KB so).
 int cnn_bwd(srmg_cnn *net, int n) {
   srmg_ctx *ctx = net->err_ctx;
-  const float *dy = (const float *)net->dy.p;
-  const unsigned char *signs = (const unsigned char *)net->signs.p;
-  __nv_bfloat16 *dz = (__nv_bfloat16 *)net->dz.p;
-  if (n <= net->nsm) k_cnn_dx<13><<<n, cnn_threads(13), bwd_smem(13), net->stream>>>(dy, net->wt, signs, dz, n);
-  else k_cnn_dx<5><<<net->nsm, cnn_threads(5), bwd_smem(5), net->stream>>>(dy, net->wt, signs, dz, n);
-  const DwParts parts = dw_parts(net->nsm, n);
-  k_cnn_dw<<<parts.first[kL], kDwThreads, kDwSmem, net->stream>>>(parts, dy, dz, (const uint32_t *)net->xc.p,
-                                                                  (const __nv_bfloat16 *)net->acts.p, n,
-                                                                  (float *)net->dwp.p, (float *)net->dbp.p);
-  k_cnn_reduce<<<(nparams() + 127) / 128, 128, 0, net->stream>>>(parts, (const float *)net->dwp.p,
-                                                                (const float *)net->dbp.p, net->grad);
+  for (int s0 = 0; s0 < n; s0 += kBwdSamples) {
+    const int m = std::min(n - s0, kBwdSamples);
+    const float *dy = (const float *)net->dy.p + (int64_t)s0 * 256;
+    const unsigned char *signs = (const unsigned char *)net->signs.p + (int64_t)s0 * (kL - 1) * kNP * 4;
+    const __nv_bfloat16 *acts = (const __nv_bfloat16 *)net->acts.p + (int64_t)s0 * (kL - 1) * kNP * kC;
+    const uint32_t *xc = (const uint32_t *)net->xc.p + (int64_t)s0 * kNP;
+    __nv_bfloat16 *dz = (__nv_bfloat16 *)net->dz.p;
+    if (m <= net->nsm) k_cnn_dx<13><<<m, cnn_threads(13), bwd_smem(13), net->stream>>>(dy, net->wt, signs, dz, m);
+    else k_cnn_dx<5><<<net->nsm, cnn_threads(5), bwd_smem(5), net->stream>>>(dy, net->wt, signs, dz, m);
+    const DwParts parts = dw_parts(net->nsm, m);
+    k_cnn_dw<<<parts.first[kL], kDwThreads, kDwSmem, net->stream>>>(parts, dy, dz, xc, acts, m, (float *)net->dwp.p,
+                                                                    (float *)net->dbp.p);
+    k_cnn_reduce<<<(nparams() + 127) / 128, 128, 0, net->stream>>>(parts, (const float *)net->dwp.p,
+                                                                  (const float *)net->dbp.p, net->grad, s0 > 0);
+  }
   CK(cudaGetLastError());
   return SRMG_OK;
 }
