@@ -1005,8 +1005,11 @@ static int L_gs_colour_push(srmg_ctx *ctx, T *u, const T *b, int l, const OpPara
                          : (p.geom == 0   ? k_gs_push<T, false, 0>
                             : p.geom == 1 ? k_gs_push<T, false, 1>
                                           : k_gs_push<T, false, 2>);
-  launch_pdl(kern, grid_for((int64_t)L.nblk * (four ? 64 : 128), threads, kGridCap), threads, 0, ctx->stream, u, b,
-             L.view(l), p, wtab<T>(ctx), four ? parity >> 1 : parity, four ? parity & 1 : 0, ctx->push_lv[l - 1], sw);
+  // a cell a thread on large levels (36k blocks: 82 us a colour, 90 with the capped grid, whose later
+  // cells are not loaded ahead of anything); the last, part-full round of a few costs more than that
+  const int64_t ctas = ((int64_t)L.nblk * (four ? 64 : 128) + threads - 1) / threads;
+  const int64_t grid = ctas <= 2 * kGridCap ? std::min<int64_t>(ctas, kGridCap) : std::min<int64_t>(ctas, 1 << 20);
+  launch_pdl(kern, grid, threads, 0, ctx->stream, u, b, L.view(l), p, wtab<T>(ctx), four ? parity >> 1 : parity, four ? parity & 1 : 0, ctx->push_lv[l - 1], sw);
   ctx->launches++;
   return SRMG_OK;
 }
