@@ -1117,7 +1117,6 @@ static int coarse_levels(srmg_ctx *ctx, int top, double *u, double *b, double *r
   A.b = b;
   A.r = r;
   A.sg = sg;
-  A.sw = sign_bits(sg);
   A.wt = wtab<double>(ctx);
   A.top = top;
   A.inner = lmax > top;

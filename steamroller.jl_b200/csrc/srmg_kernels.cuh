@@ -1087,7 +1087,6 @@ struct CoarseCycle {
   double *u, *b, *r;
   Signs sg;
   WTab<double> wt;
-  unsigned sw;                // the boundary table as bits
   int top, inner, known;      // inner: level top + 1 exists and has been restricted (residual in r);
                               // known: else, whether level top's ghosts are filled
   int ndown, ntop, nup, ncycles;
