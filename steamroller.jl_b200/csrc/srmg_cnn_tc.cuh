@@ -19,7 +19,7 @@
 // wait is bounded; on a timeout the kernel sets *err, frees its TMEM and returns.
 //
 // Measured against the mma.sync forward (k_cnn_fwd) on one B200 it is correct to the
-// same tolerance but slower (0.92 vs 0.70 ms per 4096 samples).  It is latency-bound:
+// same tolerance but slower (0.92 vs 0.45 ms per 4096 samples).  It is latency-bound:
 // one sample per CTA is in flight, and per layer the MMAs, their commit and wait, and
 // the TMEM epilogue that writes the next layer's operands run one after another (tensor
 // pipe 9.6% active, 8 warps, long-scoreboard stalls leading).  Overlapping two samples

@@ -7,12 +7,11 @@
 // stay in one CTA, ghosts go to the neighbour's CTA by stores into its shared memory, and a
 // step is a cluster barrier (0.3 us), a stencil from shared memory (0.2) and those stores (0.2)
 // away from the next: latency all the way.  Two FP64 V-cycles (2, 4, 2) on the uniform tree of
-// 1 to 256 blocks, whole in the cluster: 231 -> 130 us (one launch; 146 as two); order 4 on the 2725-block tree, levels
-// of 1 to 64 blocks here: 164 -> 78 us of a cycle; full multigrid on the 400k-cell channel
-// tree: 1507 -> 1150 us.  The same with the fields in global memory took 2.0 us a colour.
-// 256 threads a CTA: a barrier costs more with more warps (512: 87 us of that cycle, 1024 on
-// the uniform tree 86 us a cycle instead of 73), and so do several cells a thread at a time
-// (two 82 us, four 92).
+// 1 to 256 blocks, whole in the cluster: 231 -> 130 us (one launch); order 4 on the 2725-block
+// tree, levels of 1 to 64 blocks here: 164 -> 78 us of a cycle; full multigrid on the
+// 400k-cell channel tree: 1507 -> 1130 us.  256 threads a CTA, one cell a thread at a time: more
+// warps make the barriers dearer, more cells a thread the chain longer (order 4, 512 threads:
+// 87 us of that cycle; two cells: 82).
 #include <algorithm>
 
 #include "srmg_ctx.h"
