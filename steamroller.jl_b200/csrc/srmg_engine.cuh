@@ -1865,7 +1865,7 @@ __global__ void __launch_bounds__(NT, 1) k_engine_vcycle(const __grid_constant__
       const bool loc = 1 <= K;
       if (runs(loc))
         ph_direct_top<T>(A, fld(1), L > 1, loc ? 0 : blockIdx.x, loc ? 1 : gridDim.x, t, slot, s_direct, s_rhs);
-      if (!sync(true, loc, 2 <= K || L < 2)) return false;
+      if (!sync(true, loc, 2 <= K)) return false;  // on a single level every CTA's next phase waits for it
     } else {
       const bool loc = 1 <= K;
       for (int it = 0; it < A.ntop; ++it) {
@@ -1875,7 +1875,7 @@ __global__ void __launch_bounds__(NT, 1) k_engine_vcycle(const __grid_constant__
           ok = ph_gsi<T>(A, 1, fld(1), oth(1), nullptr, it == 0 && L > 1, last && L > 1, it == 0 && L > 1,
                          first_of(loc), step_of(loc), t, slot, S, pk, s_halo);
         cur ^= 1u << 1;
-        if (!sync(ok, loc, last ? (2 <= K || L < 2) : loc)) return false;
+        if (!sync(ok, loc, last ? 2 <= K : loc)) return false;
       }
     }
     // ascending leg
