@@ -1445,7 +1445,8 @@ __device__ void ph_itemnorm(const EngArgs<T> &A, bool first, int cycles, int ste
 // Coarsest level solved directly (mixed-precision solve), one item per CTA: FAS
 // right-hand side of the covered cells, then u_1 = P b_1 with the item's
 // P = -s A_1^{-1} applied in FP64 (one warp per row), ghosts pushed, and the
-// correction e = u_1 - u1 of the level.  An item's level 1 has <= 4 blocks.
+// correction e = u_1 - u1 of the level.  An item's level 1 has <= 4 blocks, a CTA three or
+// four slots.
 template <typename T>
 __device__ void ph_direct_top(const EngArgs<T> &A, T *u, bool make_e, int first, int step, int t, int slot,
                               double *sol, double *rhs) {
@@ -1459,8 +1460,8 @@ __device__ void ph_direct_top(const EngArgs<T> &A, T *u, bool make_e, int first,
     const int4 *blocks = A.tr.lvl_blocks[0] + rg.x;
     const T *par = A.it_par + k * kParStride;
     const T s = par[1], centre = par[32 + 1];
-    if (slot < n1) {
-      const int4 bk = blocks[slot];
+    for (int bi = slot; bi < n1; bi += blockDim.x >> 8) {
+      const int4 bk = blocks[bi];
       const int X = bk.x;
       const T uo = u[(int64_t)X * kSS + o];
       A.u1[(int64_t)X * kSS + o] = uo;
@@ -1499,11 +1500,11 @@ __device__ void ph_direct_top(const EngArgs<T> &A, T *u, bool make_e, int first,
       }
     }
     __syncthreads();
-    if (slot < n1) {
-      const int4 bk = blocks[slot];
+    for (int bi = slot; bi < n1; bi += blockDim.x >> 8) {
+      const int4 bk = blocks[bi];
       const int X = bk.x;
       const int4 *fc = A.tr.faces + 4 * X;
-      const T nu = (T)sol[slot * 256 + (t & 255)];
+      const T nu = (T)sol[bi * 256 + (t & 255)];
       u[(int64_t)X * kSS + o] = nu;
       push<T>(A, k, u, X, fc, x, y, nu);
       if (make_e) {

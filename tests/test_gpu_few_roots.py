@@ -43,3 +43,30 @@ def test_vcycle_equals_the_launches(root, level, ntop):
     for other in out[1:]:
         for x, y in zip(out[0], other):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("root", ROOTS)
+@pytest.mark.parametrize("level", [1, 2, 3])
+@pytest.mark.parametrize("mode", ["MODE_MIXED", "MODE_FP64_DIRECT", "MODE_FP64"])
+@pytest.mark.parametrize("direct_level", [0, 1])
+def test_solves_do_not_depend_on_the_shape(root, level, mode, direct_level):
+    import torch
+    p, out = problem(root, level), []
+    for threads in (768, 1024):
+        ctx = mg.Context(0).set_tree(p.tree, p.conn)
+        ctx.set_option("engine_threads", threads).set_option("direct_level", direct_level)
+        b = torch.from_numpy(p.b).cuda()
+        for _ in range(3):
+            u = torch.zeros_like(b)
+            # the reference's cycle (MODE_FP64) contracts slowly on 16 x 64 cells: thirty of them
+            st = mg.solve(ctx, u, b, p.s, p.geom, p.bc, tol=1e-9, mode=getattr(mg, mode),
+                          max_cycles=30 if mode == "MODE_FP64" else 400)
+            assert mode == "MODE_FP64" or st["rel_residual"] <= 1e-9, st
+            out.append((st["cycles"], u.cpu().numpy()[:, 2:18, 2:18].copy().view(np.uint64)))
+        norm = mg.resnorm(ctx, None, b, u, p.s, p.geom, p.bc)
+        scale = mg.resnorm(ctx, None, b, torch.zeros_like(b), p.s, p.geom, p.bc)
+        assert mode == "MODE_FP64" or norm <= 1.0001e-9 * scale
+        ctx.close()
+    for c, u in out[1:]:
+        assert c == out[0][0]
+        np.testing.assert_array_equal(u, out[0][1])
