@@ -27,7 +27,8 @@
 //                      new edge values, and the block's refinement-boundary ghosts
 //                      interpolated from the (final) coarser level.
 // The coarse correction e = u - u1 of a level (diffto!, src/blockfield.jl:569-576) and
-// its ghosts are produced in that level's last GS iteration.  Levels 1..local_top are
+// its ghosts are produced in that level's last GS iteration (a single one on level 1 forms the
+// FAS right-hand side from e, and the correction follows in a phase of its own).  Levels 1..local_top are
 // processed by CTA 0 alone with CTA barriers.  Block tiles reach shared memory through
 // bulk asynchronous copies (cp.async.bulk, no multicast) into a four-buffer per-slot
 // pipeline; every wait on an mbarrier or a barrier is bounded in time.  The arithmetic
@@ -1623,6 +1624,22 @@ __device__ bool ph_direct2_rows_split(const EngArgs<T> &A, T *u, int lt, bool ma
   return true;
 }
 
+// The correction e = u - u1 of level 1 with its ghost pushes, as a phase of its own: a single
+// sweep there reads the neighbours' restricted residual from e, which its own last step
+// would overwrite.  Not inlined, so that the kernel's registers stay as they are.
+template <typename T>
+__device__ __noinline__ void ph_make_e(const EngArgs<T> &A, const T *u, int first, int step, int t) {
+  const int x = 2 + (t & 15), y = 2 + (t >> 4), o = x + kS * y;
+  for (int i = first; i < A.tr.nblk[0]; i += step) {
+    const int4 bk = A.tr.lvl_blocks[0][i];
+    if (is_frozen(A, item_of(bk))) continue;
+    const int64_t at = (int64_t)bk.x * kSS + o;
+    const T ev = u[at] - A.u1[at];
+    A.e[at] = ev;
+    push<T>(A, item_of(bk), A.e, bk.x, A.tr.faces + 4 * bk.x, x, y, ev);
+  }
+}
+
 // Copy level l's blocks (valid cells and face ghosts) from src to dst.
 template <typename T>
 __device__ void ph_copy_back(const EngArgs<T> &A, int l, const T *src, T *dst, int first, int step, int t) {
@@ -1873,10 +1890,14 @@ __global__ void __launch_bounds__(NT, 1) k_engine_vcycle(const __grid_constant__
         const bool last = it == A.ntop - 1;
         bool ok = true;
         if (runs(loc))
-          ok = ph_gsi<T>(A, 1, fld(1), oth(1), nullptr, it == 0 && L > 1, last && L > 1, it == 0 && L > 1,
+          ok = ph_gsi<T>(A, 1, fld(1), oth(1), nullptr, it == 0 && L > 1, last && it > 0 && L > 1, it == 0 && L > 1,
                          first_of(loc), step_of(loc), t, slot, S, pk, s_halo);
         cur ^= 1u << 1;
-        if (!sync(ok, loc, last ? 2 <= K : loc)) return false;
+        if (!sync(ok, loc, last && (it > 0 || L < 2) ? 2 <= K : loc)) return false;
+      }
+      if (A.ntop == 1 && L > 1) {
+        if (runs(loc)) ph_make_e<T>(A, fld(1), first_of(loc), step_of(loc), t);
+        if (!sync(true, loc, 2 <= K)) return false;
       }
     }
     // ascending leg
