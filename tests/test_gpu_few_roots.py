@@ -31,7 +31,7 @@ def test_vcycle_equals_the_launches(root, level, ntop):
     for engine, threads in ((0, 0), (1, 768), (1, 1024)):
         ctx = mg.Context(0).set_tree(p.tree, p.conn)
         ctx.set_option("coarse_cluster", 0).set_option("engine", engine).set_option("engine_threads", threads)
-        for _ in range(1 if not engine else 10):
+        for _ in range(1 if not engine else 4):
             b = torch.from_numpy(p.b).cuda()
             u, r, u1 = torch.from_numpy(start).cuda(), torch.zeros_like(b), torch.zeros_like(b)
             for l in range(1, level + 1):
@@ -45,7 +45,7 @@ def test_vcycle_equals_the_launches(root, level, ntop):
             np.testing.assert_array_equal(x, y)
 
 
-@pytest.mark.parametrize("root", ROOTS)
+@pytest.mark.parametrize("root", [(1, 3), (2, 2)])
 @pytest.mark.parametrize("level", [1, 2, 3])
 @pytest.mark.parametrize("mode", ["MODE_MIXED", "MODE_FP64_DIRECT", "MODE_FP64"])
 @pytest.mark.parametrize("direct_level", [0, 1])
